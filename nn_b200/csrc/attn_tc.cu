@@ -50,7 +50,8 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
     __shared__ uint32_t tmem_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t kvf = smem_u32(bars), kve = kvf + 16, sf = kvf + 32, pf = kvf + 40;
-    const int kvh = blockIdx.x, group = a.heads / a.kv_heads, pairs = a.span.n * group, t0 = blockIdx.y * kAtRows;
+    // (the last rows first: under a wide window they see the most keys)
+    const int kvh = blockIdx.x, group = a.heads / a.kv_heads, pairs = a.span.n * group, t0 = (gridDim.y - 1 - blockIdx.y) * kAtRows;
     const int last_pair = min(pairs, t0 + kAtRows) - 1;
     const int pos0 = a.span.pos0;
     const int first = max(0, pos0 + t0 / group - a.window + 1), last = pos0 + last_pair / group;   // keys some row sees

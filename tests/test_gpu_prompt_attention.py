@@ -1,0 +1,77 @@
+"""Prompt pass of a Qwen3-shaped decoder with bf16 product inputs at the sizes where its attention changes form: below and
+from 32 query vectors per key / value head, around the edges of 128-vector and 64-key tiles, every size of head group, in
+one portion and in two."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from nn_b200 import api, decoder
+from nn_b200.formats import QuantFormat as Q
+from oracle import qwen3_ref as ref
+
+pytestmark = pytest.mark.gpu
+HIDDEN, FFN, VOCAB, EPS = 128, 192, 160, 1e-6
+
+
+def _model(group, count):
+    rng = np.random.default_rng(100 + group)
+    kv = 2 if group < 8 else 1
+    cfg = decoder.DecoderConfig(hidden=HIDDEN, n_heads=kv * group, n_kv_heads=kv, ffn=FFN, n_layers=2, vocab=VOCAB, max_seq=count + 3, act_dtype=api.BF16)
+    dec, b = decoder.Decoder(api.gpu_backend(), cfg), api.gpu_backend()
+
+    def weight(n, k):
+        w = torch.from_numpy(rng.standard_normal((n, k)).astype(np.float32) / np.sqrt(k).astype(np.float32)).to(torch.bfloat16).cuda()
+        return api.DeviceWeight.from_device(b, Q.BF16_DENSE, w.view(torch.uint8).reshape(-1), n, k), w.float().cpu().numpy()
+
+    norm = lambda n: (1.0 + 0.1 * rng.standard_normal(n)).astype(np.float32)  # noqa: E731
+    model = {"layers": [], "cfg": cfg}
+    q, k = cfg.n_heads * 128, kv * 128
+    for i in range(cfg.n_layers):
+        ws = [weight(n, m) for n, m in ((q, HIDDEN), (k, HIDDEN), (k, HIDDEN), (HIDDEN, q), (FFN, HIDDEN), (FFN, HIDDEN), (HIDDEN, FFN))]
+        ns = [norm(HIDDEN), norm(HIDDEN), norm(128), norm(128)]
+        dec.set_layer(i, *[w for w, _ in ws], *ns)
+        model["layers"].append(([f for _, f in ws], ns))
+    embed = torch.from_numpy(rng.standard_normal((VOCAB, HIDDEN)).astype(np.float32)).to(torch.bfloat16).cuda()
+    head, model["head"] = weight(VOCAB, HIDDEN)
+    model["embed"], model["final"] = embed.float().cpu().numpy(), norm(HIDDEN)
+    dec.set_head(embed, model["final"], head)
+    return dec, model
+
+
+def _forward(model, ids):
+    """All rows at once in f32, the products' inputs rounded to bf16 as the decoder rounds them."""
+    c, T, r = model["cfg"], len(ids), ref.bf16_round
+    cos, sin = ref.rope_tables(128, T, c.rope_theta)
+    h = model["embed"][ids]
+    for (q, k, v, o, g, u, d), (n1, n2, nq, nk) in model["layers"]:
+        x = r(ref.rms_norm(h, n1, EPS))
+        Q_ = ref.rotate(ref.rms_norm((x @ q.T).reshape(T, -1, 128), nq, EPS), cos[:, None], sin[:, None])
+        K = ref.rotate(ref.rms_norm((x @ k.T).reshape(T, -1, 128), nk, EPS), cos[:, None], sin[:, None])
+        V = (x @ v.T).reshape(T, -1, 128)
+        out = np.empty_like(Q_)
+        for j in range(c.n_heads):
+            m = j // (c.n_heads // c.n_kv_heads)
+            s = (Q_[:, j] @ K[:, m].T) / np.sqrt(np.float32(128))
+            s[np.triu_indices(T, 1)] = -np.inf
+            p = np.exp(s - s.max(1, keepdims=True))
+            out[:, j] = (p / p.sum(1, keepdims=True)) @ V[:, m]
+        h = h + r(out.reshape(T, -1)) @ o.T
+        x = r(ref.rms_norm(h, n2, EPS))
+        gate = x @ g.T
+        h = h + r(gate / (1 + np.exp(-gate)) * (x @ u.T)) @ d.T
+    return r(ref.rms_norm(h, model["final"], EPS)) @ model["head"].T
+
+
+@pytest.mark.parametrize("group", [1, 2, 4, 8])
+@pytest.mark.parametrize("count", [3, 7, 8, 31, 33, 64, 65, 130])
+def test_prompt_rows_of_every_group_size(group, count):
+    dec, model = _model(group, count)
+    ids = np.random.default_rng(count).integers(0, VOCAB, count)
+    want = _forward(model, ids)
+    for cut in (0, count // 3):
+        got = np.concatenate([dec.extend(ids[a:e], a, list(range(e - a))) for a, e in ((0, cut), (cut, count)) if e > a])
+        # both sides round the same five inputs of a layer's products to bf16: the bar of the decoder's bf16 tests
+        assert np.max(np.abs(got - want)) <= 1e-2 * np.max(np.abs(want)), (cut, np.max(np.abs(got - want)) / np.max(np.abs(want)))
+    dec.backend.device_status()
+    dec.release()
