@@ -5,11 +5,11 @@
 // over the raw blocks writes bf16 [N, K] into a scratch buffer owned by the context (0.56 + 2 bytes
 // per weight at HBM speed; weights up to ~60 MB stay in L2 for the GEMM), and the GEMM main loop
 // then does nothing but move tiles and issue MMAs:
-//   * persistent CTAs (one per SM), output tiles of 128 x 256, k steps of 64 (one 128-byte swizzle
-//     row of bf16), a 4-stage ring of (16 KB activation tile + 32 KB weight tile);
+//   * persistent CTAs (one per SM), output tiles of 256 x 256 by pairs of CTAs (or 128 x 256, 128 x 128 by one), k steps of
+//     64 (one 128-byte swizzle row of bf16), a ring of 6 x (16 KB activation tile + 16 KB weight tile) per CTA;
 //   * warp 0: one thread issues the TMA loads of both tiles (cp.async.bulk.tensor.2d, 128-byte
 //     swizzle, zero fill beyond M / N) onto the stage's "full" barrier;
-//   * warp 1: one thread issues tcgen05.mma (M 128, N 256, K 16, bf16 x bf16 -> f32) into one of
+//   * warp 1: one thread (of the pair) issues tcgen05.mma (M 256, N 256, K 16, bf16 x bf16 -> f32) into one of
 //     two 256-column accumulators in tensor memory and commits the stage's "empty" barrier;
 //   * warps 2..5: epilogue -- tcgen05.ld of the finished accumulator (each warp its quarter of
 //     the 128 lanes), bias, conversion, stores -- while the MMA warp already fills the other
@@ -199,15 +199,24 @@ static cudaError_t launch_dequant_bf16(const uint8_t *src, const uint8_t *scales
 // bf16 GEMM: y[M, N] = x[M, K] * Wd[N, K]^T (+ bias)
 // ---------------------------------------------------------------------------------
 
-// Tile 128 x BN x 64 with BN = 256, or 128 where 256-wide tiles would leave SMs without a tile.
-constexpr int kDgBM = 128, kDgBK = 64, kDgStages = 4;
+// Tile 128 CG x BN x 64: CG = 2 CTAs of a cluster multiply one tile together (cta_group::2), or one CTA its own. BN = 256,
+// or 128 where 256-wide tiles would leave SMs without a tile.
+constexpr int kDgBM = 128, kDgBK = 64;
 constexpr int kDgABytes = kDgBM * 128;
 constexpr int kDgThreads = 192;
-__host__ __device__ constexpr int dg_stage_bytes(int bn) { return kDgABytes + bn * 128; }
+__host__ __device__ constexpr int dg_stage_bytes(int bn, int cg) { return kDgABytes + bn / cg * 128; }
+__host__ __device__ constexpr int dg_stages(int, int cg) { return cg == 1 ? 4 : 6; }
+static int dg_smem_bytes(int bn, int cg) { return dg_stages(bn, cg) * dg_stage_bytes(bn, cg) + 1024; }
 
 __device__ __forceinline__ void dg_tma_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+// the same into this CTA's shared memory, completion counted on a barrier of either CTA of the pair (a shared::cluster address)
+__device__ __forceinline__ void dg_tma_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 
@@ -217,12 +226,18 @@ __device__ __forceinline__ void dg_tma_2d(uint32_t dst, const CUtensorMap *map, 
 // inside a tile are computed but not stored. offsets == NULL: a plain product.
 constexpr int kDgMaxGroups = 256;
 
-template <int BN>
+// A pair of CTAs (CG = 2) holds 128 rows of the activation tile and BN / 2 rows of the weight tile each: the tensor cores
+// read both halves, so an operand byte is brought to shared memory and read from it once per 256 x 256 products instead of
+// once per 128 x 256. With one CTA the two (48 KB in, 48 KB out per 64-wide k step of 512 tensor-core clocks) exceed what
+// shared memory moves. The first CTA of the pair issues the MMAs; its "full" barriers count both CTAs' copies, its "empty" and "accumulator
+// full" commits reach both CTAs, both CTAs' epilogues hand the accumulators back to it.
+// 25600 x 5120 at 4096 rows: 731 -> 696 us (1.54 PFLOP/s), the seven products of such a layer 2890 -> 2715 us.
+template <int BN, int CG>
 __global__ void __launch_bounds__(kDgThreads, 1)
 gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                   const float *__restrict__ bias, void *__restrict__ y, int M, int N, int K, int y_dt, int *status,
                   const int *__restrict__ offsets, int groups, __nv_bfloat16 *__restrict__ h_out, float swiglu_limit, int gate_kind) {
-    constexpr int kDgBN = BN, kDgStageBytes = dg_stage_bytes(BN);
+    constexpr int kDgBN = BN, kDgStageBytes = dg_stage_bytes(BN, CG), kDgStages = dg_stages(BN, CG), kDgRows = kDgBM * CG;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t bars[2 * kDgStages + 4];   // full[4], empty[4], acc_full[2], acc_empty[2]
@@ -232,6 +247,8 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t full_s = smem_u32(bars), empty_s = full_s + 8 * kDgStages;
     const uint32_t accf_s = empty_s + 8 * kDgStages, acce_s = accf_s + 16;
+    const int rank = CG == 2 ? (int)cluster_rank() : 0;
+    const int unit = blockIdx.x / CG, units = gridDim.x / CG;   // a unit multiplies one tile at a time
     __shared__ int tile_begin[kDgMaxGroups + 1], row_begin[kDgMaxGroups + 1];
     if (tid == 0) {
         if (offsets) {
@@ -239,13 +256,13 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
             for (int e = 0; e < groups; e++) {
                 tile_begin[e] = acc;
                 row_begin[e] = offsets[e];
-                acc += (offsets[e + 1] - offsets[e] + kDgBM - 1) / kDgBM;
+                acc += (offsets[e + 1] - offsets[e] + kDgRows - 1) / kDgRows;
             }
             tile_begin[groups] = acc;
             row_begin[groups] = offsets[groups];
         } else {
             tile_begin[0] = 0;
-            tile_begin[1] = (M + kDgBM - 1) / kDgBM;
+            tile_begin[1] = (M + kDgRows - 1) / kDgRows;
             row_begin[0] = 0;
             row_begin[1] = M;
         }
@@ -255,12 +272,12 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     const int m_tiles = tile_begin[ngroups], n_tiles = (N + kDgBN - 1) / kDgBN;
     const int tiles = m_tiles * n_tiles;
     const int nkb = K / kDgBK;
-    // tile t -> (group, first row, end of the group's rows, first weight row)
+    // tile t -> (group, this CTA's first row, end of the group's rows, first weight row)
     auto locate = [&](int t, int &e, int &m0, int &m_end, int &n0) {
         const int mt = t % m_tiles;
         e = 0;
         while (e + 1 < ngroups && mt >= tile_begin[e + 1]) e++;
-        m0 = row_begin[e] + (mt - tile_begin[e]) * kDgBM;
+        m0 = row_begin[e] + (mt - tile_begin[e]) * kDgRows + rank * kDgBM;
         m_end = row_begin[e + 1];
         n0 = (t / m_tiles) * kDgBN;
     };
@@ -272,17 +289,23 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(accf_s + 8 * a, 1);
-            mbar_init(acce_s + 8 * a, 4);
+            mbar_init(acce_s + 8 * a, 4 * CG);
         }
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (CG == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if (CG == 2) cluster_sync();   // both CTAs' barriers are set up
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
     bool ok = true;
@@ -290,22 +313,28 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
+            const uint32_t count_s = CG == 2 ? cluster_addr(full_s, 0) : full_s;   // the barriers that count the copies
             int slot = 0;
             uint32_t phase = 0;
             long long filled = 0;
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            for (int t = unit; t < tiles && ok; t += units) {
                 int e, m0, m_end, n0;
                 locate(t, e, m0, m_end, n0);
-                const int w0 = e * N + n0;   // weight rows of this group in the decoded [groups * N, K] matrix
+                const int w0 = e * N + n0 + rank * (BN / CG);   // weight rows of this group in the decoded [groups * N, K] matrix
                 for (int kb = 0; kb < nkb; kb++) {
                     if (filled >= kDgStages && !mbar_wait_fast(empty_s + 8 * slot, phase ^ 1u)) {
                         ok = false;
                         break;
                     }
                     const uint32_t a_s = smem_u32(smem + (size_t)slot * kDgStageBytes);
-                    mbar_expect_tx(full_s + 8 * slot, kDgStageBytes);
-                    dg_tma_2d(a_s, &xmap, kb * kDgBK, m0, full_s + 8 * slot);
-                    dg_tma_2d(a_s + kDgABytes, &wmap, kb * kDgBK, w0, full_s + 8 * slot);
+                    if (rank == 0) mbar_expect_tx(full_s + 8 * slot, CG * kDgStageBytes);
+                    if (CG == 2) {
+                        dg_tma_2d_pair(a_s, &xmap, kb * kDgBK, m0, count_s + 8 * slot);
+                        dg_tma_2d_pair(a_s + kDgABytes, &wmap, kb * kDgBK, w0, count_s + 8 * slot);
+                    } else {
+                        dg_tma_2d(a_s, &xmap, kb * kDgBK, m0, full_s + 8 * slot);
+                        dg_tma_2d(a_s + kDgABytes, &wmap, kb * kDgBK, w0, full_s + 8 * slot);
+                    }
                     filled++;
                     if (++slot == kDgStages) {
                         slot = 0;
@@ -316,13 +345,13 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            // f32 accumulate, bf16 x bf16, both K-major, N = BN, M = 128
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)BN >> 3) << 17) | ((128u >> 4) << 24);
+        if (lane == 0 && rank == 0) {
+            // f32 accumulate, bf16 x bf16, both K-major, N = BN, M = 128 CG
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)BN >> 3) << 17) | (((uint32_t)kDgRows >> 4) << 24);
             int slot = 0;
             uint32_t phase = 0;
             int it = 0;
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, it++) {
+            for (int t = unit; t < tiles && ok; t += units, it++) {
                 const int a = it & 1;
                 // the epilogue has read this accumulator's previous tile
                 if (it >= 2 && !mbar_wait_fast(acce_s + 8 * a, (uint32_t)(((it >> 1) - 1) & 1))) {
@@ -340,21 +369,27 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                     const uint32_t a_s = smem_u32(smem + (size_t)slot * kDgStageBytes);
                     const uint64_t da = smem_desc(a_s), db = smem_desc(a_s + kDgABytes);
 #pragma unroll
-                    for (int k = 0; k < 4; k++) umma_bf16(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                    umma_commit(empty_s + 8 * slot);
+                    for (int k = 0; k < 4; k++) {
+                        if (CG == 2) umma_bf16_pair(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        else umma_bf16(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                    }
+                    if (CG == 2) umma_commit_pair(empty_s + 8 * slot);
+                    else umma_commit(empty_s + 8 * slot);
                     if (++slot == kDgStages) {
                         slot = 0;
                         phase ^= 1u;
                     }
                 }
-                if (ok) umma_commit(accf_s + 8 * a);
+                if (ok && CG == 2) umma_commit_pair(accf_s + 8 * a);
+                else if (ok) umma_commit(accf_s + 8 * a);
             }
         }
     } else {
         // ---------------- epilogue ----------------
+        const uint32_t back_s = CG == 2 ? cluster_addr(acce_s, 0) : acce_s;
         const int q = warp & 3;   // the quarter of the 128 TMEM lanes this warp may read
         int it = 0;
-        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, it++) {
+        for (int t = unit; t < tiles && ok; t += units, it++) {
             const int a = it & 1;
             int e, m0, m_end, n0;
             locate(t, e, m0, m_end, n0);
@@ -444,7 +479,10 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(acce_s + 8 * a);
+            if (lane == 0) {
+                if (CG == 2) mbar_arrive_cluster(back_s + 8 * a);
+                else mbar_arrive(acce_s + 8 * a);
+            }
         }
     }
     if (!ok) {
@@ -452,14 +490,17 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
         atomicExch(status, 1);
     }
     __syncthreads();
+    // with an aborted CTA, MMAs may still be in flight: give the last accumulator a bounded chance
+    if (warp == 1 && abort_s) {
+        mbar_wait(accf_s, 0);
+        mbar_wait(accf_s + 8, 0);
+    }
+    // a CTA of a pair stays until the other one has no more use for its shared memory, barriers and tensor memory
+    if (CG == 2) cluster_sync();
     if (warp == 1) {
-        // with an aborted CTA, MMAs may still be in flight: give the last accumulator a bounded chance
-        if (abort_s) {
-            mbar_wait(accf_s, 0);
-            mbar_wait(accf_s + 8, 0);
-        }
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+        if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
 }
 
@@ -531,27 +572,67 @@ nnq_status dense_scratch_reserve(nnq_ctx *ctx, int64_t n, int64_t k) {
     return NNQ_OK;
 }
 
-// 256-wide tiles unless they would leave more than half of the SMs without a tile (few row tiles,
-// narrow weights): then twice as many 128-wide tiles still fit one wave. (Measured: 4096 x 4096 at
-// 512 rows 64 -> 128 tiles, +13 %; 1024 x 5120 at 4096 rows, 128 tiles of 256 beat 256 of 128.)
-static int dg_pick_bn(const nnq_ctx *ctx, int64_t m_tiles, int64_t n) {
-    return 2 * m_tiles * ((n + 255) / 256) <= ctx->sm_count ? 128 : 256;
+// Shape of a tile: its width and the CTAs that share it. Pairs with 256 x 256 tiles, or single CTAs with 128 x 128 tiles where
+// the large ones would leave more than half of the SMs without work. (4096 rows of the 32B shape, pair / single CTA with
+// 128 x 256: 25600 x 5120 696 / 731 us, 8192 x 5120 219 / 239, 5120 x 25600 802 / 853. 1024 x 4096 at 1024 rows, 256 x 128 by
+// a pair / 128 x 128 by a CTA: 25.6 / 22.8 us.)
+struct DgShape {
+    int bn, cg;
+};
+static DgShape dg_pick(const nnq_ctx *ctx, int64_t m, int64_t n) {
+    const int64_t pair_tiles = (m + 255) / 256 * ((n + 255) / 256);
+    return 4 * pair_tiles <= ctx->sm_count ? DgShape{128, 1} : DgShape{256, 2};
+}
+// Experts: the last row tile of each is filled by half on average, so tiles of 128 rows. (32 experts, 16384 routed rows: single
+// CTAs 572 + 328 us, pairs 564 + 322 when only they run, 1.855 against 1.879 ms for the block.)
+static DgShape dg_pick_grouped(const nnq_ctx *ctx, int64_t rows, int experts, int64_t n) {
+    const int64_t m_tiles = rows / kDgBM + experts;   // at most
+    return {2 * m_tiles * ((n + 255) / 256) <= ctx->sm_count ? 128 : 256, 1};
 }
 
-static nnq_status dg_configure(nnq_ctx *ctx, int bn) {
-    static bool configured[64][2] = {};
+struct DgArgs {
+    const float *bias;
+    void *y;
+    int m, n, k, y_dt;
+    const int *offsets;
+    int groups;
+    __nv_bfloat16 *h_out;
+    float swiglu_limit;
+    int gate_kind;
+};
+
+template <int BN, int CG>
+static nnq_status dg_launch(nnq_ctx *ctx, const CUtensorMap &xmap, const CUtensorMap &wmap, const DgArgs &a, int64_t tiles, cudaStream_t stream) {
+    static bool configured[64] = {};
+    const int smem = dg_smem_bytes(BN, CG);
     int dev = 0;
     cudaGetDevice(&dev);
-    const int which = bn == 256 ? 0 : 1;
-    if (dev >= 0 && dev < 64 && !configured[dev][which]) {
-        const int smem_bytes = kDgStages * dg_stage_bytes(bn) + 1024;
-        nnq_status s = check_cuda(ctx, bn == 256 ? cudaFuncSetAttribute(gemm_dense_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes)
-                                                 : cudaFuncSetAttribute(gemm_dense_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes),
-                                  "GEMM attribute");
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        nnq_status s = check_cuda(ctx, cudaFuncSetAttribute(gemm_dense_kernel<BN, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "GEMM attribute");
         if (s != NNQ_OK) return s;
-        configured[dev][which] = true;
+        if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    return NNQ_OK;
+    const int64_t most = ctx->sm_count / CG;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(CG * (tiles < most ? tiles : most)));
+    cfg.blockDim = dim3(kDgThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CG;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = CG == 2 ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_dense_kernel<BN, CG>, xmap, wmap, a.bias, a.y, a.m, a.n, a.k, a.y_dt, ctx->d_status, a.offsets, a.groups,
+                                             a.h_out, a.swiglu_limit, a.gate_kind);
+    ctx->launches++;
+    return check_cuda(ctx, e, "bf16 GEMM launch");
+}
+
+static nnq_status dg_launch_shape(nnq_ctx *ctx, DgShape shape, const CUtensorMap &xmap, const CUtensorMap &wmap, const DgArgs &a, int64_t tiles, cudaStream_t stream) {
+    if (shape.cg == 2) return dg_launch<256, 2>(ctx, xmap, wmap, a, tiles, stream);
+    return shape.bn == 256 ? dg_launch<256, 1>(ctx, xmap, wmap, a, tiles, stream) : dg_launch<128, 1>(ctx, xmap, wmap, a, tiles, stream);
 }
 
 // The GEMM alone: w_bf16 is a bf16 [n, k] weight in device memory (16-byte aligned). h_out: see launch_gemm_dense_pairs.
@@ -559,21 +640,12 @@ static nnq_status dense_bf16(nnq_ctx *ctx, const void *w_bf16, const TcArgs &a, 
     CUtensorMap xmap, wmap;
     memset(&xmap, 0, sizeof(xmap));
     memset(&wmap, 0, sizeof(wmap));
-    const int64_t m_tiles = (a.m + kDgBM - 1) / kDgBM;
-    const int bn = dg_pick_bn(ctx, m_tiles, a.n);
-    if (!make_map(a.x, a.m, a.k, kDgBM, &xmap) || !make_map(w_bf16, a.n, a.k, bn, &wmap))
+    const DgShape shape = dg_pick(ctx, a.m, a.n);
+    if (!make_map(a.x, a.m, a.k, kDgBM, &xmap) || !make_map(w_bf16, a.n, a.k, shape.bn / shape.cg, &wmap))
         return fail(ctx, NNQ_ERR_DISPATCH_FAILED, "tensor map creation failed");
-    nnq_status s = dg_configure(ctx, bn);
-    if (s != NNQ_OK) return s;
-    const int smem_bytes = kDgStages * dg_stage_bytes(bn) + 1024;
-    const int64_t tiles = m_tiles * ((a.n + bn - 1) / bn);
-    const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
-    if (bn == 256)
-        gemm_dense_kernel<256><<<grid, kDgThreads, smem_bytes, stream>>>(xmap, wmap, a.bias, a.y, (int)a.m, (int)a.n, (int)a.k, a.y_dt, ctx->d_status, nullptr, 0, h_out, INFINITY, gate_kind);
-    else
-        gemm_dense_kernel<128><<<grid, kDgThreads, smem_bytes, stream>>>(xmap, wmap, a.bias, a.y, (int)a.m, (int)a.n, (int)a.k, a.y_dt, ctx->d_status, nullptr, 0, h_out, INFINITY, gate_kind);
-    ctx->launches++;
-    return check_cuda(ctx, cudaGetLastError(), "bf16 GEMM launch");
+    const DgArgs d = {a.bias, a.y, (int)a.m, (int)a.n, (int)a.k, a.y_dt, nullptr, 0, h_out, INFINITY, gate_kind};
+    const int64_t rows = kDgBM * shape.cg, tiles = (a.m + rows - 1) / rows * ((a.n + shape.bn - 1) / shape.bn);
+    return dg_launch_shape(ctx, shape, xmap, wmap, d, tiles, stream);
 }
 
 nnq_status launch_gemm_dense_bf16(nnq_ctx *ctx, const void *w_bf16, const TcArgs &a, cudaStream_t stream) { return dense_bf16(ctx, w_bf16, a, nullptr, 0, stream); }
@@ -647,21 +719,11 @@ nnq_status launch_gemm_dense_grouped(nnq_ctx *ctx, const TcGroupArgs &g, cudaStr
     CUtensorMap xmap, wmap;
     memset(&xmap, 0, sizeof(xmap));
     memset(&wmap, 0, sizeof(wmap));
-    // row tiles of all experts: at most rows / 128 + one ragged tile per expert
-    const int bn = dg_pick_bn(ctx, g.rows_upper / kDgBM + g.experts, g.n);
-    if (!make_map(g.x_bf16, g.rows_upper, g.k, kDgBM, &xmap) || !make_map(w_bf16, (int64_t)g.experts * g.n, g.k, bn, &wmap))
+    const DgShape shape = dg_pick_grouped(ctx, g.rows_upper, g.experts, g.n);
+    if (!make_map(g.x_bf16, g.rows_upper, g.k, kDgBM, &xmap) || !make_map(w_bf16, (int64_t)g.experts * g.n, g.k, shape.bn / shape.cg, &wmap))
         return fail(ctx, NNQ_ERR_DISPATCH_FAILED, "tensor map creation failed");
-    s = dg_configure(ctx, bn);
-    if (s != NNQ_OK) return s;
-    const int smem_bytes = kDgStages * dg_stage_bytes(bn) + 1024;
-    if (bn == 256)
-        gemm_dense_kernel<256><<<ctx->sm_count, kDgThreads, smem_bytes, stream>>>(xmap, wmap, g.bias, g.y, (int)g.rows_upper, (int)g.n, (int)g.k, NNQ_F32,
-                                                                                  ctx->d_status, g.offsets, g.experts, fuse ? g.h_out : nullptr, g.swiglu_limit, NNQ_ACT_SILU);
-    else
-        gemm_dense_kernel<128><<<ctx->sm_count, kDgThreads, smem_bytes, stream>>>(xmap, wmap, g.bias, g.y, (int)g.rows_upper, (int)g.n, (int)g.k, NNQ_F32,
-                                                                                  ctx->d_status, g.offsets, g.experts, fuse ? g.h_out : nullptr, g.swiglu_limit, NNQ_ACT_SILU);
-    ctx->launches++;
-    return check_cuda(ctx, cudaGetLastError(), "grouped bf16 GEMM launch");
+    const DgArgs d = {g.bias, g.y, (int)g.rows_upper, (int)g.n, (int)g.k, NNQ_F32, g.offsets, g.experts, fuse ? g.h_out : nullptr, g.swiglu_limit, NNQ_ACT_SILU};
+    return dg_launch_shape(ctx, shape, xmap, wmap, d, ctx->sm_count, stream);   // (the number of tiles is known on the device only)
 }
 
 }  // namespace nnq
