@@ -397,6 +397,14 @@ static nnq_status linear_checked(nnq_ctx *ctx, const nnq_weight *w, const void *
     return NNQ_OK;
 }
 
+// Rows that the product with the weights in tensor memory takes: from where the token-column kernel's two passes end (they
+// round no weight) up to 512 bf16 rows, above which decoding the weight once pays (Q4_K 12288 x 4096: 66 us here against 73 at
+// 512 rows, 130 against 109 at 1024); f32 rows have no such path and stay.
+static bool takes_gemm_ts(const nnq_ctx *ctx, const nnq_weight *w, int64_t m, int x_dt) {
+    if ((ctx->path != NNQ_PATH_AUTO && ctx->path != NNQ_PATH_TENSOR) || !gemm_ts_supported(w, m)) return false;
+    return m > (x_dt == NNQ_BF16 ? 32 : 16) && (x_dt == NNQ_F32 || m <= 512);
+}
+
 static nnq_status linear_dispatch(nnq_ctx *ctx, const nnq_weight *w, const void *x_dev, nnq_dtype x_dt,
                                   int64_t m, const float *bias_dev, void *y_dev, nnq_dtype y_dt,
                                   cudaStream_t stream) {
@@ -432,6 +440,10 @@ static nnq_status linear_dispatch(nnq_ctx *ctx, const nnq_weight *w, const void 
         return fail(ctx, NNQ_ERR_UNSUPPORTED, "tensor path needs K to be a multiple of 64 (K=%lld)", (long long)w->k);
     if (path == NNQ_PATH_TENSOR || (path == NNQ_PATH_AUTO && !skinny_ok && tc_ok && (m > 16 || (m >= 5 && x_dt == NNQ_BF16)))) {
         TcArgs a = {w->d_raw, w->d_scales, x_dev, bias_dev, y_dev, m, w->n, w->k, w->fmt, x_dt, y_dt};
+        if (takes_gemm_ts(ctx, w, m, x_dt)) {
+            SkinnyJob job = {w, x_dev, bias_dev, y_dev};
+            return launch_gemm_ts(ctx, &job, 1, x_dt, m, y_dt, stream);
+        }
         // hundreds of rows per weight row: decode once to bf16, then the plain GEMM
         if (gemm_dense_supported(ctx, w, m, x_dt)) return launch_gemm_dense(ctx, a, stream);
         return launch_gemm_tc(ctx, a, stream);
@@ -464,11 +476,13 @@ nnq_status nnq_linear_batch(nnq_ctx *ctx, int count, const nnq_weight *const *w,
     if (!ctx) return NNQ_ERR_INVALID_ARG;
     if (count < 0 || (count && (!w || !x_dev || !y_dev))) return fail(ctx, NNQ_ERR_INVALID_ARG, "bad batch arguments");
     nnq_status s;
+    bool all_ts = count > 1 && count <= kSkinnyMaxJobs;
     bool all_skinny = count > 0 && ctx->path != NNQ_PATH_GENERIC && ctx->path != NNQ_PATH_TENSOR && ctx->path != NNQ_PATH_F32;
     for (int i = 0; i < count; i++) {
         s = linear_checked(ctx, w[i], x_dev[i], x_dt, m, bias_dev ? bias_dev[i] : nullptr, y_dev[i], y_dt);
         if (s != NNQ_OK) return s;
         all_skinny = all_skinny && skinny_supported(w[i], m, x_dt) && w[i]->fmt == w[0]->fmt;
+        all_ts = all_ts && takes_gemm_ts(ctx, w[i], m, x_dt);
     }
     if ((s = set_device(ctx)) != NNQ_OK) return s;
     if (m == 0) return NNQ_OK;
@@ -476,6 +490,11 @@ nnq_status nnq_linear_batch(nnq_ctx *ctx, int count, const nnq_weight *const *w,
         SkinnyJob jobs[kSkinnyMaxJobs];
         for (int i = 0; i < count; i++) jobs[i] = {w[i], x_dev[i], bias_dev ? bias_dev[i] : nullptr, y_dev[i]};
         return launch_skinny(ctx, jobs, count, x_dt, m, y_dt, (cudaStream_t)stream);
+    }
+    if (all_ts) {
+        SkinnyJob jobs[kSkinnyMaxJobs];
+        for (int i = 0; i < count; i++) jobs[i] = {w[i], x_dev[i], bias_dev ? bias_dev[i] : nullptr, y_dev[i]};
+        return launch_gemm_ts(ctx, jobs, count, x_dt, m, y_dt, (cudaStream_t)stream);
     }
     for (int i = 0; i < count; i++) {
         s = linear_dispatch(ctx, w[i], x_dev[i], x_dt, m, bias_dev ? bias_dev[i] : nullptr, y_dev[i], y_dt,

@@ -439,28 +439,24 @@ static EncodeFn encode_fn() {
     }
     return fn;
 }
-static bool make_x_map(const TcArgs &a, CUtensorMap *map) {
+bool encode_map_2d(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64_t inner, int64_t rows, int64_t row_bytes, uint32_t box_inner,
+                   uint32_t box_rows, CUtensorMapSwizzle swizzle) {
     EncodeFn fn = encode_fn();
-    if (!fn || ((uintptr_t)a.x & 15u) || (a.k * 2) % 16) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)a.k, (cuuint64_t)a.m};
-    const cuuint64_t strides[1] = {(cuuint64_t)a.k * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kTcBK, 128u};
+    if (!fn || ((uintptr_t)base & 15u) || row_bytes % 16 || inner < 1 || rows < 1 || rows >= (1ll << 31)) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {box_inner, box_rows};
     const cuuint32_t estr[2] = {1u, 1u};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(a.x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return fn(map, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-
-// Tensor map of raw blocks as 32-bit words: [rows, K / 256 * unit_bytes / 4], boxes of 128 rows x sb units.
+static bool make_x_map(const TcArgs &a, CUtensorMap *map) {
+    return encode_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.x, a.k, a.m, a.k * 2, kTcBK, 128u, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+// Raw blocks as 32-bit words: [rows, K / 256 * unit_bytes / 4], boxes of 128 rows x sb units.
 static bool make_w_map(const void *w, int64_t rows, int64_t k, int unit_bytes, int sb, CUtensorMap *map) {
-    EncodeFn fn = encode_fn();
-    const cuuint64_t row_bytes = (cuuint64_t)(k / 256) * (cuuint64_t)unit_bytes;
-    if (!fn || ((uintptr_t)w & 15u) || rows < 1 || rows >= (1ll << 31)) return false;
-    const cuuint64_t dims[2] = {row_bytes / 4, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {row_bytes};
-    const cuuint32_t box[2] = {(cuuint32_t)(unit_bytes / 4 * sb), 128u};
-    const cuuint32_t estr[2] = {1u, 1u};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    const int64_t row_bytes = k / 256 * unit_bytes;
+    return encode_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, w, row_bytes / 4, rows, row_bytes, (uint32_t)(unit_bytes / 4 * sb), 128u, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 template <int FMT, int MT, typename XT, bool TMAX>

@@ -1,9 +1,11 @@
 // Tensor-core (tcgen05 / TMEM) prefill product: internal declarations.
 #pragma once
+#include <cuda.h>
 #include <cuda_bf16.h>
 
 #include "blocks.h"
 #include "nnq_internal.h"
+#include "skinny.h"
 
 namespace nnq {
 
@@ -51,6 +53,15 @@ nnq_status launch_gemm_tc_grouped(nnq_ctx *ctx, const TcGroupArgs &a, cudaStream
 // K must be a multiple of 64 (one 128-byte swizzle row of bf16 per stage).
 bool gemm_tc_supported(const nnq_weight *w, int64_t m);
 nnq_status launch_gemm_tc(nnq_ctx *ctx, const TcArgs &a, cudaStream_t stream);
+
+// gemm_ts.cu: the same product with the decoded weights as the operand in tensor memory, for the formats whose raw rows (or
+// tiled copies) it reads. Jobs of the same activations go out in one launch.
+bool gemm_ts_supported(const nnq_weight *w, int64_t m);
+nnq_status launch_gemm_ts(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int x_dt, int64_t m, int y_dt, cudaStream_t stream);
+// Tensor map of a [rows, inner] array (row pitch and inner extent whole 16-byte words), zero fill beyond its edges; false when
+// the driver entry point is missing or refuses the shape.
+bool encode_map_2d(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64_t inner, int64_t rows, int64_t row_bytes, uint32_t box_inner,
+                   uint32_t box_rows, CUtensorMapSwizzle swizzle);
 
 // Large prefill (M >= 256, bf16 activations, K a multiple of 64): decode the weight to bf16 in the
 // context's scratch, then a persistent TMA + tcgen05 GEMM (gemm_dense.cu).
