@@ -11,10 +11,11 @@ from nn_b200.formats import QuantFormat as Q
 from oracle import qwen3_ref as ref
 
 pytestmark = pytest.mark.gpu
-HIDDEN, FFN, VOCAB, EPS = 128, 192, 160, 1e-6
+FFN, VOCAB, EPS = 192, 160, 1e-6
 
 
-def _model(group, count):
+def _model(group, count, hidden=128, shift=0):
+    HIDDEN = hidden
     rng = np.random.default_rng(100 + group)
     kv = 2 if group < 8 else 1
     cfg = decoder.DecoderConfig(hidden=HIDDEN, n_heads=kv * group, n_kv_heads=kv, ffn=FFN, n_layers=2, vocab=VOCAB, max_seq=count + 3, act_dtype=api.BF16)
@@ -32,7 +33,8 @@ def _model(group, count):
         ns = [norm(HIDDEN), norm(HIDDEN), norm(128), norm(128)]
         dec.set_layer(i, *[w for w, _ in ws], *ns)
         model["layers"].append(([f for _, f in ws], ns))
-    embed = torch.from_numpy(rng.standard_normal((VOCAB, HIDDEN)).astype(np.float32)).to(torch.bfloat16).cuda()
+    embed = torch.empty(VOCAB * HIDDEN + shift, dtype=torch.bfloat16, device="cuda")[shift:].view(VOCAB, HIDDEN)   # (rows off their 8-byte boundaries)
+    embed.copy_(torch.from_numpy(rng.standard_normal((VOCAB, HIDDEN)).astype(np.float32)))
     head, model["head"] = weight(VOCAB, HIDDEN)
     model["embed"], model["final"] = embed.float().cpu().numpy(), norm(HIDDEN)
     dec.set_head(embed, model["final"], head)
@@ -73,5 +75,16 @@ def test_prompt_rows_of_every_group_size(group, count):
         got = np.concatenate([dec.extend(ids[a:e], a, list(range(e - a))) for a, e in ((0, cut), (cut, count)) if e > a])
         # both sides round the same five inputs of a layer's products to bf16: the bar of the decoder's bf16 tests
         assert np.max(np.abs(got - want)) <= 1e-2 * np.max(np.abs(want)), (cut, np.max(np.abs(got - want)) / np.max(np.abs(want)))
+    dec.backend.device_status()
+    dec.release()
+
+
+@pytest.mark.parametrize("hidden,shift", [(128, 1), (4096, 0), (4352, 0), (8192, 0), (8448, 0)])
+def test_norm_of_prompt_rows_of_every_width(hidden, shift):
+    """Row norms with the row in registers (up to 4096 and up to 8192 wide) and in two passes (wider, or an odd table)."""
+    dec, model = _model(2, 9, hidden, shift)
+    ids = np.random.default_rng(hidden).integers(0, VOCAB, 9)
+    want, got = _forward(model, ids), dec.extend(ids, 0, list(range(9)))
+    assert np.max(np.abs(got - want)) <= 1e-2 * np.max(np.abs(want)), np.max(np.abs(got - want)) / np.max(np.abs(want))
     dec.backend.device_status()
     dec.release()
