@@ -260,3 +260,24 @@ def test_gptq_shape_errors():
         gptq.load_gptq_linear(_words(np.zeros((1, 8), np.uint32)), torch.ones(1, 16), _words(np.zeros((1, 1), np.uint32)), None, 8)
     with pytest.raises(api.RankMismatch):
         gptq.unpack_gptq_qweight(_words(np.zeros(8, np.uint32)))
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("n,k,g,zp_max", [(16, 128, 128, 100), (33, 2048, 256, 2), (50, 1152, 64, 100), (17, 96, 32, 100), (130, 1024, 128, 101), (40, 640, 32, 7)])
+def test_int4_products_of_bf16_rows(n, k, g, zp_max, m):
+    """Codes as exact bf16 integers on the tensor cores up to a zero point of 100, f32 decode above: steps of one, two and four
+    words, fewer steps than warps, ragged rows, one and two column groups. f32 sums of exact products: K roundings of 2^-24."""
+    rng = np.random.default_rng(n + k + m)
+    codes = rng.integers(0, 256, n * k // 2, dtype=np.uint8)
+    scale = ((rng.random(n * (k // g)) + 0.5) * 0.01).astype(f32)
+    zp = rng.integers(-zp_max, zp_max + 1, n * (k // g)).astype(np.int32)
+    zp[0] = zp_max
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(f32)).to(torch.bfloat16)
+    qt = wq.QuantizedTensor(torch.from_numpy(codes).to(DEV), torch.from_numpy(scale).to(DEV), torch.from_numpy(zp).to(DEV), _cfg(4, g, False), [n, k])
+    y = wq.quantized_matmul(x.to(DEV), qt).double().cpu().numpy()
+    q = np.stack([codes & 15, codes >> 4], -1).reshape(n, k).astype(np.int64)
+    q = np.where(q > 7, q - 16, q)
+    w = (q - np.repeat(zp, g).reshape(n, k)) * np.repeat(scale, g).reshape(n, k).astype(np.float64)
+    x64 = x.double().numpy()
+    assert np.all(np.abs(y - x64 @ w.T) <= (k + 4) * 2.0 ** -24 * (np.abs(x64) @ np.abs(w).T))
+    qt.release()
