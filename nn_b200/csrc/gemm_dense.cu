@@ -145,8 +145,9 @@ dequant_bf16_kernel(const uint8_t *__restrict__ src, const uint8_t *__restrict__
 }
 
 // nn-gptoss expert tensors [E, K, N] (MXFP4, 32-weight blocks along N, the even column in the high
-// nibble) -> bf16 [E, N, K]: a CTA turns a 64 x 64 tile through shared memory. Reads are 16 bytes per
-// thread (one block), writes 128 contiguous bytes per output row. half_rows > 0 interleaves the output
+// nibble) -> bf16 [E, N, K]: a CTA turns a 64 x 64 tile through shared memory. Reads are whole sectors
+// (32 bytes of a k row), writes 128 contiguous bytes per output row. Bound by the decode, which looks four magnitudes up at a
+// time and stores pairs of k: the 4096-token block of 32 experts of 2880, one code at a time / this: 1.84 / 1.76 ms. half_rows > 0 interleaves the output
 // rows of every expert (row j -> 2j, row half_rows + j -> 2j + 1), as the fused SwiGLU epilogue wants.
 constexpr int kKnTile = 64;
 __global__ void __launch_bounds__(128)
@@ -154,26 +155,31 @@ dequant_kn_bf16_kernel(const uint8_t *__restrict__ data, const uint8_t *__restri
                        int K, int N, int half_rows) {
     __shared__ __align__(16) uint16_t tile[kKnTile][kKnTile + 8];   // [n][k]; 144-byte rows keep 16-byte reads aligned
     const int e = blockIdx.z, k0 = blockIdx.y * kKnTile, n0 = blockIdx.x * kKnTile;
-    const int kk = threadIdx.x & 63, blk = threadIdx.x >> 6;          // this thread's k row and which 32 of the 64 columns
-    const size_t row = (size_t)e * K + k0 + kk;
-    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(data + row * (size_t)(N / 2) + n0 / 2 + blk * 16));
-    const uint32_t ex = __ldg(scales + row * (size_t)(N / 32) + n0 / 32 + blk);
-    const bool direct = ex >= 1u && ex <= 251u;
-    const uint32_t base = (ex - 1u) << 7;
-    const float scale = mx_scale_gptoss(ex);
-    auto one = [&](uint32_t nib) -> uint16_t {
-        if (direct) return (uint16_t)mx_bf16_one(nib, base);
-        return __bfloat16_as_ushort(__float2bfloat16_rn(e2m1_value(nib, scale)));
-    };
-    const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+    // this thread's pair of k rows and 16 of the 64 columns: it makes the pairs (k, k + 1) that lie side by side in the copy
+    const int pair = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const size_t row = (size_t)e * K + k0 + 2 * pair;
+    const uint2 qa = __ldg(reinterpret_cast<const uint2 *>(data + row * (size_t)(N / 2) + n0 / 2 + part * 8));
+    const uint2 qb = __ldg(reinterpret_cast<const uint2 *>(data + (row + 1) * (size_t)(N / 2) + n0 / 2 + part * 8));
+    const uint32_t ea = __ldg(scales + row * (size_t)(N / 32) + n0 / 32 + (part >> 1)), eb = __ldg(scales + (row + 1) * (size_t)(N / 32) + n0 / 32 + (part >> 1));
+    // E2M1 magnitudes as the two bytes of a bf16 (0, .5, 1, 1.5, 2, 3, 4, 6), four per table look-up; the scale 2^(e - 127)
+    // (e = 0: 2^-126) is an exact bf16 factor, e = 255 infinity
+    const uint32_t scale = max(ea << 7, 0x80u) | (max(eb << 7, 0x80u) << 16);
+    const uint32_t wa[2] = {qa.x, qa.y}, wb[2] = {qb.x, qb.y};
 #pragma unroll
-    for (int v = 0; v < 4; v++) {
+    for (int v = 0; v < 2; v++) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t byte = (qw[v] >> (8 * i)) & 0xFFu;
-            const int col = blk * 32 + v * 8 + i * 2;
-            tile[col][kk] = one(byte >> 4);
-            tile[col + 1][kk] = one(byte & 15u);
+        for (int h = 0; h < 2; h++) {   // two bytes: columns 8 v + 4 h .. + 3, the even one of a byte in its high nibble
+            const uint32_t a = wa[v] >> (16 * h), b = wb[v] >> (16 * h), sa = a & 0x7777u, sb = b & 0x7777u;
+            const uint32_t la = __byte_perm(0xC0800000u, 0xC0804000u, sa), ha = __byte_perm(0x3F3F3F00u, 0x40404040u, sa);
+            const uint32_t lb = __byte_perm(0xC0800000u, 0xC0804000u, sb), hb = __byte_perm(0x3F3F3F00u, 0x40404040u, sb);
+            const uint32_t a01 = __byte_perm(la, ha, 0x5140), a23 = __byte_perm(la, ha, 0x7362), b01 = __byte_perm(lb, hb, 0x5140), b23 = __byte_perm(lb, hb, 0x7362);
+            const uint32_t m[4] = {__byte_perm(a01, b01, 0x5410), __byte_perm(a01, b01, 0x7632), __byte_perm(a23, b23, 0x5410), __byte_perm(a23, b23, 0x7632)};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {   // nibble i of the two bytes is column i ^ 1
+                uint32_t u = m[i] | ((a << (12 - 4 * i)) & 0x8000u) | ((b << (28 - 4 * i)) & 0x80000000u);
+                const __nv_bfloat162 z = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&u), *reinterpret_cast<const __nv_bfloat162 *>(&scale));
+                *reinterpret_cast<__nv_bfloat162 *>(&tile[part * 16 + 8 * v + 4 * h + (i ^ 1)][2 * pair]) = z;
+            }
         }
     }
     __syncthreads();
