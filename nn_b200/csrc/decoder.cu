@@ -60,6 +60,7 @@ struct nnq_decoder {
     float *pf_h, *pf_delta, *pf_q, *pf_k, *pf_v, *pf_qrot, *pf_g, *pf_u;
     void *pf_xn, *pf_attn, *pf_mid;
     int *pf_tokens;
+    uint2 *pf_top;              // largest keys and values of every 64 positions, [lkv, max_seq / 64] (attn_tc.cu)
     int *pf_want;               // rows of a block whose logits are asked for, [pf_rows]
     float *d_want_logits;       // [kWantRows, vocab], allocated by the first nnq_decoder_extend that asks for any
     int embed_ld, xn_ld;        // row strides of the embedding table and of the normed rows
@@ -545,12 +546,18 @@ dec_qk_rope_rows_kernel(const float *__restrict__ q, const float *__restrict__ k
 // memory), so that a key / value row is read once per R rows; row r sees keys 0 .. pos0 + r (the mask
 // of the reference's prompt pass: crates/nn-core/src/layers/attention/sdpa.rs:118-141). Same
 // batch-of-32-keys scheme as the decode kernel, normalised output written directly.
+// top: not NULL behind the tensor-core kernel, which leaves the kv heads that hold an infinity or a NaN to this one.
 template <int G, int R>
 __global__ void __launch_bounds__(32)
 dec_attn_rows_kernel(const float *__restrict__ qrot, const float *__restrict__ kcache, const float *__restrict__ vcache, int pos0,
-                     int n, float scale, void *__restrict__ out, int act_dt, int n_heads, int hd, int max_seq) {
+                     int n, float scale, void *__restrict__ out, int act_dt, int n_heads, int hd, int max_seq, const uint2 *top, int tiles) {
     constexpr int P = G * R;   // pair p = r * G + g
     __shared__ __align__(16) float qs[P][128];
+    pdl_prologue();
+    if (top) {
+        const uint2 t = attn_largest(top + (size_t)blockIdx.x * tiles, tiles);
+        if (max(t.x, t.y) < kNotFinite) return;
+    }
     const int kvh = blockIdx.x, r0 = blockIdx.y * R, lane = threadIdx.x;
     const int rows = min(R, n - r0);
     const int jmax = pos0 + r0 + rows;   // keys the last row of this block sees
@@ -1567,9 +1574,11 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         else
             dec_qk_rope_rows_kernel<<<dim3(lh + 2 * lkv, n), hd, 0, st>>>(d->pf_q, d->pf_k, d->pf_v, L.q_norm, L.k_norm, d->d_cos, d->d_sin, pos0,
                                                                      c.rms_eps, d->pf_qrot, kc, vc, lh, lkv, hd, c.max_seq);
-        // On the tensor cores from 32 query vectors per key / value head on (attn_tc.cu: every operand as two bf16 terms).
-        // Eight layers of the Qwen3-8B shape over a 2048-token prompt: 21.5 ms on the f32 kernel below, 2.6 ms there (prompt pass 32.0 -> 13.1 ms).
-        // f32 decoders keep f32 products.
+        // bf16 decoders: on the tensor cores (attn_tc.cu, two f16 terms per operand) from 32 query vectors per key / value head and
+        // 64 keys on. Its three launches take 23 us on the fewest rows and keys, the f32 kernel 0.42 us more per key: in us, f32 /
+        // tensor cores, 16.9 / 24.6 at 32 rows, 31.1 / 25.0 at 64, 37.1 / 26.9 at 8 rows behind 64, 2328 / 287 at 2048 rows of the
+        // Qwen3-8B shape. f32 decoders keep f32 products, and so do the kv heads with an infinity or a NaN: which other rows
+        // those reach stays as in the f32 kernel.
         WindowAttn wa = {};
         wa.span = {n, pos0, nullptr};
         wa.heads = lh;
@@ -1583,18 +1592,17 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         wa.ffn.act = d->pf_attn;
         wa.ffn.act_dt = d->act_dt;
         wa.ffn.out_k = lh * hd;
-        if (attn_tc_supported(wa)) {
-            if ((s = launch_attn_tc(ctx, wa, st)) != NNQ_OK) return s;
-        } else {
-            // 16 query vectors per warp: R = 16 / G rows share each key / value row
-            ctx->launches++;
-            switch (group) {
-                case 1: dec_attn_rows_kernel<1, 16><<<dim3(lkv, (n + 15) / 16), 32, 0, st>>>(d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq); break;
-                case 2: dec_attn_rows_kernel<2, 8><<<dim3(lkv, (n + 7) / 8), 32, 0, st>>>(d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq); break;
-                case 4: dec_attn_rows_kernel<4, 4><<<dim3(lkv, (n + 3) / 4), 32, 0, st>>>(d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq); break;
-                case 8: dec_attn_rows_kernel<8, 2><<<dim3(lkv, (n + 1) / 2), 32, 0, st>>>(d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq); break;
-                default: return fail(ctx, NNQ_ERR_UNSUPPORTED, "query heads per key/value head must be 1, 2, 4 or 8");
-            }
+        const bool tc = attn_tc_supported(wa) && pos0 + n >= 64;
+        if (tc && (s = launch_attn_tc_scaled(ctx, wa, d->pf_top, st)) != NNQ_OK) return s;
+        const uint2 *top = tc ? d->pf_top : nullptr;
+        const int tiles = attn_tiles(pos0 + n);
+        // 16 query vectors per warp: R = 16 / G rows share each key / value row
+        switch (group) {
+            case 1: launch_pdl(dec_attn_rows_kernel<1, 16>, dim3(lkv, (n + 15) / 16), dim3(32), st, d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq, top, tiles); break;
+            case 2: launch_pdl(dec_attn_rows_kernel<2, 8>, dim3(lkv, (n + 7) / 8), dim3(32), st, d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq, top, tiles); break;
+            case 4: launch_pdl(dec_attn_rows_kernel<4, 4>, dim3(lkv, (n + 3) / 4), dim3(32), st, d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq, top, tiles); break;
+            case 8: launch_pdl(dec_attn_rows_kernel<8, 2>, dim3(lkv, (n + 1) / 2), dim3(32), st, d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq, top, tiles); break;
+            default: return fail(ctx, NNQ_ERR_UNSUPPORTED, "query heads per key/value head must be 1, 2, 4 or 8");
         }
         s = d->comm ? nnq_comm_linear(d->comm, L.o, d->pf_attn, adt, n, nullptr, d->pf_delta, NNQ_F32, st)
                     : nnq_linear(ctx, L.o, d->pf_attn, adt, n, nullptr, d->pf_delta, NNQ_F32, st);
@@ -1613,7 +1621,7 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         s = d->comm ? nnq_comm_linear(d->comm, L.down, d->pf_mid, adt, n, nullptr, d->pf_delta, NNQ_F32, st)
                     : nnq_linear(ctx, L.down, d->pf_mid, adt, n, nullptr, d->pf_delta, NNQ_F32, st);
         if (s != NNQ_OK) return s;
-        ctx->launches += 4;
+        ctx->launches += 5;
     }
     return NNQ_OK;
 }
@@ -1697,6 +1705,7 @@ static nnq_status row_buffers(nnq_decoder *d, int *rows_max) {
         if (s == NNQ_OK) s = dev_alloc(ctx, &d->pf_mid, R * lffn * es, "prompt buffer");
         if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_tokens, (R + 1) * 4, "prompt buffer");
         if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_want, R * 4, "prompt buffer");
+        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_top, (size_t)d->lkv * attn_tiles(c.max_seq) * sizeof(uint2), "prompt buffer");
         if (s != NNQ_OK) return s;
     }
     return NNQ_OK;
@@ -1844,7 +1853,7 @@ void nnq_decoder_destroy(nnq_decoder *d) {
     cudaFree(d->b_h2); cudaFree(d->b_proj); cudaFree(d->b_q); cudaFree(d->b_k); cudaFree(d->b_a); cudaFree(d->b_o); cudaFree(d->b_vfirst); cudaFree(d->b_act);
     cudaFree(d->b_cq); cudaFree(d->b_lin_c); cudaFree(d->b_lin_r); cudaFree(d->b_kv); cudaFree(d->b_q2); cudaFree(d->b_qrot);
     cudaFree(d->b_kfull); cudaFree(d->b_vfull); cudaFree(d->b_qlat); cudaFree(d->final_bias);
-    cudaFree(d->pf_want); cudaFree(d->d_want_logits);
+    cudaFree(d->pf_want); cudaFree(d->pf_top); cudaFree(d->d_want_logits);
     cudaFree(d->d_final_norm); cudaFree(d->d_cos); cudaFree(d->d_sin); cudaFree(d->d_kcache); cudaFree(d->d_vcache);
     cudaFree(d->d_h); cudaFree(d->d_delta); cudaFree(d->d_q); cudaFree(d->d_k); cudaFree(d->d_v); cudaFree(d->d_qrot);
     cudaFree(d->d_g); cudaFree(d->d_u); cudaFree(d->d_logits); cudaFree(d->d_part); cudaFree(d->d_arrived); cudaFree(d->d_xn); cudaFree(d->d_attn);

@@ -45,4 +45,17 @@ __device__ __forceinline__ float gelu_tanh_f32(float x) {
 // kind: nnq_gate_act
 __device__ __forceinline__ float gate_act(int kind, float x) { return kind == NNQ_ACT_GELU_TANH ? gelu_tanh_f32(x) : silu_f32(x); }
 
+// Bits of the largest absolute key and value of some tiles, for every lane of a warp; from kNotFinite on there is an infinity
+// or a NaN among them.
+constexpr uint32_t kNotFinite = 0x7F800000u;
+__device__ __forceinline__ uint2 attn_largest(const uint2 *top, int tiles) {
+    uint2 m = make_uint2(0, 0);
+    for (int i = threadIdx.x & 31; i < tiles; i += 32) {
+        const uint2 t = top[i];
+        m.x = max(m.x, t.x);
+        m.y = max(m.y, t.y);
+    }
+    return make_uint2(__reduce_max_sync(0xFFFFFFFFu, m.x), __reduce_max_sync(0xFFFFFFFFu, m.y));
+}
+
 }  // namespace nnq

@@ -7,6 +7,7 @@ import pytest
 torch = pytest.importorskip("torch")
 
 from nn_b200 import api, decoder
+from nn_b200 import formats as F
 from nn_b200.formats import QuantFormat as Q
 from oracle import qwen3_ref as ref
 
@@ -36,6 +37,7 @@ def _model(group, count, hidden=128, shift=0):
     embed = torch.empty(VOCAB * HIDDEN + shift, dtype=torch.bfloat16, device="cuda")[shift:].view(VOCAB, HIDDEN)   # (rows off their 8-byte boundaries)
     embed.copy_(torch.from_numpy(rng.standard_normal((VOCAB, HIDDEN)).astype(np.float32)))
     head, model["head"] = weight(VOCAB, HIDDEN)
+    model["head_weight"] = head
     model["embed"], model["final"] = embed.float().cpu().numpy(), norm(HIDDEN)
     dec.set_head(embed, model["final"], head)
     return dec, model
@@ -86,5 +88,65 @@ def test_norm_of_prompt_rows_of_every_width(hidden, shift):
     ids = np.random.default_rng(hidden).integers(0, VOCAB, 9)
     want, got = _forward(model, ids), dec.extend(ids, 0, list(range(9)))
     assert np.max(np.abs(got - want)) <= 1e-2 * np.max(np.abs(want)), np.max(np.abs(got - want)) / np.max(np.abs(want))
+    dec.backend.device_status()
+    dec.release()
+
+
+def test_a_value_that_is_no_number_reaches_no_earlier_block_of_rows():
+    """The f32 kernel multiplies masked values of its own block of 16 / group rows with zero and no others: rows in front of the
+    block that holds a NaN are those of a prompt without it, also where the tensor cores take 32 and more of them at once."""
+    group, count, at = 4, 100, 70
+    dec, model = _model(group, count)
+    ids = np.random.default_rng(5).integers(0, VOCAB - 1, count)
+    ids[at] = VOCAB - 1
+    want = _forward(model, ids)
+    first = at // (16 // group) * (16 // group)
+    bad = model["embed"].copy()
+    bad[VOCAB - 1] = np.nan
+    dec.set_head(torch.from_numpy(bad).to(torch.bfloat16).cuda(), model["final"], model["head_weight"])
+    got = dec.extend(ids, 0, list(range(count)))
+    assert np.all(np.isnan(got[at:]))
+    assert np.max(np.abs(got[:first] - want[:first])) <= 1e-2 * np.max(np.abs(want[:first]))
+    dec.backend.device_status()
+    dec.release()
+
+
+def test_values_that_cancel_keep_their_f32_digits():
+    """Keys of zero give every visible value the same weight; two tokens whose values are opposite but for 2^-15 of them alternate,
+    so that every second row's mean consists of the values' last bits. Two f16 terms hold a value to 2^-23, and each of the up to
+    12 sums of a tile is rounded at 2^-23 of the values at most: 2^-19 of the mean magnitude in all (two bf16 terms would be up to
+    2^-17 off). The output is rounded to bf16 twice on its way to the logits."""
+    rng = np.random.default_rng(3)
+    count, hidden, half = 100, 128, 64
+    cfg = decoder.DecoderConfig(hidden=hidden, n_heads=4, n_kv_heads=1, ffn=64, n_layers=1, vocab=VOCAB, max_seq=count, act_dtype=api.BF16)
+    b = api.gpu_backend()
+    dec = decoder.Decoder(b, cfg)
+
+    def weight(w):
+        return api.DeviceWeight.from_device(b, Q.BF16_DENSE, torch.from_numpy(w.astype(np.float32)).to(torch.bfloat16).cuda().view(torch.uint8).reshape(-1), *w.shape)
+
+    pick = np.zeros((hidden, 512))        # rows 64 .. 127 of the model take the first 64 dimensions of head 0
+    pick[half + np.arange(half), np.arange(half)] = 1
+    ws = [rng.standard_normal((512, hidden)), rng.standard_normal((128, hidden)), rng.standard_normal((128, hidden)), pick,
+          np.zeros((64, hidden)), np.zeros((64, hidden)), np.zeros((hidden, 64))]
+    dec.set_layer(0, *[weight(w) for w in ws], np.ones(hidden, np.float32), np.ones(hidden, np.float32), np.ones(128, np.float32), np.zeros(128, np.float32))
+    embed = np.zeros((VOCAB, hidden), np.float32)
+    embed[0, :half] = F.bf16_bits_to_f32(F.to_bf16_bits(rng.standard_normal(half).astype(np.float32)))
+    embed[0, 0] = 2.0 ** -5
+    embed[1] = -embed[0]
+    embed[1, 0] *= 1 + 2.0 ** -6
+    head = np.zeros((VOCAB, hidden))
+    head[np.arange(half), half + np.arange(half)] = 1
+    dec.set_head(torch.from_numpy(embed).to(torch.bfloat16).cuda(), np.ones(hidden, np.float32), weight(head))
+    ids = np.arange(count) % 2
+    got = dec.extend(ids, 0, list(range(count)))[:, :half].astype(np.float64)
+    v = dec.buffers()[1][0, 0, :count, :half].cpu().numpy().astype(np.float64)
+    mean = np.cumsum(v, 0) / np.arange(1, count + 1)[:, None]
+    h = embed[ids].astype(np.float64)
+    rms = np.sqrt((np.sum(h * h, 1) + np.sum(mean * mean, 1)) / hidden + cfg.rms_eps)
+    even = np.arange(1, count, 2)
+    assert np.max(np.abs(mean[even])) < 2.0 ** -12 * np.max(np.abs(v))
+    bound = 2.0 ** -19 * np.mean(np.abs(v), 0) + 2.0 ** -7 * np.abs(mean)
+    assert np.all((np.abs(got * rms[:, None] - mean) <= bound)[even]), np.max((np.abs(got * rms[:, None] - mean) / bound)[even])
     dec.backend.device_status()
     dec.release()
