@@ -19,6 +19,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 
 #include "blocks.h"
@@ -55,8 +56,9 @@ struct nnq_decoder {
     int head_rows, head_row0;   // rows of the vocabulary projection held by this rank and the first of them
     long long host_pos;         // position of the next step as far as the host knows it (-1: unknown)
     // prompt pass: row-major [rows, width] versions of the step's buffers, allocated by the first
-    // nnq_decoder_prefill call (pf_rows rows)
+    // nnq_decoder_prefill call (pf_rows rows) and again by the first with a long prompt
     int pf_rows;
+    void *pf_mem;               // Qwen3 layers: the one allocation they lie in
     float *pf_h, *pf_delta, *pf_q, *pf_k, *pf_v, *pf_qrot, *pf_g, *pf_u;
     void *pf_xn, *pf_attn, *pf_mid;
     int *pf_tokens;
@@ -1672,42 +1674,62 @@ static nnq_status check_tokens(nnq_decoder *d, const int32_t *tokens_host, int c
     return NNQ_OK;
 }
 
-// Rows that go through the layers together: bounded by the row buffers (allocated here for Qwen3 layers)
-// and, with tensor parallelism, by what one exchange carries.
-static nnq_status row_buffers(nnq_decoder *d, int *rows_max) {
+// The row buffers of Qwen3 layers for R rows, in one allocation: whole or not at all.
+static nnq_status alloc_row_buffers(nnq_decoder *d, size_t R) {
+    const nnq_decoder_config &c = d->cfg;
+    const size_t qdim = (size_t)d->lh * c.head_dim, kvdim = (size_t)d->lkv * c.head_dim, lffn = c.ffn / c.tp_world, es = d->act_dt == NNQ_F32 ? 4 : 2;
+    const struct {
+        void **p;
+        size_t bytes;
+    } part[] = {{(void **)&d->pf_h, R * c.hidden * 4}, {(void **)&d->pf_delta, R * c.hidden * 4}, {(void **)&d->pf_q, R * qdim * 4},
+                {(void **)&d->pf_k, R * kvdim * 4}, {(void **)&d->pf_v, R * kvdim * 4}, {(void **)&d->pf_qrot, R * qdim * 4},
+                {(void **)&d->pf_g, R * lffn * 4}, {(void **)&d->pf_u, R * lffn * 4}, {&d->pf_xn, R * c.hidden * es},
+                {&d->pf_attn, R * qdim * es}, {&d->pf_mid, R * lffn * es}, {(void **)&d->pf_tokens, (R + 1) * 4},
+                {(void **)&d->pf_want, R * 4}, {(void **)&d->pf_top, d->lkv * (size_t)attn_tiles(c.max_seq) * sizeof(uint2)}};
+    size_t total = 0;
+    for (const auto &q : part) total += (q.bytes + 255) / 256 * 256;
+    void *mem = nullptr;
+    nnq_status s = dev_alloc(d->ctx, &mem, total, "prompt buffers");
+    if (s != NNQ_OK) {
+        cudaFree(mem);
+        return s;
+    }
+    cudaFree(d->pf_mem);
+    d->pf_mem = mem;
+    d->pf_rows = (int)R;
+    uint8_t *at = (uint8_t *)mem;
+    for (const auto &q : part) {
+        *q.p = at;
+        at += (q.bytes + 255) / 256 * 256;
+    }
+    return NNQ_OK;
+}
+
+// Rows that go through the layers together: bounded by the row buffers (for Qwen3 layers allocated here, in steps of 1024 rows as
+// longer prompts come) and, with tensor parallelism, by what one exchange carries. Where larger buffers cannot be had, long
+// prompts go through in blocks of 1024 rows, or of what is there.
+static nnq_status row_buffers(nnq_decoder *d, int count, int *rows_max) {
     nnq_ctx *ctx = d->ctx;
     const nnq_decoder_config &c = d->cfg;
     nnq_status s = NNQ_OK;
-    *rows_max = d->blocks ? d->pf_rows : (c.max_seq < kPrefillRowsQwen3 ? c.max_seq : kPrefillRowsQwen3);
-    const int rows = *rows_max;
+    size_t fit = (size_t)1 << 31;
     if (d->comm) {
         CommView v;
         if ((s = comm_view(d->comm, &v)) != NNQ_OK) return s;
-        const size_t fit = v.slot_bytes / ((size_t)c.hidden * 4);
+        fit = v.slot_bytes / ((size_t)c.hidden * 4);
         if (fit < 1) return fail(ctx, NNQ_ERR_UNSUPPORTED, "communicator slots are smaller than one row of the hidden state");
-        if ((size_t)*rows_max > fit) *rows_max = (int)fit;
     }
-    const int qdim = d->lh * c.head_dim, kvdim = d->lkv * c.head_dim, lffn = d->blocks ? 0 : c.ffn / c.tp_world;
-    const size_t es = d->act_dt == NNQ_F32 ? 4 : 2;
-    if (!d->pf_h) {
-        d->pf_rows = rows;
-        const size_t R = rows;
-        s = dev_alloc(ctx, (void **)&d->pf_h, R * c.hidden * 4, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_delta, R * c.hidden * 4, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_q, R * qdim * 4, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_k, R * kvdim * 4, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_v, R * kvdim * 4, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_qrot, R * qdim * 4, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_g, R * lffn * 4, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_u, R * lffn * 4, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, &d->pf_xn, R * c.hidden * es, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, &d->pf_attn, R * qdim * es, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, &d->pf_mid, R * lffn * es, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_tokens, (R + 1) * 4, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_want, R * 4, "prompt buffer");
-        if (s == NNQ_OK) s = dev_alloc(ctx, (void **)&d->pf_top, (size_t)d->lkv * attn_tiles(c.max_seq) * sizeof(uint2), "prompt buffer");
-        if (s != NNQ_OK) return s;
+    if (!d->blocks) {
+        auto within = [&](int rows) { return (int)std::min<size_t>(std::min(rows, c.max_seq), fit); };
+        const int blocks = std::min((count - 1) / kPrefillRows + 1, kPrefillRowsQwen3 / kPrefillRows);
+        const int few = within(kPrefillRows), want = within(blocks * kPrefillRows);
+        if (want > d->pf_rows) {
+            s = alloc_row_buffers(d, want);
+            if (s != NNQ_OK && !d->comm && !d->pf_mem && want > few) s = alloc_row_buffers(d, few);
+            if (s != NNQ_OK && (d->comm || !d->pf_mem)) return s;   // (ranks have to agree on the blocks)
+        }
     }
+    *rows_max = (int)std::min<size_t>(d->pf_rows, fit);
     return NNQ_OK;
 }
 
@@ -1735,7 +1757,7 @@ nnq_status nnq_decoder_prefill(nnq_decoder *d, const int32_t *tokens_host, int c
     if ((s = check_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice")) != NNQ_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
     int rows_max = 0;
-    if ((s = row_buffers(d, &rows_max)) != NNQ_OK) return s;
+    if ((s = row_buffers(d, count, &rows_max)) != NNQ_OK) return s;
     d->host_pos = -1;   // until the call has gone through
     int n = 0;
     for (int c0 = 0; c0 < count; c0 += n) {
@@ -1776,7 +1798,7 @@ nnq_status nnq_decoder_extend(nnq_decoder *d, const int32_t *tokens_host, int co
         return s;
     }
     int rows_max = 0;
-    if ((s = row_buffers(d, &rows_max)) != NNQ_OK) return s;
+    if ((s = row_buffers(d, count, &rows_max)) != NNQ_OK) return s;
     if (n_want && !d->d_want_logits && (s = dev_alloc(ctx, (void **)&d->d_want_logits, (size_t)kWantRows * c.vocab * 4, "logits of wanted rows")) != NNQ_OK) return s;
     d->host_pos = -1;   // until the call has gone through
     int n = 0, w0 = 0;
@@ -1853,13 +1875,14 @@ void nnq_decoder_destroy(nnq_decoder *d) {
     cudaFree(d->b_h2); cudaFree(d->b_proj); cudaFree(d->b_q); cudaFree(d->b_k); cudaFree(d->b_a); cudaFree(d->b_o); cudaFree(d->b_vfirst); cudaFree(d->b_act);
     cudaFree(d->b_cq); cudaFree(d->b_lin_c); cudaFree(d->b_lin_r); cudaFree(d->b_kv); cudaFree(d->b_q2); cudaFree(d->b_qrot);
     cudaFree(d->b_kfull); cudaFree(d->b_vfull); cudaFree(d->b_qlat); cudaFree(d->final_bias);
-    cudaFree(d->pf_want); cudaFree(d->pf_top); cudaFree(d->d_want_logits);
+    cudaFree(d->pf_mem); cudaFree(d->d_want_logits);
     cudaFree(d->d_final_norm); cudaFree(d->d_cos); cudaFree(d->d_sin); cudaFree(d->d_kcache); cudaFree(d->d_vcache);
     cudaFree(d->d_h); cudaFree(d->d_delta); cudaFree(d->d_q); cudaFree(d->d_k); cudaFree(d->d_v); cudaFree(d->d_qrot);
     cudaFree(d->d_g); cudaFree(d->d_u); cudaFree(d->d_logits); cudaFree(d->d_part); cudaFree(d->d_arrived); cudaFree(d->d_xn); cudaFree(d->d_attn);
     cudaFree(d->d_mid); cudaFree(d->d_state); cudaFree(d->d_tokens);
-    cudaFree(d->pf_h); cudaFree(d->pf_delta); cudaFree(d->pf_q); cudaFree(d->pf_k); cudaFree(d->pf_v); cudaFree(d->pf_qrot);
-    cudaFree(d->pf_g); cudaFree(d->pf_u); cudaFree(d->pf_xn); cudaFree(d->pf_attn); cudaFree(d->pf_mid); cudaFree(d->pf_tokens);
+    if (!d->pf_mem) {   // of a block decoder
+        cudaFree(d->pf_h); cudaFree(d->pf_delta); cudaFree(d->pf_xn); cudaFree(d->pf_tokens); cudaFree(d->pf_want);
+    }
     cudaGetLastError();
     delete d;
 }

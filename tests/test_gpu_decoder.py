@@ -381,3 +381,55 @@ def test_decoder_argument_errors():
     with pytest.raises(api.TensorError):
         dec.reset(999, 0)   # token out of range
     dec.release()
+
+
+def test_prompt_buffers_that_cannot_be_had():
+    """Row buffers of about 0.2 MB per row: where those of 2048 rows do not fit, a long prompt goes through 1024 at a time; where
+    none fit the call fails, the next one too, and with memory given back it works."""
+    rng = np.random.default_rng(8)
+    hidden, ffn, heads, vocab = 128, 16384, 32, 128
+    b = api.gpu_backend()
+
+    def weight(n, k):
+        w = torch.from_numpy((rng.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32)).to(torch.bfloat16).cuda()
+        return api.DeviceWeight.from_device(b, Q.BF16_DENSE, w.view(torch.uint8).reshape(-1), n, k)
+
+    ws = [weight(n, k) for n, k in ((heads * 128, hidden), (512, hidden), (512, hidden), (hidden, heads * 128), (ffn, hidden), (ffn, hidden), (hidden, ffn))]
+    ones = np.ones(hidden, np.float32)
+    embed = torch.from_numpy(rng.standard_normal((vocab, hidden)).astype(np.float32)).to(torch.bfloat16).cuda()
+    head = weight(vocab, hidden)
+
+    def build():
+        cfg = decoder.DecoderConfig(hidden=hidden, n_heads=heads, n_kv_heads=4, ffn=ffn, n_layers=1, vocab=vocab, max_seq=4096, act_dtype=api.BF16)
+        d = decoder.Decoder(b, cfg)
+        d.set_layer(0, *ws, ones, ones, np.ones(128, np.float32), np.ones(128, np.float32))
+        d.set_head(embed, ones, head)
+        return d
+
+    ids = rng.integers(0, vocab, 1500)
+    few, decs = [1, 2, 3], [build() for _ in range(3)]
+    want, short = decs[0].extend(ids, 0, [1022, 1023, 1024, 1499]), decs[0].extend(few, 0, [2])
+    decs[0].release()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+
+    def fill(left):
+        return torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+
+    rest = fill(320 << 20)
+    got = decs[1].extend(ids, 0, [1022, 1023, 1024, 1499])
+    assert np.max(np.abs(got - want)) <= 1e-2 * np.max(np.abs(want))   # (sums of other tiles: the bar of the bf16 decoders)
+    del rest
+    torch.cuda.empty_cache()
+    rest = fill(120 << 20)
+    for _ in range(2):
+        with pytest.raises(api.BackendFailure) as e:
+            decs[2].extend(few, 0, [2])
+        assert e.value.kind == "OutOfMemory"
+    del rest
+    torch.cuda.empty_cache()
+    assert np.array_equal(decs[2].extend(few, 0, [2]), short)
+    assert np.max(np.abs(decs[2].extend(ids, 0, [1499]) - want[3:])) <= 1e-2 * np.max(np.abs(want))   # the buffers grow
+    b.device_status()
+    decs[1].release()
+    decs[2].release()
