@@ -583,6 +583,12 @@ bool gemm_ts_supported(const nnq_weight *w, int64_t m) {
     }
 }
 
+// Tokens of a tile at most. Q8_0's raw blocks leave room for two activation stages of 128 tokens, but the four warps that convert
+// f32 rows work on one each. Tiles of up to 128 / of up to 80 tokens, and the fused decode of gemm_tc.cu, in us: 12288 x 4096 at
+// 128 rows 82 / 55 / 69, at 256 187 / 95 / 108, at 1024 571 / 295 / 357; 4096 x 12288 at 512 rows 303 / 184 / 194; 1024 x 4096 at
+// 128 rows 18 / 11 / 16.
+static int ts_tile_tokens(int fmt, int x_dt) { return fmt == NNQ_Q8_0 && x_dt == NNQ_F32 ? 80 : kTsMaxN; }
+
 template <int FMT>
 static bool ts_w_map(const nnq_weight *w, CUtensorMap *map) {
     const bool mx = FMT == NNQ_MXFP4_SPLIT;
@@ -665,9 +671,10 @@ static nnq_status ts_run(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int x_d
     P.y_dt = y_dt;
     P.status = ctx->d_status;
     // tokens in tiles of equal size
-    const int64_t ttiles = (m + kTsMaxN - 1) / kTsMaxN;
-    P.nt = (int)(((m + ttiles - 1) / ttiles + 15) / 16 * 16);
     const bool f32x = x_dt == NNQ_F32;
+    const int most = ts_tile_tokens(FMT, x_dt);
+    const int64_t ttiles = (m + most - 1) / most;
+    P.nt = (int)(((m + ttiles - 1) / ttiles + 15) / 16 * 16);
     if (f32x) P.xf = static_cast<const float *>(jobs[0].x);
     else if (!encode_map_2d(&P.xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, jobs[0].x, k, m, 2 * k, 64, P.nt, CU_TENSOR_MAP_SWIZZLE_128B))
         return fail(ctx, NNQ_ERR_UNSUPPORTED, "tensor map of the activations");

@@ -80,3 +80,14 @@ def test_several_products_of_one_call():
         one = api.quantized_linear(xt[k], t, out_dtype=torch.float32)
         torch.testing.assert_close(y, one, rtol=0, atol=float(k * 2.0 ** -24 * (np.abs(_bf16(x[k])) @ np.abs(w64).T).max()))   # (K may be split otherwise)
         t.release()
+
+@pytest.mark.parametrize("m", [64, 80, 81, 128, 160, 161, 241])
+def test_q8_0_tiles_of_f32_rows(m):
+    """Up to 80 tokens per tile, tiles of equal size, the last one ragged."""
+    t, w64 = _weight(Q.Q8_0, 130, 1536, 17)
+    x = F.gen_activations(8, m, 1536, bf16=False)
+    y = api.quantized_linear(torch.from_numpy(x).cuda(), t)
+    torch.cuda.synchronize()
+    t.backend.device_status()
+    _check(y, x, w64, None, 1536)
+    t.release()
