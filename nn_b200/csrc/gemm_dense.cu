@@ -246,13 +246,12 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     constexpr int kDgBN = BN, kDgStageBytes = dg_stage_bytes(BN, CG), kDgStages = dg_stages(BN, CG), kDgRows = kDgBM * CG;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t bars[2 * kDgStages + 4];   // full[4], empty[4], acc_full[2], acc_empty[2]
+    __shared__ __align__(8) uint64_t bars[2 * kDgStages + 5];   // full, empty [kDgStages], acc_full[2], acc_empty[2], every MMA has ended
     __shared__ uint32_t tmem_base_s;
-    __shared__ int abort_s;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t full_s = smem_u32(bars), empty_s = full_s + 8 * kDgStages;
-    const uint32_t accf_s = empty_s + 8 * kDgStages, acce_s = accf_s + 16;
+    const uint32_t accf_s = empty_s + 8 * kDgStages, acce_s = accf_s + 16, done_s = acce_s + 16;
     const int rank = CG == 2 ? (int)cluster_rank() : 0;
     const int unit = blockIdx.x / CG, units = gridDim.x / CG;   // a unit multiplies one tile at a time
     __shared__ int tile_begin[kDgMaxGroups + 1], row_begin[kDgMaxGroups + 1];
@@ -297,7 +296,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
             mbar_init(accf_s + 8 * a, 1);
             mbar_init(acce_s + 8 * a, 4 * CG);
         }
-        abort_s = 0;
+        mbar_init(done_s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -348,6 +347,14 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                     }
                 }
             }
+            // The last use of every stage: this CTA's copies have landed and been read, and the arrivals on its barriers, which
+            // for the second CTA of a pair come from the first, are over. Behind a wait that ran out the stages may never be
+            // given back; the copies are still waited for (by the CTA whose barriers count them).
+            for (long long f = filled > kDgStages ? filled - kDgStages : 0; f < filled; f++) {
+                const uint32_t s = (uint32_t)(f % kDgStages), p = (uint32_t)(f / kDgStages) & 1u;
+                if (ok) ok = mbar_wait_fast(empty_s + 8 * s, p);
+                if (!ok && rank == 0) mbar_wait(full_s + 8 * s, p);
+            }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
@@ -389,6 +396,8 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                 if (ok && CG == 2) umma_commit_pair(accf_s + 8 * a);
                 else if (ok) umma_commit(accf_s + 8 * a);
             }
+            if (CG == 2) umma_commit_pair(done_s);   // also behind a wait that ran out
+            else umma_commit(done_s);
         }
     } else {
         // ---------------- epilogue ----------------
@@ -491,16 +500,10 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
             }
         }
     }
-    if (!ok) {
-        abort_s = 1;
-        atomicExch(status, 1);
-    }
+    if (!ok) atomicExch(status, 1);
     __syncthreads();
-    // with an aborted CTA, MMAs may still be in flight: give the last accumulator a bounded chance
-    if (warp == 1 && abort_s) {
-        mbar_wait(accf_s, 0);
-        mbar_wait(accf_s + 8, 0);
-    }
+    // all MMAs have ended (in an aborted CTA too): shared and tensor memory may be given back
+    if (warp == 1) mbar_wait(done_s, 0);
     // a CTA of a pair stays until the other one has no more use for its shared memory, barriers and tensor memory
     if (CG == 2) cluster_sync();
     if (warp == 1) {
