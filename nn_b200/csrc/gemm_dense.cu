@@ -581,16 +581,25 @@ nnq_status dense_scratch_reserve(nnq_ctx *ctx, int64_t n, int64_t k) {
     return NNQ_OK;
 }
 
-// Shape of a tile: its width and the CTAs that share it. Pairs with 256 x 256 tiles, or single CTAs with 128 x 128 tiles where
-// the large ones would leave more than half of the SMs without work. (4096 rows of the 32B shape, pair / single CTA with
-// 128 x 256: 25600 x 5120 696 / 731 us, 8192 x 5120 219 / 239, 5120 x 25600 802 / 853. 1024 x 4096 at 1024 rows, 256 x 128 by
-// a pair / 128 x 128 by a CTA: 25.6 / 22.8 us.)
+// Shape of a tile: its width and the CTAs that share it. Pair / single CTAs with 128 x 256 in us (waves of tiles in brackets):
+// - pairs with 256 x 256, whose waves are 10 to 18 % shorter from K = 4096 on and about 5 % at 1024: 25600 x 5120 at 4096 rows
+//   683 / 739 (22, 22), at 1300 rows 258 / 264 (9, 8), 151936 x 1024 at 2049 rows 572 / 577 (73, 69);
+// - single CTAs with 128 x 256 where those need fewer waves by more than that (ragged rows): 4096 x 4096 at 1025 rows 47.8 / 33.0
+//   (2, 1), 12288 x 4096 at 257 rows 51.4 / 38.7 (2, 1), at 1025 rows 93 / 86 (4, 3), 151936 x 1024 at 1025 rows 313 / 303 (41, 37);
+// - and in the first wave on a weight just decoded, while both operands fit half of L2 (start-up counts, memory does not): with the
+//   decode 4096 x 4096 at 640 rows 34.8 / 33.0, 5120 x 2048 at 640 25.6 / 24.6, 1024 x 4096 at 4096 31.4 / 30.1; but
+//   4096 x 8192 at 640 61 / 70, 1024 x 12288 at 2600 69 / 80;
+// - single CTAs with 128 x 128 where the large tiles would leave more than half of the SMs without work: 1024 x 4096 at 1024 rows,
+//   256 x 128 by a pair / 128 x 128 by a CTA 25.6 / 22.8.
 struct DgShape {
     int bn, cg;
 };
-static DgShape dg_pick(const nnq_ctx *ctx, int64_t m, int64_t n) {
-    const int64_t pair_tiles = (m + 255) / 256 * ((n + 255) / 256);
-    return 4 * pair_tiles <= ctx->sm_count ? DgShape{128, 1} : DgShape{256, 2};
+static DgShape dg_pick(const nnq_ctx *ctx, int64_t m, int64_t n, int64_t k, bool decoded) {
+    const int64_t wide = (n + 255) / 256, pair_tiles = (m + 255) / 256 * wide, tiles = (m + 127) / 128 * wide;
+    if (4 * pair_tiles <= ctx->sm_count) return {128, 1};
+    const int64_t pairs = ctx->sm_count / 2, pair_waves = (pair_tiles + pairs - 1) / pairs, waves = (tiles + ctx->sm_count - 1) / ctx->sm_count;
+    if (decoded && waves == 1 && (m + n) * k * 2 <= 60ll << 20) return {256, 1};
+    return 16 * pair_waves <= (k >= 2048 ? 18 : 17) * waves ? DgShape{256, 2} : DgShape{256, 1};
 }
 // Experts: the last row tile of each is filled by half on average, so tiles of 128 rows. (32 experts, 16384 routed rows: single
 // CTAs 572 + 328 us, pairs 564 + 322 when only they run, 1.855 against 1.879 ms for the block.)
@@ -649,7 +658,7 @@ static nnq_status dense_bf16(nnq_ctx *ctx, const void *w_bf16, const TcArgs &a, 
     CUtensorMap xmap, wmap;
     memset(&xmap, 0, sizeof(xmap));
     memset(&wmap, 0, sizeof(wmap));
-    const DgShape shape = dg_pick(ctx, a.m, a.n);
+    const DgShape shape = dg_pick(ctx, a.m, a.n, a.k, w_bf16 == ctx->d_dense);
     if (!make_map(a.x, a.m, a.k, kDgBM, &xmap) || !make_map(w_bf16, a.n, a.k, shape.bn / shape.cg, &wmap))
         return fail(ctx, NNQ_ERR_DISPATCH_FAILED, "tensor map creation failed");
     const DgArgs d = {a.bias, a.y, (int)a.m, (int)a.n, (int)a.k, a.y_dt, nullptr, 0, h_out, INFINITY, gate_kind};

@@ -9,6 +9,7 @@ torch = pytest.importorskip("torch")
 
 import rugesun_models as M
 from nn_b200 import api, models
+from nn_b200 import formats as F
 from nn_b200.formats import QuantFormat as Q
 from oracle import rugesun_ref as ref
 
@@ -35,6 +36,22 @@ def test_product(m, n, k, y_bf16, bias):
     if y_bf16:
         bound = bound * (1 + 2.0 ** -8) + want.abs() * 2.0 ** -8
     assert bool(((y.double() - want).abs() <= bound).all())
+    t.release()
+
+
+@pytest.mark.parametrize("fmt,m", [(Q.Q4_K, 1025), (Q.Q6_K, 1281), (Q.Q8_0, 4100)])
+def test_product_of_a_decoded_weight(fmt, m):
+    """Both operands inside half of the L2 cache take single CTAs with 128 x 256 in their first wave, 4100 rows pairs."""
+    n, k = 2817, 512
+    raw, sc = F.gen_weight(fmt, 5, n, k)
+    t = api.from_quantized(raw, fmt, [n, k], sc)
+    w = t.dequantize().to(torch.bfloat16).double()
+    x = torch.randn(m, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(m)).to(torch.bfloat16)
+    y = api.quantized_linear(x, t, out_dtype=torch.float32)
+    torch.cuda.synchronize()
+    t.backend.device_status()
+    want, mag = x.double() @ w.T, x.double().abs() @ w.abs().T
+    assert bool(((y.double() - want).abs() <= (k + 2) * 2.0 ** -24 * mag).all())
     t.release()
 
 
