@@ -249,7 +249,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     __shared__ __align__(8) uint64_t bars[2 * kDgStages + 5];   // full, empty [kDgStages], acc_full[2], acc_empty[2], every MMA has ended
     __shared__ uint32_t tmem_base_s;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
     const uint32_t full_s = smem_u32(bars), empty_s = full_s + 8 * kDgStages;
     const uint32_t accf_s = empty_s + 8 * kDgStages, acce_s = accf_s + 16, done_s = acce_s + 16;
     const int rank = CG == 2 ? (int)cluster_rank() : 0;
@@ -358,7 +358,9 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0 && rank == 0) {
+        // (the warp waits together, an elected lane issues: behind `lane == 0` the compiler loops over the active lanes around every
+        // instruction that takes uniform registers)
+        if (rank == 0) {
             // f32 accumulate, bf16 x bf16, both K-major, N = BN, M = 128 CG
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)BN >> 3) << 17) | (((uint32_t)kDgRows >> 4) << 24);
             int slot = 0;
@@ -367,37 +369,39 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
             for (int t = unit; t < tiles && ok; t += units, it++) {
                 const int a = it & 1;
                 // the epilogue has read this accumulator's previous tile
-                if (it >= 2 && !mbar_wait_fast(acce_s + 8 * a, (uint32_t)(((it >> 1) - 1) & 1))) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
+                if (it >= 2) ok = __all_sync(0xFFFFFFFFu, mbar_wait_fast(acce_s + 8 * a, (uint32_t)(((it >> 1) - 1) & 1)));
                 const uint32_t acc = tmem_base + (uint32_t)(a * kDgBN);
-                for (int kb = 0; kb < nkb; kb++) {
-                    if (!mbar_wait_fast(full_s + 8 * slot, phase)) {
-                        ok = false;
-                        break;
-                    }
+                for (int kb = 0; kb < nkb && ok; kb++) {
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait_fast(full_s + 8 * slot, phase));
+                    if (!ok) break;
                     tc_fence_after();
-                    const uint32_t a_s = smem_u32(smem + (size_t)slot * kDgStageBytes);
-                    const uint64_t da = smem_desc(a_s), db = smem_desc(a_s + kDgABytes);
+                    if (elect_one()) {
+                        const uint32_t a_s = smem_u32(smem + (size_t)slot * kDgStageBytes);
+                        const uint64_t da = smem_desc(a_s), db = smem_desc(a_s + kDgABytes);
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        if (CG == 2) umma_bf16_pair(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                        else umma_bf16(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        for (int k = 0; k < 4; k++) {
+                            if (CG == 2) umma_bf16_pair(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                            else umma_bf16(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        }
+                        if (CG == 2) umma_commit_pair(empty_s + 8 * slot);
+                        else umma_commit(empty_s + 8 * slot);
+                        if (kb == nkb - 1) {
+                            if (CG == 2) umma_commit_pair(accf_s + 8 * a);
+                            else umma_commit(accf_s + 8 * a);
+                        }
                     }
-                    if (CG == 2) umma_commit_pair(empty_s + 8 * slot);
-                    else umma_commit(empty_s + 8 * slot);
+                    __syncwarp();
                     if (++slot == kDgStages) {
                         slot = 0;
                         phase ^= 1u;
                     }
                 }
-                if (ok && CG == 2) umma_commit_pair(accf_s + 8 * a);
-                else if (ok) umma_commit(accf_s + 8 * a);
             }
-            if (CG == 2) umma_commit_pair(done_s);   // also behind a wait that ran out
-            else umma_commit(done_s);
+            if (elect_one()) {   // also behind a wait that ran out
+                if (CG == 2) umma_commit_pair(done_s);
+                else umma_commit(done_s);
+            }
+            __syncwarp();
         }
     } else {
         // ---------------- epilogue ----------------
