@@ -1618,7 +1618,11 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         if (lffn % 4 == 0) {
             launch_silu_mul_rows(ctx, d->pf_g, d->pf_u, d->pf_mid, d->act_dt, total, st);
         } else {
-            dec_silu_mul_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(d->pf_g, d->pf_u, d->pf_mid, d->act_dt, (int)total);
+            const int64_t some = 1 << 30;   // (the kernel counts in 32 bits)
+            for (int64_t at = 0; at < total; at += some) {
+                const int part = (int)std::min(some, total - at);
+                dec_silu_mul_kernel<<<(part + 255) / 256, 256, 0, st>>>(d->pf_g + at, d->pf_u + at, (char *)d->pf_mid + at * (d->act_dt == NNQ_F32 ? 4 : 2), d->act_dt, part);
+            }
         }
         s = d->comm ? nnq_comm_linear(d->comm, L.down, d->pf_mid, adt, n, nullptr, d->pf_delta, NNQ_F32, st)
                     : nnq_linear(ctx, L.down, d->pf_mid, adt, n, nullptr, d->pf_delta, NNQ_F32, st);
