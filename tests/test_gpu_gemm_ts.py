@@ -81,6 +81,24 @@ def test_several_products_of_one_call():
         torch.testing.assert_close(y, one, rtol=0, atol=float(k * 2.0 ** -24 * (np.abs(_bf16(x[k])) @ np.abs(w64).T).max()))   # (K may be split otherwise)
         t.release()
 
+# The steady state: at least five units of 256 weights per CTA. 130 rows: two tiles, K over the eight CTAs of a cluster; 20000
+# rows: 157 tiles, one CTA each. The rings of two raw and four operand stages turn at least twice.
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("n,k,m", [(130, 10496, 37), (130, 10496, 128), (20001, 1280, 40)])
+@pytest.mark.parametrize("x_bf16", [True, False])
+def test_many_units(fmt, n, k, m, x_bf16):
+    if fmt == Q.MXFP4_SPLIT:
+        k += 64   # a broken last unit behind whole ones
+    t, w64 = _weight(fmt, n, k, 13)
+    x = F.gen_activations(6, m, k, bf16=x_bf16)
+    xt = torch.from_numpy(x).cuda()
+    y = api.quantized_linear(xt.to(torch.bfloat16) if x_bf16 else xt, t, out_dtype=torch.float32)
+    torch.cuda.synchronize()
+    t.backend.device_status()
+    _check(y, x, w64, None, k)
+    t.release()
+
+
 @pytest.mark.parametrize("m", [64, 80, 81, 128, 160, 161, 241])
 def test_q8_0_tiles_of_f32_rows(m):
     """Up to 80 tokens per tile, tiles of equal size, the last one ragged."""
