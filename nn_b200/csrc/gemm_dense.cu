@@ -9,7 +9,7 @@
 //     64 (one 128-byte swizzle row of bf16), a ring of 6 x (16 KB activation tile + 16 KB weight tile) per CTA;
 //   * warp 0: one thread issues the TMA loads of both tiles (cp.async.bulk.tensor.2d, 128-byte
 //     swizzle, zero fill beyond M / N) onto the stage's "full" barrier;
-//   * warp 1: one thread (of the pair) issues tcgen05.mma (M 256, N 256, K 16, bf16 x bf16 -> f32) into one of
+//   * warp 1 (of the pair's first CTA): an elected lane issues tcgen05.mma (M 256, N 256, K 16, bf16 x bf16 -> f32) into one of
 //     two 256-column accumulators in tensor memory and commits the stage's "empty" barrier;
 //   * warps 2..5: epilogue -- tcgen05.ld of the finished accumulator (each warp its quarter of
 //     the 128 lanes), bias, conversion, stores -- while the MMA warp already fills the other
@@ -557,16 +557,6 @@ bool gemm_dense_shape_ok(const nnq_ctx *ctx, int64_t m, int64_t n, int64_t k, in
     return x_dt == NNQ_BF16 && m >= min_m && k >= kDgBK && k % kDgBK == 0 && n >= 1 && m < (1ll << 31) && n < (1ll << 31) && encode_fn() != nullptr;
 }
 bool gemm_dense_supported(const nnq_ctx *ctx, const nnq_weight *w, int64_t m, int x_dt) {
-    // Formats whose fused decode reads its raw blocks through the TMA ring keep it for longer. Measured on
-    // 4096 x 4096, 12288 x 4096 and 4096 x 12288 (us, fused / decoded once): Q4_K (either element order)
-    // 26 / 34, 53 / 68, 50 / 97 at 256 rows, 38 / 37, 75 / 95, 69 / 99 at 512 rows, 64 / 41, 142 / 122,
-    // 127 / 113 at 1024 rows; Q8_0 29 / 42, 58 / 84, 55 / 113 at 256 rows, 47 / 43, 113 / 111, 100 / 115 at
-    // 512 rows (its 512-row tile has no room for the ring).
-    if (w) {
-        const bool q4k = w->fmt == NNQ_Q4_K || w->fmt == NNQ_Q4_K_GGML;
-        const bool q8 = w->fmt == NNQ_Q8_0 && w->k % 256 == 0;
-        if ((q4k && m <= 512) || (q8 && m < 384)) return false;
-    }
     if (!w || !w->d_raw || !gemm_dense_shape_ok(ctx, m, w->n, w->k, x_dt)) return false;
     // a bf16 weight is multiplied in place, the others are decoded into the scratch
     return (w->fmt == NNQ_BF16_DENSE && !((uintptr_t)w->d_raw & 15u)) || (ctx->d_dense && (size_t)w->n * (size_t)w->k * 2 <= ctx->dense_bytes);

@@ -524,9 +524,11 @@ static cudaError_t launch_one(const TcArgs &a, int *status, int ksplit, float *p
 template <int FMT>
 static cudaError_t launch_fmt(const TcArgs &a, int *status, int mt, int ksplit, float *partials, cudaStream_t stream) {
     const bool f32 = a.x_dt == NNQ_F32;
-    if (mt == 1) return f32 ? launch_one<FMT, 1, float>(a, status, ksplit, partials, stream) : launch_one<FMT, 1, __nv_bfloat16>(a, status, ksplit, partials, stream);
-    if (mt == 2) return f32 ? launch_one<FMT, 2, float>(a, status, ksplit, partials, stream) : launch_one<FMT, 2, __nv_bfloat16>(a, status, ksplit, partials, stream);
-    return f32 ? launch_one<FMT, 4, float>(a, status, ksplit, partials, stream) : launch_one<FMT, 4, __nv_bfloat16>(a, status, ksplit, partials, stream);
+    if constexpr (FMT != NNQ_Q4_K && FMT != NNQ_Q4_K_GGML) {   // (more than 32 rows of these go to gemm_ts.cu)
+        if (mt == 2) return f32 ? launch_one<FMT, 2, float>(a, status, ksplit, partials, stream) : launch_one<FMT, 2, __nv_bfloat16>(a, status, ksplit, partials, stream);
+        if (mt == 4) return f32 ? launch_one<FMT, 4, float>(a, status, ksplit, partials, stream) : launch_one<FMT, 4, __nv_bfloat16>(a, status, ksplit, partials, stream);
+    }
+    return f32 ? launch_one<FMT, 1, float>(a, status, ksplit, partials, stream) : launch_one<FMT, 1, __nv_bfloat16>(a, status, ksplit, partials, stream);
 }
 
 template <int FMT, int MT>
@@ -588,7 +590,6 @@ nnq_status launch_gemm_tc(nnq_ctx *ctx, const TcArgs &a, cudaStream_t stream) {
     // by the context and are added in slice order by a second kernel.
     const int64_t ntiles = (a.n + 127) / 128;
     int mt = a.m > 256 ? 4 : (a.m > 128 ? 2 : 1);
-    if (mt == 4 && a.fmt == NNQ_Q8_0 && tc_raw_ring(a.fmt, a.k)) mt = 2;   // the 512-row tile leaves no room for the Q8_0 ring
     static const char *env_mt = diag_env("NNQ_TC_MT");   // tuning aid
     if (env_mt && (atoi(env_mt) == 1 || atoi(env_mt) == 2 || atoi(env_mt) == 4)) mt = atoi(env_mt);
     int ksplit = 1;

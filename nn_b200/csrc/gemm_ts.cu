@@ -21,6 +21,7 @@
 // Every wait is bounded; a CTA that gives up records it, still meets its cluster and frees its tensor memory.
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <limits.h>
 #include <string.h>
 
 #include <type_traits>
@@ -573,7 +574,7 @@ gemm_ts_kernel(const __grid_constant__ TsParams P) {
 
 // Raw rows a tensor map can address: whole 16-byte words per row. Q6_K comes from the tiled copy.
 bool gemm_ts_supported(const nnq_weight *w, int64_t m) {
-    if (!w || m < 1 || m > (1 << 20) || w->n < 1 || w->n > (1 << 24) || w->k < 64 || w->k > (1 << 24)) return false;
+    if (!w || m < 1 || w->n < 1 || w->n > INT_MAX - 128 || w->k < 64 || w->k > INT_MAX - 256) return false;
     switch (w->fmt) {
         case NNQ_Q4_K: case NNQ_Q4_K_GGML: case NNQ_Q4_0: case NNQ_Q8_0:
             return w->d_raw && w->k % 256 == 0 && ((uintptr_t)w->d_raw & 15u) == 0;
@@ -690,6 +691,15 @@ static nnq_status ts_run(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int x_d
 }
 
 nnq_status launch_gemm_ts(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int x_dt, int64_t m, int y_dt, cudaStream_t stream) {
+    constexpr int64_t kRows = 1 << 22;   // of a launch: at most 65535 token tiles
+    for (int64_t m0 = 0; m > kRows && m0 < m; m0 += kRows) {
+        SkinnyJob part[kSkinnyMaxJobs];
+        for (int i = 0; i < count; i++)
+            part[i] = {jobs[i].w, static_cast<const uint8_t *>(jobs[i].x) + m0 * jobs[i].w->k * (x_dt == NNQ_F32 ? 4 : 2), jobs[i].bias,
+                       static_cast<uint8_t *>(jobs[i].y) + m0 * jobs[i].w->n * (y_dt == NNQ_F32 ? 4 : 2)};
+        nnq_status s = launch_gemm_ts(ctx, part, count, x_dt, m - m0 < kRows ? m - m0 : kRows, y_dt, stream);
+        if (s != NNQ_OK || m0 + kRows >= m) return s;
+    }
     int i = 0;
     while (i < count) {   // jobs of the same activations, K and format go out together
         int e = i + 1;

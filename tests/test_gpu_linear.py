@@ -441,12 +441,11 @@ def test_qwen3_32b_shapes_prefill_and_decode(fmt, n, k):
 
 
 @pytest.mark.parametrize("fmt", [Q.Q4_K, Q.Q8_0, Q.Q6_K, Q.MXFP4_SPLIT, Q.Q5_K, Q.F32_DENSE, Q.BF16_DENSE])
-@pytest.mark.parametrize("m,n,k", [(256, 200, 512), (300, 520, 1024), (1000, 72, 2304)])
+@pytest.mark.parametrize("m,n,k", [(256, 200, 512), (300, 520, 1024), (513, 136, 512), (700, 520, 1024), (1000, 72, 2304)])
 def test_large_batch_takes_the_decode_once_path(fmt, m, n, k):
-    """From 256 rows of bf16 activations on (Q8_0: 384, Q4_K: 513 -- their fused decode is the faster
-    one below that, so the smaller cases here run it with two accumulators per CTA and K split over
-    CTAs), the weight is decoded to bf16 once and a plain TMA + tcgen05 product follows: ragged M and
-    N tiles, K a multiple of 64, bias, both outputs."""
+    """From 513 rows of bf16 activations on (256 for the formats that gemm_ts.cu does not read: Q5_K, unquantized), the weight is
+    decoded to bf16 once and a plain TMA + tcgen05 product follows: ragged M and N tiles, K a multiple of 64, bias, both
+    outputs. The cases of 256 and 300 rows of the other formats run the product with the weights in tensor memory."""
     _run(fmt, n, k, m, x_bf16=True, y_bf16=(m == 300), with_bias=(m != 256), seed=900 + m)
 
 
