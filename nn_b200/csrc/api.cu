@@ -398,8 +398,11 @@ static nnq_status linear_checked(nnq_ctx *ctx, const nnq_weight *w, const void *
 }
 
 // Rows that the product with the weights in tensor memory takes: from where the token-column kernel's two passes end (they
-// round no weight) up to 512 bf16 rows, above which decoding the weight once pays (Q4_K 12288 x 4096: 66 us here against 73 at
-// 512 rows, 130 against 109 at 1024); f32 rows have no such path and stay.
+// round no weight) up to 512 bf16 rows. Decoded once / here in us: 4096 x 4096, 12288 x 4096, 4096 x 12288 in Q6_K at 384 rows 34 / 29,
+// 70 / 54, 102 / 69, at 512 rows 35 / 29, 93 / 82, 103 / 75; at 513 rows in Q4_K 34 / 38, 73 / 76, 105 / 78 and 1024 x 4096 24 / 14, Q6_K
+// and MXFP4 12288 x 4096 82 / 92 and 82 / 100; at 1024 rows Q4_K 34 / 39, 95 / 116, 108 / 104, 24 / 16. (Deep and narrow weights would
+// stay ahead here for longer.) f32 rows have the fused decode as the only other way, which is behind at every count measured: at 4096
+// rows of 12288 x 4096 Q4_K 1436 / 968, Q8_0 1235 / 1055, Q6_K 1865 / 1246, MXFP4 1564 / 1013.
 static bool takes_gemm_ts(const nnq_ctx *ctx, const nnq_weight *w, int64_t m, int x_dt) {
     if ((ctx->path != NNQ_PATH_AUTO && ctx->path != NNQ_PATH_TENSOR) || !gemm_ts_supported(w, m)) return false;
     return m > (x_dt == NNQ_BF16 ? 32 : 16) && (x_dt == NNQ_F32 || m <= 512);

@@ -9,9 +9,9 @@
 // One CTA: 128 query vectors of one kv head (consecutive (row, query head of the group) pairs), key tiles of
 // 64 over the union of the rows' windows.
 //   warps 0-3: softmax. Thread r owns query vector r: reads its 64 scores from tensor memory, updates maximum
-//              and sum, writes the weights as two swizzled bf16 tiles; adds the previous tile's weighted values
+//              and sum, writes the weights as two swizzled 16-bit tiles; adds the previous tile's weighted values
 //              from tensor memory to its f32 accumulators.
-//   warps 4-6: loaders. Convert the next key / value tile from the f32 ring cache into swizzled bf16 pairs
+//   warps 4-6: loaders. Convert the next key / value tile from the f32 ring cache into swizzled 16-bit pairs
 //              (values transposed), two stages.
 //   warp 7:    one thread issues the MMAs: S(t + 1) = Q K^T right behind O(t) = P V.
 // A commit after S(t + 1) tells the softmax warps that both are complete. Every wait is bounded.

@@ -147,7 +147,7 @@ dequant_bf16_kernel(const uint8_t *__restrict__ src, const uint8_t *__restrict__
 // nn-gptoss expert tensors [E, K, N] (MXFP4, 32-weight blocks along N, the even column in the high
 // nibble) -> bf16 [E, N, K]: a CTA turns a 64 x 64 tile through shared memory. Reads are whole sectors
 // (32 bytes of a k row), writes 128 contiguous bytes per output row. Bound by the decode, which looks four magnitudes up at a
-// time and stores pairs of k: the 4096-token block of 32 experts of 2880, one code at a time / this: 1.84 / 1.76 ms. half_rows > 0 interleaves the output
+// time and stores pairs of k: the 4096-token block of 32 experts of 2880, one code at a time / this: 1.82 / 1.74 ms. half_rows > 0 interleaves the output
 // rows of every expert (row j -> 2j, row half_rows + j -> 2j + 1), as the fused SwiGLU epilogue wants.
 constexpr int kKnTile = 64;
 __global__ void __launch_bounds__(128)
@@ -237,7 +237,7 @@ constexpr int kDgMaxGroups = 256;
 // once per 128 x 256. With one CTA the two (48 KB in, 48 KB out per 64-wide k step of 512 tensor-core clocks) exceed what
 // shared memory moves. The first CTA of the pair issues the MMAs; its "full" barriers count both CTAs' copies, its "empty" and "accumulator
 // full" commits reach both CTAs, both CTAs' epilogues hand the accumulators back to it.
-// 25600 x 5120 at 4096 rows: 731 -> 696 us (1.54 PFLOP/s), the seven products of such a layer 2890 -> 2715 us.
+// 25600 x 5120 at 4096 rows: 739 -> 683 us (1.57 PFLOP/s), the seven products of such a layer in Q6_K 3.68 -> 3.42 ms, decode included.
 template <int BN, int CG>
 __global__ void __launch_bounds__(kDgThreads, 1)
 gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,

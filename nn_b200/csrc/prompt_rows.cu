@@ -73,7 +73,7 @@ dec_norm_rows4_kernel(float *__restrict__ h, const float *__restrict__ delta, co
 }
 
 // Heads of 128: a warp per head of a row, four dimensions per lane (the pair of a dimension, 64 on, is 16 lanes away), eight
-// heads per CTA: 0.57 -> 0.20 ms for eight layers of 2048 rows. Same numbers as the kernel below but for the order of the sum
+// heads per CTA: 0.57 -> 0.20 ms for eight layers of 2048 rows. Same numbers as dec_qk_rope_rows_kernel (decoder.cu) but for the order of the sum
 // of squares.
 __global__ void __launch_bounds__(256)
 dec_qk_rope_rows128_kernel(const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v, const float *__restrict__ qw,

@@ -67,7 +67,8 @@ def test_broken_unit(k, x_bf16):
 
 
 def test_several_products_of_one_call():
-    """Jobs of one input share a launch, another input and another K start their own; results are those of single calls."""
+    """Jobs of one input share a launch, another input and another K start their own; results are those of single calls but for the
+    rounding of sums (K may be split for all tiles of a launch)."""
     m, pairs = 70, []
     for i, (n, k) in enumerate([(300, 512), (64, 512), (128, 512), (200, 1024)]):
         pairs.append((_weight(Q.Q4_K, n, k, 20 + i), k))
