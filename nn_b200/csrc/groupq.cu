@@ -583,11 +583,15 @@ void gq_set_fast(nnq_gq_weight *w, float zp_abs_max) {
 }
 
 // 4-bit codes and up to 16 bf16 rows, groups that hold whole steps of 32 weights (one word per lane) or more. Steps of one word
-// bring a scale and a zero point per word: for one and two rows the streaming kernel stays ahead (groups of 32, streaming / this
-// in us: 12288 x 4096 20.4 / 29.9, 23.9 / 30.6, 35.3 / 31.3 at 1, 2, 4 rows; 4096 x 4096 10.6 / 11.2, 11.3 / 11.2, 14.7 / 11.5).
+// fetch a scale and a zero point per word, and the streaming kernel stays ahead for one and two rows of large weights. Streaming /
+// this in us at 1 and 2 rows, groups of 32: 20000 x 8192 50 / 78, 61 / 78; 12288 x 4096 20.4 / 29.9, 23.9 / 30.6; 8192 x 4096 14.2 / 18.1,
+// 17.5 / 18.4; 4096 x 4096 10.7 / 11.1, 11.2 / 11.3; 4096 x 12800 28.4 / 25.5, 29.9 / 25.8; 2048 x 8192 16.3 / 15.0, 15.8 / 15.0; 1000 x 1024
+// 2.8 / 3.2, 3.6 / 3.2. Groups of 96: 12288 x 12288 51 / 79, 60 / 81; 2048 x 8160 16.5 / 19.7, 17.6 / 19.7; 20000 x 4032 31.5 / 29.7,
+// 39.8 / 29.9; 4096 x 2016 6.3 / 4.9, 7.8 / 5.0. At 3 rows this is ahead everywhere (20000 x 4096 50.6 / 47.0).
 bool gq_mma_takes(const nnq_gq_weight *w, int x_dt, int64_t m) {
     const bool wide = w->group_size % 64 == 0 && w->k % 64 == 0;
-    return w->bits == 4 && w->exact16 && x_dt == NNQ_BF16 && m <= 16 && (wide || m > 2) && w->group_size % 32 == 0 && w->n <= (1ll << 31) && w->k < (1ll << 31);
+    const bool stream = m <= 2 && !wide && (w->group_size == 32 ? w->n > 4096 || (m == 1 && w->k < 4096) : w->k > 4096);
+    return w->bits == 4 && w->exact16 && x_dt == NNQ_BF16 && m <= 16 && !stream && w->group_size % 32 == 0 && w->n <= (1ll << 31) && w->k < (1ll << 31);
 }
 
 template <int W>

@@ -263,10 +263,11 @@ def test_gptq_shape_errors():
 
 
 @pytest.mark.parametrize("m", [1, 2, 3, 8, 9, 16])
-@pytest.mark.parametrize("n,k,g,zp_max", [(16, 128, 128, 100), (33, 2048, 256, 2), (50, 1152, 64, 100), (17, 96, 32, 100), (130, 1024, 128, 101), (40, 640, 32, 7)])
+@pytest.mark.parametrize("n,k,g,zp_max", [(16, 128, 128, 100), (33, 2048, 256, 2), (50, 1152, 64, 100), (17, 96, 32, 100), (130, 1024, 128, 101), (40, 640, 32, 7), (4112, 256, 32, 5), (24, 4128, 32, 9),
+                                        (18, 4128, 96, 3)])
 def test_int4_products_of_bf16_rows(n, k, g, zp_max, m):
-    """Codes as exact bf16 integers on the tensor cores up to a zero point of 100, f32 decode above and for one and two rows of
-    groups of 32: steps of one, two and four words, fewer steps than warps, ragged rows, one and two column groups. f32 sums of exact products: K roundings of 2^-24."""
+    """Codes as exact bf16 integers on the tensor cores up to a zero point of 100, f32 decode above and for one and two rows
+    where steps of one word are behind: steps of one, two and four words, fewer steps than warps, ragged rows, one and two column groups. f32 sums of exact products: K roundings of 2^-24."""
     rng = np.random.default_rng(n + k + m)
     codes = rng.integers(0, 256, n * k // 2, dtype=np.uint8)
     scale = ((rng.random(n * (k // g)) + 0.5) * 0.01).astype(f32)
