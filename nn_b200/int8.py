@@ -21,7 +21,7 @@ class Int8QuantParams:
 
 
 def _stream(torch, dev):
-    return api._stream_ptr(torch.cuda.current_stream(dev))
+    return api._stream_ptr(None, dev.index)
 
 
 def quantize_per_channel(weights, mode: int, backend: Optional[api.Backend] = None):
