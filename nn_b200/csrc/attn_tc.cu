@@ -81,7 +81,7 @@ __device__ __forceinline__ uint32_t swz_at(int r, int e) { return swz(r, e >> 3)
 template <int ATOMS, int NV, bool SCALED>
 __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn a, const uint2 *__restrict__ top, int all_tiles, int *status) {
     extern __shared__ __align__(1024) uint8_t at_smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(at_smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = at_smem_raw + (-smem_u32(at_smem_raw) & 1023u);   // (stays an address in shared memory to the compiler)
     __shared__ __align__(8) uint64_t bars[6];   // kv_full[2], kv_empty[2], s_full, p_full
     __shared__ uint32_t tmem_s;
     __shared__ float q_unscale[SCALED ? kAtRows : 1];

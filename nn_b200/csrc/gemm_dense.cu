@@ -245,7 +245,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                   const int *__restrict__ offsets, int groups, __nv_bfloat16 *__restrict__ h_out, float swiglu_limit, int gate_kind) {
     constexpr int kDgBN = BN, kDgStageBytes = dg_stage_bytes(BN, CG), kDgStages = dg_stages(BN, CG), kDgRows = kDgBM * CG;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = smem_raw + (-smem_u32(smem_raw) & 1023u);   // (stays an address in shared memory to the compiler)
     __shared__ __align__(8) uint64_t bars[2 * kDgStages + 5];   // full, empty [kDgStages], acc_full[2], acc_empty[2], every MMA has ended
     __shared__ uint32_t tmem_base_s;
 

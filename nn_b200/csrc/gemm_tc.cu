@@ -102,7 +102,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
                int64_t K, int y_dt, int stages, int use_ring, float *__restrict__ partials, int *status, const TcGroup grp) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // 1024-byte alignment of the tiles (the dynamic window is not guaranteed to start on one)
-    uint8_t *smem_al = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem_al = smem_raw + (-smem_u32(smem_raw) & 1023u);   // (stays an address in shared memory to the compiler)
     using RG = TcRawGeom<FMT, MT>;
     const bool kRawRing = RG::kRing && use_ring;   // (compile-time false for formats without a ring)
     uint8_t *rawring = smem_al;                                  // two raw chunks (ring formats only)

@@ -302,7 +302,7 @@ gemm_ts_kernel(const __grid_constant__ TsParams P) {
     using G = TsGeom<FMT>;
     constexpr int W = G::kStages;
     extern __shared__ uint8_t ts_smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(ts_smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = ts_smem_raw + (-smem_u32(ts_smem_raw) & 1023u);   // (stays an address in shared memory to the compiler)
     // w_full, w_empty [W], x_full, x_empty [8], a_full, a_empty [4], accumulators ready
     __shared__ __align__(8) uint64_t bars[2 * W + 2 * kTsMaxX + 9];
     __shared__ uint32_t tmem_s;

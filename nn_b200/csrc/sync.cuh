@@ -27,8 +27,9 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
 }
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    // the last operand caps the time one try may suspend the thread (nanoseconds)
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 2000;\n selp.u32 %0, 1, 0, p;\n}"
+    // (suspends the thread until the phase ends, some microseconds at most; with a time of its own the instruction becomes a loop
+    // that polls and sleeps: 129 instead of 99 clocks from an arrival to the waiting warp, and a tenth more issue slots in gemm_ts.cu)
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
@@ -46,7 +47,7 @@ __device__ __forceinline__ bool mbar_wait_fast(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n .reg .pred p;\n .reg .u32 n;\n mov.u32 n, %3;\n"
-        "W_%=:\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 2000;\n @p bra D_%=;\n"
+        "W_%=:\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n @p bra D_%=;\n"
         " sub.u32 n, n, 1;\n setp.ne.u32 p, n, 0;\n @p bra W_%=;\n mov.u32 %0, 0;\n bra E_%=;\n"
         "D_%=:\n mov.u32 %0, 1;\nE_%=:\n}"
         : "=r"(ok) : "r"(bar), "r"(parity), "r"(kWaitSpins) : "memory");
