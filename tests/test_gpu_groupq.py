@@ -282,3 +282,17 @@ def test_int4_products_of_bf16_rows(n, k, g, zp_max, m):
     x64 = x.double().numpy()
     assert np.all(np.abs(y - x64 @ w.T) <= (k + 4) * 2.0 ** -24 * (np.abs(x64) @ np.abs(w).T))
     qt.release()
+
+
+@pytest.mark.parametrize("m", [1, 16])
+@pytest.mark.parametrize("n,k,g", [(40, 5248, 128), (24, 4224, 64), (24, 2720, 32), (18, 1024, 128), (18, 640, 64)])
+def test_int4_products_in_several_batches_of_steps(n, k, g, m):
+    """A warp's steps in whole batches, in a broken one behind one or two whole ones, and none at all for some warps. Exact products and
+    f32 sums: k f32 roundings of partial sums."""
+    rng = np.random.default_rng(n + k)
+    w = _weights(k, n, k)
+    qt = wq.quantize_per_group(torch.from_numpy(w), _cfg(4, g, True))
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(f32)).to(torch.bfloat16).cuda()
+    w64, x64 = wq.dequantize(qt).double().cpu().numpy(), x.double().cpu().numpy()
+    y = wq.quantized_matmul(x, qt).double().cpu().numpy()
+    assert np.all(np.abs(y - x64 @ w64.T) <= (k + 2) * 2.0 ** -24 * (np.abs(x64) @ np.abs(w64).T))
