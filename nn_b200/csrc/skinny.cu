@@ -344,26 +344,83 @@ static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, i
     return check_cuda(ctx, e, "skinny launch");
 }
 
-template <int FMT, int SB, int NT, bool F32X>
-static cudaError_t launch_grouped_t(const GroupedParams &P, int grid, int smem_bytes, cudaStream_t stream) {
-    static bool configured[64] = {};
+// Launch geometry of the grouped kernel: ways to split K (CTAs of a cluster), ring depth, tiles of K staged together,
+// clusters. `units` units of eight row tiles. The shortest estimate in tiles of a warp that has its SM's share of a CTA for itself.
+struct GroupedShape {
+    int slices, stages, chunk, clusters, smem;
+};
+
+static GroupedShape grouped_shape(int kblocks, int sb, int tile_bytes, int nt, bool f32x, int sums, int64_t units, int sms) {
+    static const int fit148[9] = {0, 296, 148, 93, 71, 56, 45, 37, 33};   // clusters resident at two CTAs per SM
+    static const char *env = diag_env("NNQ_GROUPED_SLICES"), *env_st = diag_env("NNQ_GROUPED_STAGES");   // tuning aids
+    const int forced = env ? atoi(env) : 0, forced_st = env_st ? atoi(env_st) : 0;
+    GroupedShape best = {};
+    double least = 1e30;
+    for (int c = 1; c <= 8 && c <= kblocks; c++) {
+        if (forced && c != forced) continue;
+        GroupedShape s;
+        s.slices = c;
+        const int slice = (kblocks + c - 1) / c;
+        s.chunk = slice;
+        s.stages = forced_st ? forced_st : kMaxStages;
+        auto total = [&]() { return grouped_plan(tile_bytes, s.stages, nt, f32x, sums, s.chunk * sb, c > 1).total; };
+        while (s.stages > 2 && total() > kGroupedSmem) s.stages--;
+        while (s.chunk > 1 && total() > kGroupedSmem) s.chunk--;
+        s.smem = total();
+        const int64_t slots = sms * fit148[c] / 148 > 0 ? sms * fit148[c] / 148 : 1;
+        s.clusters = (int)(units < slots ? units : slots);
+        const int64_t iters = (units + slots - 1) / slots;
+        const double tile = s.clusters * c <= sms ? 1.0 : 1.6;
+        double t = iters * (slice * tile + (c > 1 ? 0.8 : 0.3)) + 0.3 * slice;
+        if (s.chunk < slice) t += iters * 0.5 * slice;
+        if (t < least - 1e-9) {
+            least = t;
+            best = s;
+        }
+    }
+    return best;
+}
+
+template <class Params>
+static cudaError_t grouped_launch(void (*kernel)(Params), const Params &P, const GroupedShape &s, bool *configured, cudaStream_t stream) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(skinny_grouped_kernel<FMT, SB, NT, F32X>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             kSmemMax - 1024);   // the kernel also has a small static table
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupedSmem);
         if (e != cudaSuccess) return e;
         configured[dev] = true;
     }
-    skinny_grouped_kernel<FMT, SB, NT, F32X><<<grid, kWarps * 32, smem_bytes, stream>>>(P);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(s.clusters * s.slices));
+    cfg.blockDim = dim3(kWarps * 32);
+    cfg.dynamicSmemBytes = s.smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)s.slices;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kernel, P);
+}
+
+template <int FMT, int SB, int NT, bool F32X>
+static cudaError_t launch_grouped_t(GroupedParams &P, int64_t groups, int sms, cudaStream_t stream) {
+    static bool configured[64] = {};
+    using TF = TileFmt<FMT, SB>;
+    const GroupedShape s = grouped_shape(P.kblocks, SB, TF::kBytes, NT, F32X, TF::kSums, groups * ((P.row_tiles + kWarps - 1) / kWarps), sms);
+    P.slices = s.slices;
+    P.stages = s.stages;
+    P.chunk = s.chunk;
+    return grouped_launch<GroupedParams>(skinny_grouped_kernel<FMT, SB, NT, F32X>, P, s, configured, stream);
 }
 
 template <int FMT, int SB>
-static cudaError_t launch_grouped_x(const GroupedParams &P, bool f32x, int nt, int grid, int smem_bytes, cudaStream_t stream) {
-    if (f32x) return launch_grouped_t<FMT, SB, 1, true>(P, grid, smem_bytes, stream);   // two MMAs per product: 8 rows
-    return nt == 2 ? launch_grouped_t<FMT, SB, 2, false>(P, grid, smem_bytes, stream)
-                   : launch_grouped_t<FMT, SB, 1, false>(P, grid, smem_bytes, stream);
+static cudaError_t launch_grouped_x(GroupedParams &P, bool f32x, int nt, int64_t groups, int sms, cudaStream_t stream) {
+    if (f32x) return launch_grouped_t<FMT, SB, 1, true>(P, groups, sms, stream);   // two MMAs per product: 8 rows
+    return nt == 2 ? launch_grouped_t<FMT, SB, 2, false>(P, groups, sms, stream) : launch_grouped_t<FMT, SB, 1, false>(P, groups, sms, stream);
 }
 
 nnq_status launch_grouped(nnq_ctx *ctx, const GroupedArgs &a, cudaStream_t stream) {
@@ -385,33 +442,28 @@ nnq_status launch_grouped(nnq_ctx *ctx, const GroupedArgs &a, cudaStream_t strea
     P.n = (int)a.n;
     P.row_tiles = (int)((a.n + 15) / 16);
     P.kblocks = (int)(a.k / (32 * sb));
-    P.stages = 2;
     P.status = ctx->d_status;
     const bool f32x = a.x_dt == NNQ_F32;
     // 16-row groups once the experts see 5 or more rows on average (bf16 activations only)
-    const int nt = !f32x && a.max_rows >= 5 * (int64_t)a.experts ? 2 : 1;
-    const int smem_bytes = mn_plan(a.kn_gptoss ? 288 * sb : tile_bytes_of(a.fmt, sb), P.stages, nt).total;
-    // every expert may end with a partly filled row group
-    const int64_t max_units = (a.max_rows / (8 * nt) + a.experts) * P.row_tiles;
-    int64_t grid = 2 * (int64_t)ctx->sm_count;
-    if (grid > max_units) grid = max_units;
-    if (grid < 1) grid = 1;
+    const int nt = !f32x && a.max_rows >= 5 * (int64_t)a.experts ? 2 : 1, sms = ctx->sm_count;
+    // row groups to be expected: at most one per row, about half of the last group of an expert empty
+    int64_t groups = (a.max_rows + 4 * nt * (int64_t)a.experts) / (8 * nt);
+    if (groups > a.max_rows) groups = a.max_rows;
+    if (groups < 1) groups = 1;
     cudaError_t e;
     if (a.kn_gptoss) {
-        e = sb == 8 ? launch_grouped_x<NNQ_MXFP4_GPTOSS, 8>(P, f32x, nt, (int)grid, smem_bytes, stream)
-                    : launch_grouped_x<NNQ_MXFP4_GPTOSS, 6>(P, f32x, nt, (int)grid, smem_bytes, stream);
+        e = sb == 8 ? launch_grouped_x<NNQ_MXFP4_GPTOSS, 8>(P, f32x, nt, groups, sms, stream) : launch_grouped_x<NNQ_MXFP4_GPTOSS, 6>(P, f32x, nt, groups, sms, stream);
         ctx->launches++;
         return check_cuda(ctx, e, "grouped product launch");
     }
     switch (layout_of(a.fmt)) {
-        case kTiledQ4K: e = launch_grouped_x<NNQ_Q4_K, 8>(P, f32x, nt, (int)grid, smem_bytes, stream); break;
-        case kTiledQ8_0: e = launch_grouped_x<NNQ_Q8_0, 8>(P, f32x, nt, (int)grid, smem_bytes, stream); break;
-        case kTiledQ6K: e = launch_grouped_x<NNQ_Q6_K, 8>(P, f32x, nt, (int)grid, smem_bytes, stream); break;
-        case kTiledQ4_0: e = launch_grouped_x<NNQ_Q4_0, 8>(P, f32x, nt, (int)grid, smem_bytes, stream); break;
-        case kTiledQ4_1: e = launch_grouped_x<NNQ_Q4_1, 8>(P, f32x, nt, (int)grid, smem_bytes, stream); break;
+        case kTiledQ4K: e = launch_grouped_x<NNQ_Q4_K, 8>(P, f32x, nt, groups, sms, stream); break;
+        case kTiledQ8_0: e = launch_grouped_x<NNQ_Q8_0, 8>(P, f32x, nt, groups, sms, stream); break;
+        case kTiledQ6K: e = launch_grouped_x<NNQ_Q6_K, 8>(P, f32x, nt, groups, sms, stream); break;
+        case kTiledQ4_0: e = launch_grouped_x<NNQ_Q4_0, 8>(P, f32x, nt, groups, sms, stream); break;
+        case kTiledQ4_1: e = launch_grouped_x<NNQ_Q4_1, 8>(P, f32x, nt, groups, sms, stream); break;
         default:
-            e = sb == 8 ? launch_grouped_x<NNQ_MXFP4_SPLIT, 8>(P, f32x, nt, (int)grid, smem_bytes, stream)
-                        : launch_grouped_x<NNQ_MXFP4_SPLIT, 6>(P, f32x, nt, (int)grid, smem_bytes, stream);
+            e = sb == 8 ? launch_grouped_x<NNQ_MXFP4_SPLIT, 8>(P, f32x, nt, groups, sms, stream) : launch_grouped_x<NNQ_MXFP4_SPLIT, 6>(P, f32x, nt, groups, sms, stream);
             break;
     }
     ctx->launches++;

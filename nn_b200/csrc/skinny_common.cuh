@@ -13,6 +13,7 @@ constexpr int kTileBytes = 2304;
 constexpr int kWarps = 8;          // compute warps per CTA; they split K of one row tile
 constexpr int kMaxStages = 4;      // bulk-copy ring depth per warp (tiles in flight)
 constexpr int kSmemMax = 227 * 1024;         // one CTA per SM
+constexpr int kGroupedSmem = 113 * 1024 - 512;   // grouped kernel: two CTAs per SM
 constexpr int kMoeMaxExperts = 64;
 
 struct SkinnyJobDev {

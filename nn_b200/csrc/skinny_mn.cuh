@@ -107,19 +107,58 @@ struct MnConsts {
     }
 };
 
+// The activations of a tile's blocks in shared memory, in the order in which the lanes of an MMA take them: per block of 32
+// weights and eight tokens 512 bytes, 16 per lane (lane 4g + t: token g, the eight elements of a weight lane t), then the
+// remainders of f32 activations; and the sums over the blocks (or their halves), [block][half][token].
+struct MnSharedX {
+    const uint4 *f;   // at this lane's 16 bytes of the tile's first block
+    const float *s;   // at tokens 2t, 2t + 1 of the tile's first block
+    template <int NT, bool F32X>
+    __device__ __forceinline__ XB<F32X> frag(int block, int nt, int) const {
+        XB<F32X> r;
+        r.hi = f[(block * NT + nt) * (F32X ? 64 : 32)];
+        r.lo = F32X ? f[(block * NT + nt) * 64 + 32] : make_uint4(0, 0, 0, 0);
+        return r;
+    }
+    template <int NT, int SUMS, bool F32X>
+    __device__ __forceinline__ void sum(float (&v)[4], int block, int half, int nt, const XB<F32X> &, const MnConsts &) const {
+        const float2 u = *reinterpret_cast<const float2 *>(s + (block * SUMS + half) * NT * 8 + nt * 8);
+        v[0] = v[2] = u.x;
+        v[1] = v[3] = u.y;
+    }
+};
+
+// The same from global memory (L1 / L2 resident), the sums by a second MMA with ones in place of the weights. HALVES: a lane has
+// four elements of each half of a block.
+template <int NT_, bool HALVES>
+struct MnGlobalX {
+    const uint8_t *row[NT_];
+    int koff;   // the tile's first element
+    template <int NT, bool F32X>
+    __device__ __forceinline__ XB<F32X> frag(int block, int nt, int t) const {
+        const int e0 = koff + block * 32 + (HALVES ? 4 : 8) * t;
+        return load_xb<F32X>(row[nt], e0, e0 + (HALVES ? 16 : 4));
+    }
+    template <int NT, int SUMS, bool F32X>
+    __device__ __forceinline__ void sum(float (&v)[4], int, int half, int, const XB<F32X> &xb, const MnConsts &K) const {
+        const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        mma_x<F32X>(v, K.ones, K.ones, K.ones, K.ones, xb, half, zero);
+        if (SUMS == 1) mma_x<F32X>(v, K.ones, K.ones, K.ones, K.ones, xb, 1, v);
+    }
+};
+
 template <int FMT, int SB = 8>
 struct TileFmt;   // SB = sub-blocks of 32 weights per tile row
 
 // ---- Q4_K (both element orders share the tiled layout) ----
 template <>
 struct TileFmt<NNQ_Q4_K, 8> {
+    static constexpr int kSums = 1;
     static constexpr int kBytes = 2304;
     static constexpr int kElems = 256;
-    template <int NT, bool F32X>
-    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *sct4, const uint8_t *const (&xrow)[NT],
-                                                int koff, int lane, int g, int t, const MnConsts &K,
+    template <int NT, bool F32X, class X>
+    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *sct4, const X &x, int lane, int g, int t, const MnConsts &K,
                                                 float (&y)[NT][4]) {
-        constexpr int ES = F32X ? 4 : 2;
         const uint4 *st = reinterpret_cast<const uint4 *>(stage);
         const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         // (d sc, 128 d sc + dmin m) of the tile: this lane's share (rows g, g+8; sub-blocks 2t, 2t+1)
@@ -152,13 +191,11 @@ struct TileFmt<NNQ_Q4_K, 8> {
                 const float dsc8 = s2 ? sg8.z : sg8.x, e8 = s2 ? sg8.w : sg8.y;
 #pragma unroll
                 for (int nt = 0; nt < NT; nt++) {
-                    const int e0 = koff + (2 * p + s2) * 32 + 8 * t;
-                    const XB<F32X> xb = load_xb<F32X>(xrow[nt], e0, e0 + 4);
+                    const XB<F32X> xb = x.template frag<NT, F32X>(2 * p + s2, nt, t);
                     float c[4], sx[4];
                     mma_x<F32X>(c, a0, a1, a2, a3, xb, 0, zero);
                     mma_x<F32X>(c, a4, a5, a6, a7, xb, 1, c);
-                    mma_x<F32X>(sx, K.ones, K.ones, K.ones, K.ones, xb, 0, zero);
-                    mma_x<F32X>(sx, K.ones, K.ones, K.ones, K.ones, xb, 1, sx);
+                    x.template sum<NT, 1, F32X>(sx, 2 * p + s2, 0, nt, xb, K);
                     y[nt][0] = fmaf(dsc, c[0], fmaf(-e, sx[0], y[nt][0]));
                     y[nt][1] = fmaf(dsc, c[1], fmaf(-e, sx[1], y[nt][1]));
                     y[nt][2] = fmaf(dsc8, c[2], fmaf(-e8, sx[2], y[nt][2]));
@@ -166,18 +203,17 @@ struct TileFmt<NNQ_Q4_K, 8> {
                 }
             }
         }
-        (void)ES;
     }
 };
 
 // ---- Q8_0 ----
 template <>
 struct TileFmt<NNQ_Q8_0, 8> {
+    static constexpr int kSums = 1;
     static constexpr int kBytes = 4352;
     static constexpr int kElems = 256;
-    template <int NT, bool F32X>
-    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *, const uint8_t *const (&xrow)[NT],
-                                                int koff, int lane, int g, int t, const MnConsts &K,
+    template <int NT, bool F32X, class X>
+    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *, const X &x, int lane, int g, int t, const MnConsts &K,
                                                 float (&y)[NT][4]) {
         const uint4 *st = reinterpret_cast<const uint4 *>(stage);
         const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -199,15 +235,13 @@ struct TileFmt<NNQ_Q8_0, 8> {
             }
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const int e0 = koff + sb * 32 + 8 * t;
-                const XB<F32X> xb = load_xb<F32X>(xrow[nt], e0, e0 + 4);
+                const XB<F32X> xb = x.template frag<NT, F32X>(sb, nt, t);
                 float c[4], sx[4];
                 mma_x<F32X>(c, L[0], L8[0], L[1], L8[1], xb, 0, zero);
                 mma_x<F32X>(c, L[2], L8[2], L[3], L8[3], xb, 1, c);
                 mma_x<F32X>(c, H[0], H8[0], H[1], H8[1], xb, 0, c);
                 mma_x<F32X>(c, H[2], H8[2], H[3], H8[3], xb, 1, c);
-                mma_x<F32X>(sx, K.ones, K.ones, K.ones, K.ones, xb, 0, zero);
-                mma_x<F32X>(sx, K.ones, K.ones, K.ones, K.ones, xb, 1, sx);
+                x.template sum<NT, 1, F32X>(sx, sb, 0, nt, xb, K);
                 y[nt][0] = fmaf(d, fmaf(-2304.0f, sx[0], c[0]), y[nt][0]);
                 y[nt][1] = fmaf(d, fmaf(-2304.0f, sx[1], c[1]), y[nt][1]);
                 y[nt][2] = fmaf(d8, fmaf(-2304.0f, sx[2], c[2]), y[nt][2]);
@@ -220,11 +254,11 @@ struct TileFmt<NNQ_Q8_0, 8> {
 // ---- Q6_K ----
 template <>
 struct TileFmt<NNQ_Q6_K, 8> {
+    static constexpr int kSums = 2;   // scale groups of 16
     static constexpr int kBytes = 3360;
     static constexpr int kElems = 256;
-    template <int NT, bool F32X>
-    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *sct4, const uint8_t *const (&xrow)[NT],
-                                                int koff, int lane, int g, int t, const MnConsts &K,
+    template <int NT, bool F32X, class X>
+    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *sct4, const X &x, int lane, int g, int t, const MnConsts &K,
                                                 float (&y)[NT][4]) {
         const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         const uint32_t *sw = reinterpret_cast<const uint32_t *>(stage);
@@ -254,15 +288,14 @@ struct TileFmt<NNQ_Q6_K, 8> {
             }
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const int e0 = koff + sb * 32 + 4 * t;
-                const XB<F32X> xb = load_xb<F32X>(xrow[nt], e0, e0 + 16);
+                const XB<F32X> xb = x.template frag<NT, F32X>(sb, nt, t);
                 float ca[4], cb[4], sa[4], sb4[4];
                 mma_x<F32X>(ca, L[0], L8[0], L[1], L8[1], xb, 0, zero);
                 mma_x<F32X>(ca, H[0], H8[0], H[1], H8[1], xb, 0, ca);
-                mma_x<F32X>(sa, K.ones, K.ones, K.ones, K.ones, xb, 0, zero);
+                x.template sum<NT, 2, F32X>(sa, sb, 0, nt, xb, K);
                 mma_x<F32X>(cb, L[2], L8[2], L[3], L8[3], xb, 1, zero);
                 mma_x<F32X>(cb, H[2], H8[2], H[3], H8[3], xb, 1, cb);
-                mma_x<F32X>(sb4, K.ones, K.ones, K.ones, K.ones, xb, 1, zero);
+                x.template sum<NT, 2, F32X>(sb4, sb, 1, nt, xb, K);
                 y[nt][0] = fmaf(sg.x, fmaf(-2208.0f, sa[0], ca[0]), fmaf(sg.y, fmaf(-2208.0f, sb4[0], cb[0]), y[nt][0]));
                 y[nt][1] = fmaf(sg.x, fmaf(-2208.0f, sa[1], ca[1]), fmaf(sg.y, fmaf(-2208.0f, sb4[1], cb[1]), y[nt][1]));
                 y[nt][2] = fmaf(sg8.x, fmaf(-2208.0f, sa[2], ca[2]), fmaf(sg8.y, fmaf(-2208.0f, sb4[2], cb[2]), y[nt][2]));
@@ -279,12 +312,12 @@ struct TileFmt<NNQ_Q6_K, 8> {
 //   Q4_1  y += d * (c - 128 s) + m * s
 template <int FMT>
 struct TileQ4x {
+    static constexpr int kSums = 1;
     static constexpr bool kMin = FMT == NNQ_Q4_1;
     static constexpr int kBytes = (kMin ? 512 : 256) + 2048;
     static constexpr int kElems = 256;
-    template <int NT, bool F32X>
-    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *, const uint8_t *const (&xrow)[NT],
-                                                int koff, int lane, int g, int t, const MnConsts &K,
+    template <int NT, bool F32X, class X>
+    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *, const X &x, int lane, int g, int t, const MnConsts &K,
                                                 float (&y)[NT][4]) {
         const uint4 *st = reinterpret_cast<const uint4 *>(stage);
         const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -320,13 +353,11 @@ struct TileQ4x {
             const float e = kMin ? fmaf(-128.0f, d, mn) : -136.0f * d, e8 = kMin ? fmaf(-128.0f, d8, mn8) : -136.0f * d8;
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const int e0 = koff + sb * 32 + 8 * t;
-                const XB<F32X> xb = load_xb<F32X>(xrow[nt], e0, e0 + 4);
+                const XB<F32X> xb = x.template frag<NT, F32X>(sb, nt, t);
                 float c[4], sx[4];
                 mma_x<F32X>(c, L[0], L8[0], L[1], L8[1], xb, 0, zero);
                 mma_x<F32X>(c, L[2], L8[2], L[3], L8[3], xb, 1, c);
-                mma_x<F32X>(sx, K.ones, K.ones, K.ones, K.ones, xb, 0, zero);
-                mma_x<F32X>(sx, K.ones, K.ones, K.ones, K.ones, xb, 1, sx);
+                x.template sum<NT, 1, F32X>(sx, sb, 0, nt, xb, K);
                 y[nt][0] = fmaf(d, c[0], fmaf(e, sx[0], y[nt][0]));
                 y[nt][1] = fmaf(d, c[1], fmaf(e, sx[1], y[nt][1]));
                 y[nt][2] = fmaf(d8, c[2], fmaf(e8, sx[2], y[nt][2]));
@@ -350,6 +381,7 @@ struct TileFmt<NNQ_Q4_1, 8> : TileQ4x<NNQ_Q4_1> {};
 // f32 accumulators.
 template <int SB>
 struct TileFmt<NNQ_MXFP4_SPLIT, SB> {
+    static constexpr int kSums = 0;
     static constexpr int kBytes = 128 + 256 * SB;
     static constexpr int kElems = 32 * SB;
     static __device__ __forceinline__ void pairs(uint32_t w, const MnConsts &K, uint32_t (&a)[4]) {
@@ -367,9 +399,8 @@ struct TileFmt<NNQ_MXFP4_SPLIT, SB> {
         const uint32_t bits = (i < 3 ? w << (23 - 8 * i) : w >> 1) & 0x7F800000u;
         return __uint_as_float(max(bits, 0x00400000u));
     }
-    template <int NT, bool F32X>
-    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *, const uint8_t *const (&xrow)[NT],
-                                                int koff, int lane, int g, int t, const MnConsts &K,
+    template <int NT, bool F32X, class X>
+    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *, const X &x, int lane, int g, int t, const MnConsts &K,
                                                 float (&y)[NT][4]) {
         const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         const uint2 sg = reinterpret_cast<const uint2 *>(stage)[g], sg8 = reinterpret_cast<const uint2 *>(stage)[g + 8];
@@ -383,8 +414,7 @@ struct TileFmt<NNQ_MXFP4_SPLIT, SB> {
             const float d = scale_of(sg, sb), d8 = scale_of(sg8, sb);
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const int e0 = koff + sb * 32 + 8 * t;
-                const XB<F32X> xb = load_xb<F32X>(xrow[nt], e0, e0 + 4);
+                const XB<F32X> xb = x.template frag<NT, F32X>(sb, nt, t);
                 float c[4];
                 mma_x<F32X>(c, A[0], A8[0], A[1], A8[1], xb, 0, zero);
                 mma_x<F32X>(c, A[2], A8[2], A[3], A8[3], xb, 1, c);
@@ -404,6 +434,7 @@ struct TileFmt<NNQ_MXFP4_SPLIT, SB> {
 // the accumulators need no further scaling.
 template <int SB>
 struct TileFmt<NNQ_MXFP4_GPTOSS, SB> {
+    static constexpr int kSums = 0;
     static constexpr int kBytes = 32 * SB + 256 * SB;
     static constexpr int kElems = 32 * SB;
     static __device__ __forceinline__ uint32_t scale_pair(uint32_t w, uint32_t sel) {   // two bytes -> bf16x2 2^(e-127)
@@ -413,9 +444,8 @@ struct TileFmt<NNQ_MXFP4_GPTOSS, SB> {
         __nv_bfloat162 r = __hmul2(*reinterpret_cast<__nv_bfloat162 *>(&a), *reinterpret_cast<__nv_bfloat162 *>(&b));
         return *reinterpret_cast<uint32_t *>(&r);
     }
-    template <int NT, bool F32X>
-    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *, const uint8_t *const (&xrow)[NT],
-                                                int koff, int lane, int g, int t, const MnConsts &K,
+    template <int NT, bool F32X, class X>
+    static __device__ __forceinline__ void tile(const uint8_t *stage, float4 *, const X &x, int lane, int g, int t, const MnConsts &K,
                                                 float (&y)[NT][4]) {
         const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         const uint2 *cw = reinterpret_cast<const uint2 *>(stage + 32 * SB);
@@ -430,8 +460,7 @@ struct TileFmt<NNQ_MXFP4_GPTOSS, SB> {
             const uint32_t s2 = scale_pair(e8.y, 0x4140), s3 = scale_pair(e8.y, 0x4342);
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const int e0 = koff + sb * 32 + 8 * t;
-                XB<F32X> xb = load_xb<F32X>(xrow[nt], e0, e0 + 4);
+                XB<F32X> xb = x.template frag<NT, F32X>(sb, nt, t);
                 xb.hi = make_uint4(mul2(xb.hi.x, s0), mul2(xb.hi.y, s1), mul2(xb.hi.z, s2), mul2(xb.hi.w, s3));
                 if (F32X) xb.lo = make_uint4(mul2(xb.lo.x, s0), mul2(xb.lo.y, s1), mul2(xb.lo.z, s2), mul2(xb.lo.w, s3));
                 float c[4];
@@ -453,6 +482,122 @@ __device__ __forceinline__ void issue_tile_n(uint32_t dst, const void *src, uint
         " @q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], %4;\n"
         " @q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %4, [%2];\n}"
         ::"r"(dst), "l"(src), "r"(bar), "r"(pred), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void mn_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void mn_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Shared memory of a CTA of the grouped kernel: rings, activations of `chunk` tiles of K with their sums, scale scratch, partial sums.
+struct GroupedPlan {
+    int x_off, sums_off, sct_off, part_off, bar_off, total;
+};
+
+__host__ __device__ inline GroupedPlan grouped_plan(int tile_bytes, int stages, int nt, bool f32x, int sums, int blocks, bool parts) {
+    GroupedPlan p;
+    p.x_off = (kWarps * stages * tile_bytes + 127) & ~127;
+    p.sums_off = p.x_off + blocks * nt * (f32x ? 1024 : 512);
+    p.sct_off = p.sums_off + blocks * sums * nt * 32;
+    p.part_off = p.sct_off + kWarps * 1024;
+    p.bar_off = p.part_off + (parts ? 2 * kWarps * nt * 512 : 0);
+    p.total = p.bar_off + kWarps * kMaxStages * 8;
+    return p;
+}
+
+// A warp's ring of weight tiles: `next` gives the source of the following run of tiles (false: none left).
+template <int TB>
+struct MnRing {
+    uint32_t ring_s, bar_s;
+    const uint8_t *ring, *src;
+    int stages, left, run, lane0;   // tiles left of the run being asked for, tiles of a run
+    int pf_slot, slot;
+    uint32_t phase;
+    unsigned issued, consumed;
+    bool failed;
+    __device__ __forceinline__ void init(uint8_t *smem, uint64_t *bars, int warp, int lane, int stages_, int run_) {
+        stages = stages_;
+        run = run_;
+        ring = smem + warp * stages * TB;
+        ring_s = smem_u32(ring);
+        bar_s = smem_u32(bars + warp * kMaxStages);
+        lane0 = lane == 0;
+        left = pf_slot = slot = 0;
+        phase = 0;
+        issued = consumed = 0;
+        failed = false;
+        src = nullptr;
+        if (lane0) {
+            for (int d = 0; d < stages; d++) mbar_init(bar_s + 8 * d, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncwarp();
+    }
+    template <class Next>
+    __device__ __forceinline__ void issue(Next &&next) {
+        if (left == 0) {
+            if (!next(src)) return;
+            left = run;
+        }
+        issue_tile_n<TB>(ring_s + pf_slot * TB, src, bar_s + 8 * pf_slot, lane0);
+        issued++;
+        pf_slot = pf_slot + 1 == stages ? 0 : pf_slot + 1;
+        src += TB;
+        left--;
+    }
+    __device__ __forceinline__ const uint8_t *wait() {
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait_fast(bar_s + 8 * slot, phase))) failed = true;
+        return ring + slot * TB;
+    }
+    __device__ __forceinline__ void release() {
+        consumed++;
+        if (++slot == stages) {
+            slot = 0;
+            phase ^= 1u;
+        }
+        __syncwarp();   // all lanes have read the slot and the scale scratch
+    }
+    // gives the copies in flight a bounded chance to land before the CTA's shared memory goes away
+    __device__ __forceinline__ void drain() {
+        for (unsigned n = consumed; n < issued; n++) {
+            mbar_wait(bar_s + 8 * slot, phase);
+            if (++slot == stages) {
+                slot = 0;
+                phase ^= 1u;
+            }
+        }
+    }
+};
+
+// Puts tiles [t0, t0 + tiles) of K of the CTA's activation rows into shared memory; row(tok) = address of a token's row, or
+// NULL for a column that stays zero. All warps of the CTA.
+template <class TF, int NT, bool F32X, class Row>
+__device__ __forceinline__ void mn_stage(uint8_t *xs, float *sums, int t0, int tiles, int warp, int lane, int g, int t, const MnConsts &K, Row &&row) {
+    constexpr int SUMS = TF::kSums;
+    const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const int pairs = tiles * (TF::kElems / 32) * NT;
+    const uint8_t *xrow[NT];
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++) xrow[nt] = row(nt * 8 + g);
+#pragma unroll 4
+    for (int i = warp; i < pairs; i += kWarps) {
+        const int block = i / NT, nt = i % NT;
+        const uint8_t *r = nt ? xrow[NT - 1] : xrow[0];
+        XB<F32X> xb;
+        xb.hi = xb.lo = make_uint4(0, 0, 0, 0);
+        const int e = t0 * TF::kElems + block * 32;
+        if (r) xb = SUMS == 2 ? load_xb<F32X>(r, e + 4 * t, e + 4 * t + 16) : load_xb<F32X>(r, e + 8 * t, e + 8 * t + 4);
+        uint4 *dst = reinterpret_cast<uint4 *>(xs) + i * (F32X ? 64 : 32) + lane;
+        dst[0] = xb.hi;
+        if (F32X) dst[32] = xb.lo;
+        if (SUMS > 0) {
+            float c[2][4];
+            mma_x<F32X>(c[0], K.ones, K.ones, K.ones, K.ones, xb, 0, zero);
+            if (SUMS == 1) mma_x<F32X>(c[0], K.ones, K.ones, K.ones, K.ones, xb, 1, c[0]);
+            else mma_x<F32X>(c[1], K.ones, K.ones, K.ones, K.ones, xb, 1, zero);
+            if (g == 0) {
+#pragma unroll
+                for (int h = 0; h < SUMS; h++) *reinterpret_cast<float2 *>(sums + (block * SUMS + h) * NT * 8 + nt * 8 + 2 * t) = make_float2(c[h][0], c[h][1]);
+            }
+        }
+    }
 }
 
 struct MnPlan {
@@ -548,11 +693,11 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // activations of this lane's token column(s); a column beyond M reads token 0 and is never stored
-    const uint8_t *xrow[NT];
+    MnGlobalX<NT, TF::kSums == 2> x;
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) {
         const int tok = nt * 8 + g;
-        xrow[nt] = reinterpret_cast<const uint8_t *>(P.x) + (size_t)(tok < P.m ? tok : 0) * P.kblocks * TE * (F32X ? 4 : 2);
+        x.row[nt] = reinterpret_cast<const uint8_t *>(P.x) + (size_t)(tok < P.m ? tok : 0) * P.kblocks * TE * (F32X ? 4 : 2);
     }
     MnConsts K;
     K.init();
@@ -609,7 +754,8 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
 #pragma unroll 1
         for (int k = 0; k < nkb; k++) {
             ok &= mbar_wait_fast(bar_s + 8 * slot, phase);
-            TF::template tile<NT, F32X>(ring + slot * TB, sct4, xrow, (kb_lo + k) * TE, lane, g, t, K, y);
+            x.koff = (kb_lo + k) * TE;
+            TF::template tile<NT, F32X>(ring + slot * TB, sct4, x, lane, g, t, K, y);
             consumed++;
             if (++slot == stages) {
                 slot = 0;
@@ -651,13 +797,17 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
 // Grouped token-column kernel: the expert products of a mixture-of-experts block
 // ---------------------------------------------------------------------------------
 //
-// One launch covers every local expert. The routed rows arrive sorted by expert (offset[e] ..
-// offset[e+1], computed on the device by the grouping kernels); a unit is (expert, group of up
-// to 8 routed rows, row tile of the expert's weight), units are numbered expert-major, then
-// row group, then row tile, and CTA c handles units c, c + grid, ... The eight MMA columns are
-// the rows of the group; their activations are read through the row -> token table (first
-// product) or directly (second product). Everything else is the token-column kernel: per-warp
-// rings of bulk-copied tiles, K split over the 8 warps, partial tiles met in shared memory.
+// One launch covers every local expert. The routed rows arrive sorted by expert (offset[e] .. offset[e + 1], computed on the
+// device by the grouping kernels); a unit is (expert, group of up to 8 NT routed rows, eight row tiles of the expert's weight),
+// numbered in this order, and every cluster of `slices` CTAs takes a contiguous run of units, so that the rows of a group are
+// staged once or twice. The columns are the rows of the group, read through the row -> token table (first product) or directly
+// (second product).
+//
+// What bounds it: shared memory and integer instructions, about 220 clocks per SM and tile at 16 rows. A warp has a row tile of its
+// own and all of the CTA's K, so the eight warps share one copy of the activations, laid out as the MMA reads them, and their
+// sums are formed once per group; with K split over the warps every warp read the group's rows and summed them again for each row
+// tile (415 clocks). K is split over the CTAs of a cluster instead, which add up through each other's shared memory.
+// Block of 64 tokens, 32 experts of 2880, top 4: 334 -> 295 us; 32 tokens 272 -> 215, 128 518 -> 450, one token 66 -> 60.
 
 struct GroupedParams {
     const uint8_t *tiled;     // expert e at tiled + e * expert_stride
@@ -667,7 +817,7 @@ struct GroupedParams {
     const int *rowtok;        // routed row -> flat assignment index (token = index / top_k), or NULL: row itself
     const int *offset;        // [E + 1] first routed row of each expert
     float *out;               // [rows][n]
-    int experts, top_k, n, row_tiles, kblocks, stages;
+    int experts, top_k, n, row_tiles, kblocks, stages, slices, chunk;
     int *status;
 };
 
@@ -675,188 +825,171 @@ template <int FMT, int SB, int NT, bool F32X>
 __global__ void __launch_bounds__(kWarps * 32, 2)
 skinny_grouped_kernel(const __grid_constant__ GroupedParams P) {
     using TF = TileFmt<FMT, SB>;
-    constexpr int TB = TF::kBytes;
-    constexpr int TE = TF::kElems;
+    constexpr int TB = TF::kBytes, TE = TF::kElems, XT = SB * NT * (F32X ? 1024 : 512);
     constexpr int kGroupRows = 8 * NT;   // routed rows per unit
     extern __shared__ __align__(128) uint8_t smem[];
-    const MnPlan L = mn_plan(TB, P.stages, NT);
+    const GroupedPlan L = grouped_plan(TB, P.stages, NT, F32X, TF::kSums, P.chunk * SB, P.slices > 1);
     __shared__ int goff[kMoeMaxExperts + 1];   // first row group of each expert
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
     const int g = lane >> 2, t = lane & 3;
-    const int cta = blockIdx.x, grid = gridDim.x;
-    const int stages = P.stages;
-    uint8_t *ring = smem + warp * stages * TB;
+    const int slices = P.slices, rank = blockIdx.x % slices, cl = blockIdx.x / slices, ncl = gridDim.x / slices;
+    uint8_t *xs = smem + L.x_off;
+    float *sums = reinterpret_cast<float *>(smem + L.sums_off);
     float4 *sct4 = reinterpret_cast<float4 *>(smem + L.sct_off + warp * 1024);
     float4 *part4 = reinterpret_cast<float4 *>(smem + L.part_off);
-    const uint32_t ring_s = smem_u32(ring);
-    const uint32_t bars_s = smem_u32(smem + L.bar_off);
-    const uint32_t bar_s = bars_s + warp * kMaxStages * 8;
-    const uint32_t full_s = bars_s + kWarps * kMaxStages * 8;
-    const uint32_t empty_s = full_s + 16;
 
-    if (tid == 0) {
-        mbar_init(full_s, kWarps);
-        mbar_init(full_s + 8, kWarps);
-        mbar_init(empty_s, 1);
-        mbar_init(empty_s + 8, 1);
-    }
-    if (lane == 0) {
-        for (int d = 0; d < stages; d++) mbar_init(bar_s + 8 * d, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
+    const int kb_lo = rank * P.kblocks / slices, nkb = (rank + 1) * P.kblocks / slices - kb_lo;
+    MnRing<TB> R;
+    R.init(smem, reinterpret_cast<uint64_t *>(smem + L.bar_off), warp, lane, P.stages, nkb);
     // the routing tables come from the kernels before this one
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (tid == 0) {
-        int acc = 0;
-        for (int e = 0; e < P.experts; e++) {
-            goff[e] = acc;
-            acc += (P.offset[e + 1] - P.offset[e] + kGroupRows - 1) / kGroupRows;
+    if (warp == 0) {   // (at most 64 experts: two per lane)
+        int c[2], sum = 0;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int e = 2 * lane + i;
+            c[i] = e < P.experts ? (P.offset[e + 1] - P.offset[e] + kGroupRows - 1) / kGroupRows : 0;
+            sum += c[i];
         }
-        goff[P.experts] = acc;
+        int before = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int v = __shfl_up_sync(0xFFFFFFFFu, before, off);
+            if (lane >= off) before += v;
+        }
+        before -= sum;
+        if (2 * lane <= P.experts) goff[2 * lane] = before;
+        if (2 * lane + 1 <= P.experts) goff[2 * lane + 1] = before + c[0];
+        if (lane == 31 && P.experts == kMoeMaxExperts) goff[kMoeMaxExperts] = before + sum;
     }
     __syncthreads();
-    const int total_units = goff[P.experts] * P.row_tiles;
-
-    const int kb_lo = (warp * P.kblocks) / kWarps, kb_hi = ((warp + 1) * P.kblocks) / kWarps;
-    const int nkb = kb_hi - kb_lo;
-    const int n_units = cta < total_units ? (total_units - cta + grid - 1) / grid : 0;
-    // expert, first routed row, rows in the group and row tile of a unit. A CTA's units come in
-    // increasing order, so the expert is found by advancing a cursor (one for the copy stream, which
-    // runs ahead, one for the arithmetic).
-    auto locate = [&](int unit, int &ecur, int &r0, int &cnt, int &rt) {
-        const int u = cta + unit * grid;
-        const int q = u / P.row_tiles;
-        rt = u - q * P.row_tiles;
-        while (ecur + 1 < P.experts && q >= goff[ecur + 1]) ecur++;
-        r0 = P.offset[ecur] + (q - goff[ecur]) * kGroupRows;
-        cnt = min(kGroupRows, P.offset[ecur + 1] - r0);
+    const int per = (P.row_tiles + kWarps - 1) / kWarps;   // units of a row group
+    const int total = goff[P.experts] * per;
+    const int u0 = (int)((long long)total * cl / ncl), n_units = (int)((long long)total * (cl + 1) / ncl) - u0;
+    // expert, row group and row tile of a unit. Units come in increasing order, so the expert is found by advancing a cursor (one
+    // for the copies, which run ahead, one for the arithmetic).
+    auto locate = [&](int unit, int w, int &e, int &q, int &rt) {
+        const int u = u0 + unit;
+        q = u / per;
+        rt = (u - q * per) * kWarps + w;
+        while (e + 1 < P.experts && q >= goff[e + 1]) e++;
+        return rt < P.row_tiles;
     };
-    int e_pf = 0, e_main = 0;
-
-    int pf_unit = -1, pf_k = 0, pf_slot = 0;
-    unsigned issued = 0;
-    const uint8_t *pf_src = nullptr;
-    bool pf_done = nkb == 0 || n_units == 0;
-    auto pf_advance_unit = [&]() {
-        if (++pf_unit >= n_units) {
-            pf_done = true;
-            return;
+    int pf_unit = 0, e_pf = 0;
+    auto next = [&](const uint8_t *&src) {
+        int q, rt;
+        while (nkb > 0 && pf_unit < n_units) {
+            if (locate(pf_unit++, warp, e_pf, q, rt)) {
+                src = P.tiled + (size_t)e_pf * P.expert_stride + ((size_t)rt * P.kblocks + kb_lo) * TB;
+                return true;
+            }
         }
-        int r0, cnt, rt;
-        locate(pf_unit, e_pf, r0, cnt, rt);
-        pf_src = P.tiled + (size_t)e_pf * P.expert_stride + ((size_t)rt * P.kblocks + kb_lo) * TB;
-        pf_k = 0;
+        return false;
     };
-    if (!pf_done) pf_advance_unit();
-    const int is_lane0 = lane == 0;
-    auto issue = [&]() {
-        if (!pf_done) {
-            issue_tile_n<TB>(ring_s + pf_slot * TB, pf_src, bar_s + 8 * pf_slot, is_lane0);
-            issued++;
-            pf_slot = pf_slot + 1 == stages ? 0 : pf_slot + 1;
-            pf_src += TB;
-            if (++pf_k == nkb) pf_advance_unit();
-        }
-    };
-    for (int d = 0; d < stages; d++) issue();
+    for (int d = 0; d < P.stages; d++) R.issue(next);
 
     MnConsts K;
     K.init();
-    unsigned consumed = 0;
-    int slot = 0;
-    uint32_t phase = 0;
-    bool failed = false;
-    const size_t xstride = (size_t)P.kblocks * TE * (F32X ? 4 : 2);
+    const size_t ldx = (size_t)P.kblocks * TE * (F32X ? 4 : 2);
+    const bool whole = nkb <= P.chunk;
 
-    auto finish = [&](int unit, int e, int r0, int cnt, int rt) {
-        const int b = unit & 1;
-        if (!mbar_wait_fast(full_s + 8 * b, (unit >> 1) & 1u)) {
-            failed = true;
-            return;
+    auto put4 = [&](int e, int q, int rt, int nt, int l, float4 v) {
+        if (rt >= P.row_tiles) return;
+        const int r0 = P.offset[e] + (q - goff[e]) * kGroupRows, cnt = min(kGroupRows, P.offset[e + 1] - r0);
+        const int r = rt * 16 + (l >> 2), tok = nt * 8 + 2 * (l & 3);
+        const float vals[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int tk = tok + (i & 1), rw = r + (i >> 1) * 8;
+            if (tk < cnt && rw < P.n) P.out[(size_t)(r0 + tk) * P.n + rw] = P.bias ? vals[i] + __ldg(P.bias + (size_t)e * P.n + rw) : vals[i];
         }
-#pragma unroll
-        for (int nt = 0; nt < NT; nt++) {
+    };
+    auto reduce = [&](int unit, int e, int q) {
+        constexpr int T = kWarps * NT * 32;
+        const uint32_t base = smem_u32(part4 + (unit & 1) * T);
+        const int lo = rank * T / slices, hi = (rank + 1) * T / slices, rt0 = (u0 + unit - q * per) * kWarps;
+        for (int i = lo + tid; i < hi; i += kWarps * 32) {
             float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-            for (int w = 0; w < kWarps; w++) {
-                const float4 a = part4[((b * kWarps + w) * NT + nt) * 32 + lane];
+#pragma unroll 4
+            for (int z = 0; z < slices; z++) {
+                const float4 a = ld_cluster_f4(cluster_addr(base + 16 * i, (uint32_t)z));
                 v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
             }
-            const int row = rt * 16 + g, tok = nt * 8 + 2 * t;
-            const float vals[4] = {v.x, v.y, v.z, v.w};
+            put4(e, q, rt0 + i / (NT * 32), i / 32 % NT, i & 31, v);
+        }
+    };
+
+    int e = 0, q = 0, staged = -1, pe = 0, pq = 0;
+#pragma unroll 1
+    for (int unit = 0; unit < n_units; unit++) {
+        int rt;
+        const bool live = locate(unit, warp, e, q, rt);
+        const int r0 = P.offset[e] + (q - goff[e]) * kGroupRows, cnt = min(kGroupRows, P.offset[e + 1] - r0);
+        auto row = [&](int col) -> const uint8_t * {
+            if (col >= cnt) return nullptr;
+            const int src = P.rowtok ? __ldg(P.rowtok + r0 + col) / P.top_k : r0 + col;
+            return reinterpret_cast<const uint8_t *>(P.x) + (size_t)src * ldx;
+        };
+        float y[NT][4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int tk = tok + (i & 1), rw = row + (i >> 1) * 8;
-                if (tk < cnt && rw < P.n) {
-                    float o = vals[i];
-                    if (P.bias) o += __ldg(P.bias + (size_t)e * P.n + rw);
-                    P.out[(size_t)(r0 + tk) * P.n + rw] = o;
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+            for (int r = 0; r < 4; r++) y[nt][r] = 0.0f;
+        for (int k0 = 0; k0 < nkb; k0 += P.chunk) {
+            const int k1 = min(nkb, k0 + P.chunk);
+            if (!whole || staged != q) {
+                __syncthreads();
+                mn_stage<TF, NT, F32X>(xs, sums, kb_lo + k0, k1 - k0, warp, lane, g, t, K, row);
+                __syncthreads();
+                staged = q;
+            }
+            if (!live) continue;
+            MnSharedX x;
+            x.f = reinterpret_cast<const uint4 *>(xs) + lane;
+            x.s = sums + 2 * t;
+#pragma unroll 1
+            for (int k = k0; k < k1; k++) {
+                if (!R.failed) {
+                    const uint8_t *stage = R.wait();
+                    TF::template tile<NT, F32X>(stage, sct4, x, lane, g, t, K, y);
+                    x.f += XT / 16;
+                    x.s += SB * TF::kSums * NT * 8;
+                    if (!R.failed) {
+                        R.release();
+                        R.issue(next);
+                    }
                 }
             }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(empty_s + 8 * b);
-    };
-
-#pragma unroll 1
-    int pe = 0, pr0 = 0, pcnt = 0, prt = 0;   // the previous unit, for its deferred write-out
-    for (int unit = 0; unit < n_units && !failed; unit++) {
-        int r0, cnt, rt;
-        locate(unit, e_main, r0, cnt, rt);
-        // this lane's column(s): routed row r0 + g (+ 8); a column beyond the group reads row r0 and is never stored
-        const uint8_t *xrow[NT];
-        float y[NT][4];
+        if (slices == 1) {
 #pragma unroll
-        for (int nt = 0; nt < NT; nt++) {
-            const int col = nt * 8 + g;
-            const int r = r0 + (col < cnt ? col : 0);
-            const int src = P.rowtok ? __ldg(P.rowtok + r) / P.top_k : r;
-            xrow[nt] = reinterpret_cast<const uint8_t *>(P.x) + (size_t)src * xstride;
-#pragma unroll
-            for (int i = 0; i < 4; i++) y[nt][i] = 0.0f;
+            for (int nt = 0; nt < NT; nt++) put4(e, q, rt, nt, lane, make_float4(y[nt][0], y[nt][1], y[nt][2], y[nt][3]));
+            continue;
         }
-        bool ok = true;
-#pragma unroll 1
-        for (int k = 0; k < nkb; k++) {
-            ok &= mbar_wait_fast(bar_s + 8 * slot, phase);
-            TF::template tile<NT, F32X>(ring + slot * TB, sct4, xrow, (kb_lo + k) * TE, lane, g, t, K, y);
-            consumed++;
-            if (++slot == stages) {
-                slot = 0;
-                phase ^= 1u;
-            }
-            __syncwarp();
-            issue();
-        }
-        if (!ok) {
-            failed = true;
-            break;
-        }
-        const int b = unit & 1;
-        if (unit >= 2 && !mbar_wait_fast(empty_s + 8 * b, ((unit >> 1) - 1) & 1u)) {
-            failed = true;
-            break;
+        if (unit) {
+            mn_cluster_wait();
+            reduce(unit - 1, pe, pq);
         }
 #pragma unroll
         for (int nt = 0; nt < NT; nt++)
-            part4[((b * kWarps + warp) * NT + nt) * 32 + lane] = make_float4(y[nt][0], y[nt][1], y[nt][2], y[nt][3]);
+            part4[(((unit & 1) * kWarps + warp) * NT + nt) * 32 + lane] = make_float4(y[nt][0], y[nt][1], y[nt][2], y[nt][3]);
         __syncwarp();
-        if (lane == 0) mbar_arrive(full_s + 8 * b);
-        if (unit >= 1 && warp == (unit - 1) % kWarps) finish(unit - 1, pe, pr0, pcnt, prt);
-        pe = e_main; pr0 = r0; pcnt = cnt; prt = rt;
+        mn_cluster_arrive();
+        pe = e;
+        pq = q;
     }
-    if (!failed && n_units >= 1 && warp == (n_units - 1) % kWarps) finish(n_units - 1, pe, pr0, pcnt, prt);
-    if (failed) {
+    if (slices > 1 && n_units) {
+        mn_cluster_wait();
+        reduce(n_units - 1, pe, pq);
+        __syncwarp();
+        mn_cluster_arrive();
+        mn_cluster_wait();
+    }
+    if (R.failed) {
         if (lane == 0) atomicExch(P.status, 1);
-        for (unsigned n = consumed; n < issued; n++) {
-            mbar_wait(bar_s + 8 * slot, phase);
-            if (++slot == stages) {
-                slot = 0;
-                phase ^= 1u;
-            }
-        }
+        R.drain();
     }
 }
 
