@@ -27,6 +27,7 @@
 #include "decoder_common.cuh"
 #include "gemm_tc.h"
 #include "moe.h"
+#include "skinny.h"
 
 namespace nnq {
 nnq_status comm_view(nnq_comm *c, CommView *out);   // comm.cu
@@ -97,7 +98,7 @@ struct nnq_decoder {
 
 namespace nnq {
 
-constexpr int kAttnRanges = 32;   // CTAs per kv head in the decode step's attention
+constexpr int kAttnRanges = 37;   // CTAs per kv head in the decode step's attention: eight heads, two CTAs on each of 148 SMs
 constexpr int kAttnWarps = 4;
 // Rows of a prompt that go through the layers together: large enough that the products run on the
 // decode-once tensor path with several row tiles per weight tile.
@@ -112,7 +113,7 @@ constexpr int kArgmaxBlocks = 128;
 constexpr int kStateWords = 8;    // token, position, steps, context full, previous token
 constexpr int kWantRows = 64;     // rows of logits formed together
 
-// h = embedding row of the current token (first layer), or h += delta; xn = RMSNorm(h) * w.
+// h = embedding row of the current token (first layer), or h += delta (NULL: none); xn = RMSNorm(h) * w.
 // One CTA; every thread keeps its (up to 8) elements in registers between the two phases.
 __global__ void __launch_bounds__(1024)
 dec_norm_kernel(float *__restrict__ h, const float *__restrict__ delta, const __nv_bfloat16 *__restrict__ embed,
@@ -129,14 +130,14 @@ dec_norm_kernel(float *__restrict__ h, const float *__restrict__ delta, const __
         v[r] = 0.0f;
         wv[r] = 0.0f;
         if (i < hidden) {
-            v[r] = embed ? __bfloat162float(embed[(size_t)tok * hidden + i]) : h[i] + delta[i];
+            v[r] = embed ? __bfloat162float(embed[(size_t)tok * hidden + i]) : (delta ? h[i] + delta[i] : h[i]);
             wv[r] = w[i];
             h[i] = v[r];
             ss = fmaf(v[r], v[r], ss);
         }
     }
     for (int i = threadIdx.x + 8 * 1024; i < hidden; i += 1024) {   // wider models: the tail goes through memory
-        const float t = embed ? __bfloat162float(embed[(size_t)tok * hidden + i]) : h[i] + delta[i];
+        const float t = embed ? __bfloat162float(embed[(size_t)tok * hidden + i]) : (delta ? h[i] + delta[i] : h[i]);
         h[i] = t;
         ss = fmaf(t, t, ss);
     }
@@ -184,35 +185,94 @@ dec_qk_rope_kernel(const float *__restrict__ q, const float *__restrict__ k, con
     else kcache[((size_t)(head - n_heads) * max_seq + pos) * hd + d] = y;
 }
 
-// Grouped-query attention over the cache in one launch. The keys are taken in batches of 32; a
-// kv head's batches are dealt to kAttnRanges CTAs (contiguous ranges) and inside a CTA to its four
-// warps. For a batch, lane j forms the dot products of key j with every query head of the group (the
-// query vectors sit in shared memory, the key row is read once for the whole group), the batch joins
-// the running softmax of each head (maximum, sum), then the value rows are read coalesced (lane l
-// owns dimensions 4l .. 4l+3) and weighted with the probabilities passed by shuffle. The warps of a
-// CTA merge through shared memory into one record per head, (m, l, acc[hd]), in global memory; the
-// CTA that finishes last for its kv head (an arrival counter, reset by that CTA for the next
+// What the attention kernel of a fused step does before it attends: see ROPE below.
+struct NewRows {
+    const float *k, *v, *q_norm, *k_norm, *cosv, *sinv;
+    float eps;
+};
+
+// RMSNorm and half-split rotation of a head by one warp, four dimensions per lane
+__device__ __forceinline__ float4 dec_rope_head(const float *src, const float *w, float eps, float4 c, float4 s, int lane) {
+    const float4 x = *reinterpret_cast<const float4 *>(src + 4 * lane), wv = *reinterpret_cast<const float4 *>(w + 4 * lane);
+    float ss = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w)));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
+    const float rms = sqrtf(ss / 128.0f + eps);
+    const float n[4] = {(x.x / rms) * wv.x, (x.y / rms) * wv.y, (x.z / rms) * wv.z, (x.w / rms) * wv.w};
+    const float cc[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
+    float y[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {   // y1 = x1 cos - x2 sin; y2 = x1 sin + x2 cos
+        const float o = __shfl_xor_sync(0xFFFFFFFFu, n[i], 16);
+        y[i] = lane < 16 ? n[i] * cc[i] - o * sn[i] : o * sn[i] + n[i] * cc[i];
+    }
+    return make_float4(y[0], y[1], y[2], y[3]);
+}
+
+// Grouped-query attention over the cache in one launch. The keys are taken in batches of 16, dealt in turn to the four warps of
+// kAttnRanges CTAs per kv head. What bounds it is the time to the first bytes, so a warp asks for all keys and values of a batch at
+// once (32 16-byte loads per lane, whole 128-byte lines). Eight lanes share a key, 16 dimensions each, and form its dot products with
+// every query head of the group; the batch joins the running softmax of each head (maximum, sum); the probabilities go through
+// shared memory to all lanes, which own four dimensions of the values each. The warps of a CTA merge into one record per head,
+// (m, l, acc[hd]), in global memory; the CTA that finishes last for its kv head (an arrival counter, reset by that CTA for the next
 // launch) merges the records of all ranges and writes the output rows:
 // out[head, d] = sum_s acc_s[d] e^(m_s - M) / sum_s l_s e^(m_s - M).
-template <int G>
-__global__ void __launch_bounds__(kAttnWarps * 32)
-dec_attn_kernel(const float *__restrict__ qrot, const float *__restrict__ kcache, const float *__restrict__ vcache,
-                const int *__restrict__ state, float scale, float *__restrict__ part, unsigned int *__restrict__ arrived,
-                void *__restrict__ out, int act_dt, int hd, int max_seq) {
-    pdl_prologue();
+// ROPE: the kernel takes the products' rows instead of prepared queries. Every CTA norms and rotates the query heads of its kv head;
+// the CTA that has the batch of the current position also does so with the key head and appends key and value. The rest of
+// the cache is older than the kernel in front (a step writes each layer's cache once), so its batches are asked for before
+// that one has ended.
+// A step of eight Qwen3-8B-shaped layers behind 16 / 2048 / 8000 positions, with a lane per key, batches of 32, values loaded behind
+// the softmax, and rotation, norms, activation and sums in kernels of their own 653 / 701 / 809 us, now 550 / 565 / 651.
+template <int G, bool ROPE>
+__global__ void __launch_bounds__(kAttnWarps * 32, 2)
+dec_attn_kernel(const float *q, float *kcache, float *vcache, const NewRows nr, const int *state, float scale, float *part, unsigned int *arrived, void *out,
+                int act_dt, int hd, int max_seq) {
+    if (!ROPE) pdl_prologue();
     __shared__ __align__(16) float qs[G][128];
     __shared__ __align__(16) float wacc[kAttnWarps][G][128];
+    __shared__ __align__(16) float ps[kAttnWarps][16][G];
+    __shared__ __align__(16) float fresh[2][128];
     __shared__ float wm[kAttnWarps][G], wl[kAttnWarps][G];
     __shared__ int s_last;
     const int kvh = blockIdx.x, range = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ctx = state[1] + 1;
-    const int nb = (ctx + 31) >> 5;                              // batches of 32 keys in the context
-    const int bper = (nb + kAttnRanges - 1) / kAttnRanges;       // batches per range
-    const int used = (nb + bper - 1) / bper;                     // ranges that hold keys
-    const int b_lo = range * bper, b_hi = min(nb, b_lo + bper);
-    if (b_lo < b_hi) {
-        for (int i = threadIdx.x; i < G * 32; i += kAttnWarps * 32)
-            *reinterpret_cast<float4 *>(&qs[i >> 5][4 * (i & 31)]) = *reinterpret_cast<const float4 *>(qrot + (kvh * G + (i >> 5)) * hd + 4 * (i & 31));
+    const int sub = lane >> 3, seg = lane & 7;
+    const int ctx = state[1] + 1, old = ROPE ? ctx - 1 : ctx;    // keys in the cache
+    const int nb = (ctx + 15) >> 4;                              // batches of 16 keys in the context
+    const int used = min(kAttnRanges, (nb + kAttnWarps - 1) / kAttnWarps);   // ranges that hold keys
+    const int first = range * kAttnWarps + warp;
+    float4 kr[16], vr[16];
+    const float *kb = kcache + (size_t)kvh * max_seq * 128 + 4 * seg, *vb = vcache + (size_t)kvh * max_seq * 128 + 4 * lane;
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto fetch = [&](int b) {
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            const int key = b * 16 + 4 * p + sub;
+#pragma unroll
+            for (int i = 0; i < 4; i++) kr[4 * p + i] = key < old ? *reinterpret_cast<const float4 *>(kb + (size_t)key * 128 + 32 * i) : none;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; j++) vr[j] = b * 16 + j < old ? *reinterpret_cast<const float4 *>(vb + (size_t)(b * 16 + j) * 128) : none;
+    };
+    if (first < nb) fetch(first);
+    if (ROPE) pdl_prologue();
+    if (range < used) {
+        if (ROPE) {
+            const float4 c = *reinterpret_cast<const float4 *>(nr.cosv + (size_t)(ctx - 1) * 64 + 4 * (lane & 15));
+            const float4 s = *reinterpret_cast<const float4 *>(nr.sinv + (size_t)(ctx - 1) * 64 + 4 * (lane & 15));
+            for (int g = warp; g < G; g += kAttnWarps)
+                *reinterpret_cast<float4 *>(&qs[g][4 * lane]) = dec_rope_head(q + (size_t)(kvh * G + g) * 128, nr.q_norm, nr.eps, c, s, lane);
+            if ((nb - 1) % (kAttnRanges * kAttnWarps) / kAttnWarps == range && warp == kAttnWarps - 1) {
+                const size_t at = ((size_t)kvh * max_seq + ctx - 1) * 128 + 4 * lane;
+                const float4 k = dec_rope_head(nr.k + kvh * 128, nr.k_norm, nr.eps, c, s, lane), v = *reinterpret_cast<const float4 *>(nr.v + kvh * 128 + 4 * lane);
+                *reinterpret_cast<float4 *>(kcache + at) = k;
+                *reinterpret_cast<float4 *>(vcache + at) = v;
+                *reinterpret_cast<float4 *>(&fresh[0][4 * lane]) = k;
+                *reinterpret_cast<float4 *>(&fresh[1][4 * lane]) = v;
+            }
+        } else {
+            for (int i = threadIdx.x; i < G * 32; i += kAttnWarps * 32)
+                *reinterpret_cast<float4 *>(&qs[i >> 5][4 * (i & 31)]) = *reinterpret_cast<const float4 *>(q + (size_t)(kvh * G + (i >> 5)) * 128 + 4 * (i & 31));
+        }
         __syncthreads();
         float m[G], l[G];
         float4 acc[G];
@@ -220,62 +280,81 @@ dec_attn_kernel(const float *__restrict__ qrot, const float *__restrict__ kcache
         for (int g = 0; g < G; g++) {
             m[g] = -INFINITY;
             l[g] = 0.0f;
-            acc[g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            acc[g] = none;
         }
-        const float *kb = kcache + (size_t)kvh * max_seq * hd, *vb = vcache + (size_t)kvh * max_seq * hd;
-        for (int b = b_lo + warp; b < b_hi; b += kAttnWarps) {
-            const int b0 = b << 5, j1 = min(ctx, b0 + 32);
-            const int j = b0 + lane;
-            const bool valid = j < j1;
-            const float4 *krow = reinterpret_cast<const float4 *>(kb + (size_t)(valid ? j : b0) * hd);
-            // the value rows of the batch are wanted after the softmax: ask L2 for them now (lane j: row j)
-            if (valid) {
-                const char *vrow = reinterpret_cast<const char *>(vb + (size_t)j * hd);
+#pragma unroll 1
+        for (int b = first; b < nb; b += kAttnRanges * kAttnWarps) {
+            if (b != first) fetch(b);
+            if (ROPE && b == nb - 1) {
 #pragma unroll
-                for (int c = 0; c < 4; c++) asm volatile("prefetch.global.L2 [%0];" ::"l"(vrow + 128 * c));
+                for (int p = 0; p < 4; p++)
+                    if (b * 16 + 4 * p + sub == ctx - 1)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) kr[4 * p + i] = *reinterpret_cast<const float4 *>(&fresh[0][32 * i + 4 * seg]);
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (b * 16 + j == ctx - 1) vr[j] = *reinterpret_cast<const float4 *>(&fresh[1][4 * lane]);
             }
-            float dot[G];
+            float dot[4][G];
 #pragma unroll
-            for (int g = 0; g < G; g++) dot[g] = 0.0f;
-#pragma unroll 16
-            for (int d4 = 0; d4 < 32; d4++) {
-                const float4 kv = krow[d4];
+            for (int p = 0; p < 4; p++)
+#pragma unroll
+                for (int g = 0; g < G; g++) dot[p][g] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
 #pragma unroll
                 for (int g = 0; g < G; g++) {
-                    const float4 qv = *reinterpret_cast<const float4 *>(&qs[g][4 * d4]);
-                    dot[g] = fmaf(qv.x, kv.x, fmaf(qv.y, kv.y, fmaf(qv.z, kv.z, fmaf(qv.w, kv.w, dot[g]))));
+                    const float4 qv = *reinterpret_cast<const float4 *>(&qs[g][32 * i + 4 * seg]);
+#pragma unroll
+                    for (int p = 0; p < 4; p++) {
+                        const float4 kv = kr[4 * p + i];
+                        dot[p][g] = fmaf(qv.x, kv.x, fmaf(qv.y, kv.y, fmaf(qv.z, kv.z, fmaf(qv.w, kv.w, dot[p][g]))));
+                    }
                 }
-            }
-            float p[G];
 #pragma unroll
             for (int g = 0; g < G; g++) {
-                const float s = valid ? dot[g] * scale : -INFINITY;
-                float bm = s;
+                float bm = -INFINITY;
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, off));
+                for (int p = 0; p < 4; p++) {
+#pragma unroll
+                    for (int off = 1; off < 8; off <<= 1) dot[p][g] += __shfl_xor_sync(0xFFFFFFFFu, dot[p][g], off);
+                    dot[p][g] = b * 16 + 4 * p + sub < ctx ? dot[p][g] * scale : -INFINITY;
+                    bm = fmaxf(bm, dot[p][g]);
+                }
+                bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, 8));
+                bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, 16));
                 const float mn = fmaxf(m[g], bm);   // finite: the batch holds at least one key
                 const float corr = expf(m[g] - mn);
-                p[g] = expf(s - mn);
-                float ps = p[g];
+                float sum = 0.0f;
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) ps += __shfl_xor_sync(0xFFFFFFFFu, ps, off);
-                l[g] = l[g] * corr + ps;
+                for (int p = 0; p < 4; p++) {
+                    dot[p][g] = expf(dot[p][g] - mn);
+                    sum += dot[p][g];
+                }
+                sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 8);
+                sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 16);
+                l[g] = l[g] * corr + sum;
                 acc[g].x *= corr; acc[g].y *= corr; acc[g].z *= corr; acc[g].w *= corr;
                 m[g] = mn;
             }
-            const int nk = j1 - b0;
-#pragma unroll 4
-            for (int jj = 0; jj < nk; jj++) {
-                const float4 vv = *reinterpret_cast<const float4 *>(vb + (size_t)(b0 + jj) * hd + 4 * lane);
+            __syncwarp();   // the probabilities of the batch before have been read
+            if (seg == 0) {
+#pragma unroll
+                for (int p = 0; p < 4; p++)
+#pragma unroll
+                    for (int g = 0; g < G; g++) ps[warp][4 * p + sub][g] = dot[p][g];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 16; j++)
 #pragma unroll
                 for (int g = 0; g < G; g++) {
-                    const float pj = __shfl_sync(0xFFFFFFFFu, p[g], jj);
-                    acc[g].x = fmaf(pj, vv.x, acc[g].x);
-                    acc[g].y = fmaf(pj, vv.y, acc[g].y);
-                    acc[g].z = fmaf(pj, vv.z, acc[g].z);
-                    acc[g].w = fmaf(pj, vv.w, acc[g].w);
+                    const float pj = ps[warp][j][g];
+                    acc[g].x = fmaf(pj, vr[j].x, acc[g].x);
+                    acc[g].y = fmaf(pj, vr[j].y, acc[g].y);
+                    acc[g].z = fmaf(pj, vr[j].z, acc[g].z);
+                    acc[g].w = fmaf(pj, vr[j].w, acc[g].w);
                 }
-            }
         }
         // the warps of the CTA -> one record per head
 #pragma unroll
@@ -304,7 +383,7 @@ dec_attn_kernel(const float *__restrict__ qrot, const float *__restrict__ kcache
                 o[0] = M;
                 o[1] = L;
             }
-            if (dd < hd) o[4 + dd] = a;
+            o[4 + dd] = a;
         }
     }
     // arrival: the records above are published before the count, the last CTA reads them after it
@@ -314,46 +393,50 @@ dec_attn_kernel(const float *__restrict__ qrot, const float *__restrict__ kcache
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // a warp per head, a lane per four dimensions; every load of a pass is issued before the first
-    // is used (the records sit in L2: the pass costs one round trip, not one per range)
+    // a warp per head: lane s has the maxima and sums of records s and s + 32, then four dimensions of every record
+    static_assert(kAttnRanges <= 64, "two records per lane");
     for (int g = warp; g < G; g += kAttnWarps) {
         const float *rec = part + ((size_t)(kvh * kAttnRanges) * G + g) * (hd + 4);
         const size_t step = (size_t)G * (hd + 4);
-        float2 ml[kAttnRanges];
+        float2 e0 = lane < used ? __ldcg(reinterpret_cast<const float2 *>(rec + lane * step)) : make_float2(-INFINITY, 0.0f);
+        float2 e1 = lane + 32 < used ? __ldcg(reinterpret_cast<const float2 *>(rec + (lane + 32) * step)) : make_float2(-INFINITY, 0.0f);
+        float M = fmaxf(e0.x, e1.x);
 #pragma unroll
-        for (int s = 0; s < kAttnRanges; s++)
-            ml[s] = s < used ? __ldcg(reinterpret_cast<const float2 *>(rec + s * step)) : make_float2(-INFINITY, 0.0f);
-        float M = ml[0].x;
+        for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, off));
+        e0.x = expf(e0.x - M);
+        e1.x = expf(e1.x - M);
+        float L = fmaf(e0.x, e0.y, e1.x * e1.y);
 #pragma unroll
-        for (int s = 1; s < kAttnRanges; s++) M = fmaxf(M, ml[s].x);
-        float L = 0.0f;
+        for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xFFFFFFFFu, L, off);
+        float4 a = none;
+        for (int h = 0; h < used; h += 20) {
+            float4 v[20];
 #pragma unroll
-        for (int s = 0; s < kAttnRanges; s++) {
-            ml[s].x = s < used ? expf(ml[s].x - M) : 0.0f;
-            L = fmaf(ml[s].y, ml[s].x, L);
-        }
-        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int s = 0; s < 20; s++) v[s] = h + s < used ? __ldcg(reinterpret_cast<const float4 *>(rec + (h + s) * step + 4) + lane) : none;
 #pragma unroll
-        for (int h = 0; h < kAttnRanges; h += 16) {
-            float4 v[16];
-#pragma unroll
-            for (int s = 0; s < 16; s++)
-                v[s] = h + s < used ? __ldcg(reinterpret_cast<const float4 *>(rec + (h + s) * step + 4) + lane) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-            for (int s = 0; s < 16; s++) {
-                a.x = fmaf(v[s].x, ml[h + s].x, a.x);
-                a.y = fmaf(v[s].y, ml[h + s].x, a.y);
-                a.z = fmaf(v[s].z, ml[h + s].x, a.z);
-                a.w = fmaf(v[s].w, ml[h + s].x, a.w);
+            for (int s = 0; s < 20; s++) {
+                const float w = __shfl_sync(0xFFFFFFFFu, h + s < 32 ? e0.x : e1.x, (h + s) & 31);
+                a.x = fmaf(v[s].x, w, a.x);
+                a.y = fmaf(v[s].y, w, a.y);
+                a.z = fmaf(v[s].z, w, a.z);
+                a.w = fmaf(v[s].w, w, a.w);
             }
         }
-        const int at = (kvh * G + g) * hd + 4 * lane;
+        const int at = (kvh * G + g) * 128 + 4 * lane;
         store_act(out, act_dt, at, a.x / L);
         store_act(out, act_dt, at + 1, a.y / L);
         store_act(out, act_dt, at + 2, a.z / L);
         store_act(out, act_dt, at + 3, a.w / L);
     }
     if (threadIdx.x == 0) arrived[kvh] = 0;   // the next launch starts after this grid has ended
+}
+
+template <int G>
+static void launch_dec_attn(nnq_decoder *d, bool rope, float *kc, float *vc, const NewRows &nr, float scale, cudaStream_t st) {
+    const dim3 grid(d->lkv, kAttnRanges), block(kAttnWarps * 32);
+    const int hd = d->cfg.head_dim, max_seq = d->cfg.max_seq;
+    if (rope) launch_pdl(dec_attn_kernel<G, true>, grid, block, st, d->d_q, kc, vc, nr, d->d_state, scale, d->d_part, d->d_arrived, d->d_attn, d->act_dt, hd, max_seq);
+    else launch_pdl(dec_attn_kernel<G, false>, grid, block, st, d->d_qrot, kc, vc, nr, d->d_state, scale, d->d_part, d->d_arrived, d->d_attn, d->act_dt, hd, max_seq);
 }
 
 __global__ void dec_silu_mul_kernel(const float *__restrict__ g, const float *__restrict__ u, void *__restrict__ mid,
@@ -1500,6 +1583,20 @@ static nnq_status rows_blocks(nnq_decoder *d, int n, int pos0, cudaStream_t st) 
     return NNQ_OK;
 }
 
+// One GPU, bf16 activations and the Q4_K kernels for the products: norms, rotation, activation and residual sums are parts of the
+// kernels around them (five launches a layer instead of nine).
+static bool step_is_fused(const nnq_decoder *d) {
+    const nnq_decoder_config &c = d->cfg;
+    if (d->blocks || d->comm || c.tp_world > 1 || d->act_dt != NNQ_BF16 || d->ctx->path != NNQ_PATH_AUTO || c.head_dim != 128) return false;
+    for (int l = 0; l < c.n_layers; l++) {
+        const nnq_decoder::Layer &L = d->layers[l];
+        for (const nnq_weight *w : {L.q, L.k, L.v, L.gate, L.up})
+            if (!skinny_norm_supported(w)) return false;
+        if (!skinny_supported(L.o, 1, NNQ_BF16) || !skinny_supported(L.down, 1, NNQ_BF16)) return false;
+    }
+    return true;
+}
+
 static nnq_status step_qwen3(nnq_decoder *d, cudaStream_t st) {
     nnq_ctx *ctx = d->ctx;
     const nnq_decoder_config &c = d->cfg;
@@ -1509,26 +1606,42 @@ static nnq_status step_qwen3(nnq_decoder *d, cudaStream_t st) {
     const size_t layer_cache = (size_t)lkv * c.max_seq * hd;
     const float scale = (float)(1.0 / sqrt((double)hd));
     const __nv_bfloat16 *embed = (const __nv_bfloat16 *)d->d_embed;
+    const bool fused = step_is_fused(d);
     for (int l = 0; l < c.n_layers; l++) {
         const nnq_decoder::Layer &L = d->layers[l];
-        DEC_RUN(1, launch_pdl(dec_norm_kernel, dim3(1), dim3(1024), st, d->d_h, d->d_delta, l == 0 ? embed : nullptr, d->d_state, L.in_norm, c.rms_eps, d->d_xn, d->act_dt, c.hidden));
+        if (!fused || l == 0) DEC_RUN(1, launch_pdl(dec_norm_kernel, dim3(1), dim3(1024), st, d->d_h, d->d_delta, l == 0 ? embed : nullptr, d->d_state, L.in_norm, c.rms_eps, d->d_xn, d->act_dt, c.hidden));
         const nnq_weight *w3[3] = {L.q, L.k, L.v};
         const void *x3[3] = {d->d_xn, d->d_xn, d->d_xn};
         void *y3[3] = {d->d_q, d->d_k, d->d_v};
-        DEC_RUN(32, if ((s = nnq_linear_batch(ctx, 3, w3, x3, adt, 1, nullptr, y3, NNQ_F32, st)) != NNQ_OK) return s);
-        DEC_RUN(2, launch_pdl(dec_qk_rope_kernel, dim3(lh + 2 * lkv), dim3(hd), st, d->d_q, d->d_k, d->d_v, L.q_norm, L.k_norm, d->d_cos, d->d_sin, d->d_state,
+        if (fused) {
+            const SkinnyJob j3[3] = {{L.q, d->d_h, nullptr, d->d_q}, {L.k, d->d_h, nullptr, d->d_k}, {L.v, d->d_h, nullptr, d->d_v}};
+            const StepPart part = {L.in_norm, c.rms_eps, 0, 0};
+            DEC_RUN(32, if ((s = launch_skinny_step(ctx, j3, 3, part, NNQ_F32, st)) != NNQ_OK) return s);
+        } else {
+            DEC_RUN(32, if ((s = nnq_linear_batch(ctx, 3, w3, x3, adt, 1, nullptr, y3, NNQ_F32, st)) != NNQ_OK) return s);
+        }
+        if (!fused) DEC_RUN(2, launch_pdl(dec_qk_rope_kernel, dim3(lh + 2 * lkv), dim3(hd), st, d->d_q, d->d_k, d->d_v, L.q_norm, L.k_norm, d->d_cos, d->d_sin, d->d_state,
                               c.rms_eps, d->d_qrot, d->d_kcache + l * layer_cache, d->d_vcache + l * layer_cache, lh, lkv, hd, c.max_seq));
         DEC_RUN(4, {
-            const dim3 ag(lkv, kAttnRanges), ab(kAttnWarps * 32);
-            const float *kc = d->d_kcache + l * layer_cache, *vc = d->d_vcache + l * layer_cache;
+            float *kc = d->d_kcache + l * layer_cache, *vc = d->d_vcache + l * layer_cache;
+            const NewRows nr = {d->d_k, d->d_v, L.q_norm, L.k_norm, d->d_cos, d->d_sin, c.rms_eps};
             switch (group) {
-                case 1: launch_pdl(dec_attn_kernel<1>, ag, ab, st, d->d_qrot, kc, vc, d->d_state, scale, d->d_part, d->d_arrived, d->d_attn, d->act_dt, hd, c.max_seq); break;
-                case 2: launch_pdl(dec_attn_kernel<2>, ag, ab, st, d->d_qrot, kc, vc, d->d_state, scale, d->d_part, d->d_arrived, d->d_attn, d->act_dt, hd, c.max_seq); break;
-                case 4: launch_pdl(dec_attn_kernel<4>, ag, ab, st, d->d_qrot, kc, vc, d->d_state, scale, d->d_part, d->d_arrived, d->d_attn, d->act_dt, hd, c.max_seq); break;
-                case 8: launch_pdl(dec_attn_kernel<8>, ag, ab, st, d->d_qrot, kc, vc, d->d_state, scale, d->d_part, d->d_arrived, d->d_attn, d->act_dt, hd, c.max_seq); break;
+                case 1: launch_dec_attn<1>(d, fused, kc, vc, nr, scale, st); break;
+                case 2: launch_dec_attn<2>(d, fused, kc, vc, nr, scale, st); break;
+                case 4: launch_dec_attn<4>(d, fused, kc, vc, nr, scale, st); break;
+                case 8: launch_dec_attn<8>(d, fused, kc, vc, nr, scale, st); break;
                 default: return fail(ctx, NNQ_ERR_UNSUPPORTED, "query heads per key/value head must be 1, 2, 4 or 8");
             }
         });
+        if (fused) {
+            const SkinnyJob jo = {L.o, d->d_attn, nullptr, d->d_h}, j2[2] = {{L.gate, d->d_h, nullptr, d->d_mid}, {L.up, d->d_h, nullptr, d->d_mid}}, jd = {L.down, d->d_mid, nullptr, d->d_h};
+            const StepPart add = {nullptr, 0.0f, 0, 1}, pg = {L.post_norm, c.rms_eps, 1, 0};
+            DEC_RUN(32, if ((s = launch_skinny_step(ctx, &jo, 1, add, NNQ_F32, st)) != NNQ_OK) return s);
+            DEC_RUN(32, if ((s = launch_skinny_step(ctx, j2, 2, pg, NNQ_BF16, st)) != NNQ_OK) return s);
+            DEC_RUN(32, if ((s = launch_skinny_step(ctx, &jd, 1, add, NNQ_F32, st)) != NNQ_OK) return s);
+            ctx->launches += l == 0 ? 2 : 1;
+            continue;
+        }
         // row-parallel products: with tensor parallelism the partial sums are exchanged inside the kernel
         DEC_RUN(32, s = d->comm ? nnq_comm_linear(d->comm, L.o, d->d_attn, adt, 1, nullptr, d->d_delta, NNQ_F32, st)
                                 : nnq_linear(ctx, L.o, d->d_attn, adt, 1, nullptr, d->d_delta, NNQ_F32, st));
@@ -1657,7 +1770,7 @@ nnq_status nnq_decoder_step(nnq_decoder *d, void *stream) {
         return launch_argmax(d, vocab_parallel, cv, st);
     }
     if ((s = step_qwen3(d, st)) != NNQ_OK) return s;
-    launch_pdl(dec_norm_kernel, dim3(1), dim3(1024), st, d->d_h, d->d_delta, nullptr, d->d_state, d->d_final_norm, c.rms_eps, d->d_xn, d->act_dt, c.hidden);
+    launch_pdl(dec_norm_kernel, dim3(1), dim3(1024), st, d->d_h, step_is_fused(d) ? nullptr : d->d_delta, nullptr, d->d_state, d->d_final_norm, c.rms_eps, d->d_xn, d->act_dt, c.hidden);
     ctx->launches++;
     return launch_head(d, vocab_parallel, cv, st);
 }

@@ -165,13 +165,13 @@ bool skinny_supported(const nnq_weight *w, int64_t m, int x_dt) {
     return st > 0;
 }
 
-template <bool F32X, int KS, bool FUSED = false>
+template <bool F32X, int KS, bool FUSED = false, int STEP = 0>
 static cudaError_t launch_kernel(const SkinnyParams &P, int grid, int smem_bytes, cudaStream_t stream) {
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(skinny_q4k_m1_kernel<F32X, KS, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax - 1024);
+        cudaError_t e = cudaFuncSetAttribute(skinny_q4k_m1_kernel<F32X, KS, FUSED, STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax - 1024);
         if (e != cudaSuccess) return e;
         configured[dev] = true;
     }
@@ -188,7 +188,7 @@ static cudaError_t launch_kernel(const SkinnyParams &P, int grid, int smem_bytes
     cfg.attrs = attr;
     static const char *env_pdl = diag_env("NNQ_SKINNY_PDL");  // tuning aid
     cfg.numAttrs = env_pdl && atoi(env_pdl) == 0 ? 0 : 1;
-    return cudaLaunchKernelEx(&cfg, skinny_q4k_m1_kernel<F32X, KS, FUSED>, P);
+    return cudaLaunchKernelEx(&cfg, skinny_q4k_m1_kernel<F32X, KS, FUSED, STEP>, P);
 }
 
 template <bool F32X, bool FUSED>
@@ -255,10 +255,12 @@ __global__ void __launch_bounds__(256) stream_read_kernel(const SkinnyParams P, 
 
 // One launch: jobs that share their activations (same x pointer, same K).
 static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int x_dt, int m, int y_dt,
-                               cudaStream_t stream, const FusedReduce *fr = nullptr) {
+                               cudaStream_t stream, const FusedReduce *fr = nullptr, const StepPart *step = nullptr) {
     SkinnyParams P;
     memset(&P, 0, sizeof(P));
     if (fr) P.fr = *fr;
+    if (step) P.step = *step;
+    const bool norm = step && step->norm_w;
     P.njobs = count;
     P.m = m;
     P.y_dt = y_dt;
@@ -280,7 +282,7 @@ static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, i
     int64_t job_tiles = 0;
     for (int i = 0; i < count; i++) job_tiles += (jobs[i].w->n + 15) / 16;
     const int64_t tokcol_limit = env_tc ? atoi(env_tc) : 2 * ctx->sm_count;
-    const bool token_columns = m > 1 || layout != kTiledQ4K || (!f32x && !fr && job_tiles <= tokcol_limit);
+    const bool token_columns = m > 1 || layout != kTiledQ4K || (!f32x && !fr && !norm && job_tiles <= tokcol_limit);
     if (!token_columns) pick_stages(P.kblocks, f32x, &P.stages, &ctas_per_sm);
     else P.stages = 2;
     if (fr && ctas_per_sm > 2) ctas_per_sm = 2;   // register budget of the fused variant
@@ -332,14 +334,16 @@ static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, i
     if (env_ks && atoi(env_ks) > 0) ksplit = atoi(env_ks);
     // persistent grid: every CTA resident
     const int rg = kWarps / ksplit;
-    const int units = (tiles + rg - 1) / rg;
+    const int units = norm && step->pair ? P.job[0].row_tiles : (tiles + rg - 1) / rg;
     int grid = units < slots ? units : slots;
     static const char *env_grid = diag_env("NNQ_SKINNY_GRID");  // tuning aid
     if (env_grid && atoi(env_grid) > 0) grid = atoi(env_grid);
     if (grid > units) grid = units;
     if (grid < 1) grid = 1;
     int smem_bytes = smem_plan(P.kblocks, P.stages, f32x).total;
-    cudaError_t e = f32x ? launch_ks<true>(ksplit, P, grid, smem_bytes, stream) : launch_ks<false>(ksplit, P, grid, smem_bytes, stream);
+    cudaError_t e;
+    if (norm) e = step->pair ? launch_kernel<false, kWarps, false, 2>(P, grid, smem_bytes, stream) : launch_kernel<false, kWarps, false, 1>(P, grid, smem_bytes, stream);
+    else e = f32x ? launch_ks<true>(ksplit, P, grid, smem_bytes, stream) : launch_ks<false>(ksplit, P, grid, smem_bytes, stream);
     ctx->launches++;
     return check_cuda(ctx, e, "skinny launch");
 }
@@ -478,6 +482,14 @@ nnq_status launch_skinny_fused(nnq_ctx *ctx, const SkinnyJob &job, int x_dt, int
                                cudaStream_t stream) {
     if (!skinny_fused_supported(job.w, 1, x_dt)) return fail(ctx, NNQ_ERR_UNSUPPORTED, "fused product + all-reduce needs the M = 1 Q4_K kernel");
     return launch_group(ctx, &job, 1, x_dt, 1, y_dt, stream, &fr);
+}
+
+// (eight warps share each row tile: at least a super-block of K for each, see launch_group)
+bool skinny_norm_supported(const nnq_weight *w) { return w && w->tiled_layout == kTiledQ4K && w->k >= 256 * kWarps && skinny_supported(w, 1, NNQ_BF16); }
+
+nnq_status launch_skinny_step(nnq_ctx *ctx, const SkinnyJob *jobs, int count, const StepPart &step, int y_dt, cudaStream_t stream) {
+    if (count < 1 || count > kSkinnyMaxJobs) return fail(ctx, NNQ_ERR_INVALID_ARG, "bad job count %d", count);
+    return launch_group(ctx, jobs, count, NNQ_BF16, 1, y_dt, stream, nullptr, &step);
 }
 
 nnq_status launch_skinny(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int x_dt, int64_t m, int y_dt,

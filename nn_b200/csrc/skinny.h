@@ -59,6 +59,21 @@ bool skinny_supported(const nnq_weight *w, int64_t m, int x_dt);
 nnq_status launch_skinny(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int x_dt, int64_t m, int y_dt,
                          cudaStream_t stream);
 
+// What a decode step does around its one-token products, inside their kernels:
+//   norm_w   x is the f32 residual row; the product is of x * norm_w / rms(x). Every warp of the M = 1 kernel multiplies its part
+//            of x by norm_w as it stages it and sums its squares; the one number 1 / rms is applied to the finished sums.
+//   pair     jobs 0 and 1 (gate, up) have equal rows: y of job 0 = silu(gate) * up as bf16
+//   add      y (f32) += the product
+struct StepPart {
+    const float *norm_w;
+    float eps;
+    int pair, add;
+};
+// True when launch_skinny_step can read a residual row of w->k values for this weight.
+bool skinny_norm_supported(const nnq_weight *w);
+// One token; x is f32 with step.norm_w, else bf16.
+nnq_status launch_skinny_step(nnq_ctx *ctx, const SkinnyJob *jobs, int count, const StepPart &step, int y_dt, cudaStream_t stream);
+
 // Row-parallel product fused with its all-reduce (M = 1 Q4_K kernel): the warp that finishes a row
 // tile sends its 16 f32 partial sums to every peer as 8-byte (value, sequence number) stores, waits
 // (bounded) for the peers' pairs of the same rows, adds them in rank order, adds the bias and

@@ -38,6 +38,7 @@ struct SkinnyParams {
                         // bit 1 = do not wait for the previous kernel; 4 = plain streaming read
     int l2_prefetch;    // 1 = ask L2 for the warp's whole weight stream at kernel start
     int *status;
+    StepPart step;      // a decode step's work around its product
     FusedReduce fr;     // row-parallel product + all-reduce in one kernel (M = 1 kernel, one job)
 };
 

@@ -711,6 +711,7 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
         if (tok < P.m && row < J.n) {
             if (J.bias) v += __ldg(J.bias + row);
             const size_t at = (size_t)tok * J.n + row;
+            if (P.step.add) v += reinterpret_cast<const float *>(J.y)[at];
             if (P.y_dt == NNQ_F32) reinterpret_cast<float *>(J.y)[at] = v;
             else reinterpret_cast<__nv_bfloat16 *>(J.y)[at] = __float2bfloat16_rn(v);
         }
