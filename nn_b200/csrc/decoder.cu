@@ -1597,6 +1597,25 @@ static bool step_is_fused(const nnq_decoder *d) {
     return true;
 }
 
+// `part` with the tiled copies of up to three weights as the next ones, at most kNextBytes of them in all. A token of the Qwen3-8B
+// shape (36 layers, 2048 positions) with 0 / 4 / 8 / 16 / 32 / 64 MB: 1953 / 1943 / 1932 / 1919 / 1951 / 1985 us; more than the
+// products in between leave in L2 is read twice.
+constexpr int kNextBytes = 16 << 20;
+static StepPart next_weights(StepPart part, const nnq_weight *a, const nnq_weight *b, const nnq_weight *e) {
+    static const char *env = diag_env("NNQ_NEXT_MB");   // tuning aid
+    const size_t most = env ? (size_t)atoi(env) << 20 : (size_t)kNextBytes;
+    const nnq_weight *w[3] = {a, b, e};
+    size_t total = 0;
+    for (const nnq_weight *x : w)
+        if (x && x->d_tiled) total += x->tiled_bytes;
+    for (int i = 0; i < 3; i++)
+        if (w[i] && w[i]->d_tiled) {
+            const size_t n = total > most ? (size_t)((double)w[i]->tiled_bytes * most / total) : w[i]->tiled_bytes;
+            part.next[i] = {w[i]->d_tiled, (unsigned)(n / 16 * 16), 0};
+        }
+    return part;
+}
+
 static nnq_status step_qwen3(nnq_decoder *d, cudaStream_t st) {
     nnq_ctx *ctx = d->ctx;
     const nnq_decoder_config &c = d->cfg;
@@ -1615,7 +1634,7 @@ static nnq_status step_qwen3(nnq_decoder *d, cudaStream_t st) {
         void *y3[3] = {d->d_q, d->d_k, d->d_v};
         if (fused) {
             const SkinnyJob j3[3] = {{L.q, d->d_h, nullptr, d->d_q}, {L.k, d->d_h, nullptr, d->d_k}, {L.v, d->d_h, nullptr, d->d_v}};
-            const StepPart part = {L.in_norm, c.rms_eps, 0, 0};
+            const StepPart part = next_weights({L.in_norm, c.rms_eps, 0, 0, {}}, L.o, nullptr, nullptr);
             DEC_RUN(32, if ((s = launch_skinny_step(ctx, j3, 3, part, NNQ_F32, st)) != NNQ_OK) return s);
         } else {
             DEC_RUN(32, if ((s = nnq_linear_batch(ctx, 3, w3, x3, adt, 1, nullptr, y3, NNQ_F32, st)) != NNQ_OK) return s);
@@ -1635,10 +1654,13 @@ static nnq_status step_qwen3(nnq_decoder *d, cudaStream_t st) {
         });
         if (fused) {
             const SkinnyJob jo = {L.o, d->d_attn, nullptr, d->d_h}, j2[2] = {{L.gate, d->d_h, nullptr, d->d_mid}, {L.up, d->d_h, nullptr, d->d_mid}}, jd = {L.down, d->d_mid, nullptr, d->d_h};
-            const StepPart add = {nullptr, 0.0f, 0, 1}, pg = {L.post_norm, c.rms_eps, 1, 0};
-            DEC_RUN(32, if ((s = launch_skinny_step(ctx, &jo, 1, add, NNQ_F32, st)) != NNQ_OK) return s);
+            const bool last = l + 1 == c.n_layers;
+            const nnq_decoder::Layer &N = d->layers[last ? l : l + 1];
+            const StepPart add = {nullptr, 0.0f, 0, 1, {}}, po = next_weights(add, L.gate, L.up, nullptr), pg = next_weights({L.post_norm, c.rms_eps, 1, 0, {}}, L.down, nullptr, nullptr),
+                           pd = last ? next_weights(add, d->lm_head, nullptr, nullptr) : next_weights(add, N.q, N.k, N.v);
+            DEC_RUN(32, if ((s = launch_skinny_step(ctx, &jo, 1, po, NNQ_F32, st)) != NNQ_OK) return s);
             DEC_RUN(32, if ((s = launch_skinny_step(ctx, j2, 2, pg, NNQ_BF16, st)) != NNQ_OK) return s);
-            DEC_RUN(32, if ((s = launch_skinny_step(ctx, &jd, 1, add, NNQ_F32, st)) != NNQ_OK) return s);
+            DEC_RUN(32, if ((s = launch_skinny_step(ctx, &jd, 1, pd, NNQ_F32, st)) != NNQ_OK) return s);
             ctx->launches += l == 0 ? 2 : 1;
             continue;
         }

@@ -253,6 +253,11 @@ __global__ void __launch_bounds__(256) stream_read_kernel(const SkinnyParams P, 
 }
 #endif
 
+static void share_next(SkinnyParams &P, int grid) {
+    const unsigned warps = (unsigned)grid * kWarps;
+    for (auto &w : P.step.next) w.share = ((w.bytes + warps - 1) / warps + 15) / 16 * 16;
+}
+
 // One launch: jobs that share their activations (same x pointer, same K).
 static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int x_dt, int m, int y_dt,
                                cudaStream_t stream, const FusedReduce *fr = nullptr, const StepPart *step = nullptr) {
@@ -307,6 +312,7 @@ static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, i
         int per_sm = kSmemMax / (smem_bytes + 1024);
         if (per_sm > 2) per_sm = 2;   // register budget of the kernel
         int grid = tiles < ctx->sm_count * per_sm ? tiles : ctx->sm_count * per_sm;
+        share_next(P, grid);
         cudaError_t e;
         if (layout == kTiledQ4K) e = launch_mn_fmt<NNQ_Q4_K>(P, nt, f32x, grid, smem_bytes, stream);
         else if (layout == kTiledQ8_0) e = launch_mn_fmt<NNQ_Q8_0>(P, nt, f32x, grid, smem_bytes, stream);
@@ -341,6 +347,7 @@ static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, i
     if (grid > units) grid = units;
     if (grid < 1) grid = 1;
     int smem_bytes = smem_plan(P.kblocks, P.stages, f32x).total;
+    share_next(P, grid);
     cudaError_t e;
     if (norm) e = step->pair ? launch_kernel<false, kWarps, false, 2>(P, grid, smem_bytes, stream) : launch_kernel<false, kWarps, false, 1>(P, grid, smem_bytes, stream);
     else e = f32x ? launch_ks<true>(ksplit, P, grid, smem_bytes, stream) : launch_ks<false>(ksplit, P, grid, smem_bytes, stream);

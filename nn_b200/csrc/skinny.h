@@ -64,10 +64,16 @@ nnq_status launch_skinny(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int x_d
 //            of x by norm_w as it stages it and sums its squares; the one number 1 / rms is applied to the finished sums.
 //   pair     jobs 0 and 1 (gate, up) have equal rows: y of job 0 = silu(gate) * up as bf16
 //   add      y (f32) += the product
+//   next     weights that a product behind this one reads: every warp asks L2 for its share of them when it has read the last of
+//            its own tiles, so that memory is busy while this product ends and the next begins
 struct StepPart {
     const float *norm_w;
     float eps;
     int pair, add;
+    struct {
+        const uint8_t *p;
+        unsigned bytes, share;   // multiples of 16; a warp's share (set by the launch)
+    } next[3];
 };
 // True when launch_skinny_step can read a residual row of w->k values for this weight.
 bool skinny_norm_supported(const nnq_weight *w);

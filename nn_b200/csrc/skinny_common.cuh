@@ -42,4 +42,14 @@ struct SkinnyParams {
     FusedReduce fr;     // row-parallel product + all-reduce in one kernel (M = 1 kernel, one job)
 };
 
+// Warp i's share of the step's next weights (one lane).
+__device__ __forceinline__ void ask_next(const StepPart &s, unsigned i) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const unsigned at = i * s.next[k].share;
+        if (at < s.next[k].bytes)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(s.next[k].p + at), "r"(min(s.next[k].share, s.next[k].bytes - at)) : "memory");
+    }
+}
+
 }  // namespace nnq

@@ -699,6 +699,7 @@ skinny_q4k_m1_kernel(const __grid_constant__ SkinnyParams P) {
         // the previous unit's partial sums are long complete: write it out (one warp per row tile)
         if (unit >= 1 && ks == ((unit - 1) >> (STEP == 2)) % KS) finish(unit - 1);
     }
+    if (STEP > 0 && lane == 0) ask_next(P.step, cta * kWarps + warp);
     if (KS > 1 && !failed && n_units >= 1 && ks == ((n_units - 1) >> (STEP == 2)) % KS) finish(n_units - 1);
     if (failed) {
         // record the failure, then give this warp's copies still in flight a bounded chance to

@@ -781,6 +781,7 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
         if (lane == 0) mbar_arrive(full_s + 8 * b);
         if (unit >= 1 && warp == (unit - 1) % kWarps) finish(unit - 1);
     }
+    if (lane == 0) ask_next(P.step, cta * kWarps + warp);
     if (!failed && n_units >= 1 && warp == (n_units - 1) % kWarps) finish(n_units - 1);
     if (failed) {
         if (lane == 0) atomicExch(P.status, 1);
