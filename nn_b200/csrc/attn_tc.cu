@@ -3,8 +3,7 @@
 // q, k, v and the softmax weights are f32 and stay so in effect: every operand enters the tensor core as two
 // bf16 terms (x = hi + lo, the remainder is below 2^-16 of x), and a product is hi hi + hi lo + lo hi with f32
 // accumulation in tensor memory. Scores, maxima, exponentials, sums and the output accumulators are f32.
-// The Qwen3 layers, whose other attention kernels multiply in f32, take the same kernel with two f16 terms of
-// operands scaled by powers of two (SCALED: the remainder is below 2^-23 of x): see launch_attn_tc_scaled.
+// (The Qwen3 layers, whose other attention kernels multiply in f32, have a kernel of their own: attn_split.cu.)
 //
 // One CTA: 128 query vectors of one kv head (consecutive (row, query head of the group) pairs), key tiles of
 // 64 over the union of the rows' windows.
@@ -27,7 +26,6 @@ constexpr int kAtKeys = 64, kAtRows = 128;
 constexpr int kAtQAtom = kAtRows * 128, kAtKAtom = kAtKeys * 128;   // bytes of a tile of 64 columns (one swizzle row)
 constexpr int kAtThreads = 256, kAtLoaders = 3;   // (eight warps: two per scheduler, 255 registers each)
 constexpr float kLog2E = 1.4426950408889634f;
-constexpr float kAtProb = 16384.0f;   // scale of the softmax weights where they are f16 pairs
 
 // atoms: 64-wide pieces of the query / key dimension; nv: 32-wide pieces of the value dimension
 __host__ __device__ constexpr int at_q_bytes(int atoms) { return 2 * atoms * kAtQAtom; }
@@ -42,49 +40,15 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t &hi, uint32_t 
     lo = pack_bf16(x - __uint_as_float(hi << 16), y - __uint_as_float(hi & 0xFFFF0000u));
 }
 
-// the same of scale * x and scale * y as f16 pairs
-__device__ __forceinline__ void split2_f16(float x, float y, float scale, uint32_t &hi, uint32_t &lo) {
-    const float2 v = __fmul2_rn(make_float2(x, y), make_float2(scale, scale));
-    const __half2 h = __floats2half2_rn(v.x, v.y);
-    const float2 r = __ffma2_rn(__half22float2(h), make_float2(-1.0f, -1.0f), v);
-    const __half2 l = __floats2half2_rn(r.x, r.y);
-    hi = *reinterpret_cast<const uint32_t *>(&h);
-    lo = *reinterpret_cast<const uint32_t *>(&l);
-}
-template <bool SCALED>
-__device__ __forceinline__ void split2_as(float x, float y, float scale, uint32_t &hi, uint32_t &lo) {
-    if (SCALED) split2_f16(x, y, scale, hi, lo);
-    else split2(x, y, hi, lo);
-}
-
-// The power of two that brings the largest of some values (the bits of its absolute value) to 2^14 .. 2^15, and its inverse
-// (largest values below 2^-112 are scaled like that one: the inverse stays a normal number).
-__device__ __forceinline__ uint32_t top_exponent(uint32_t bits) { return min(max(bits >> 23, 15u), 254u); }
-__device__ __forceinline__ float top_scale(uint32_t bits) { return __uint_as_float((268u - top_exponent(bits)) << 23); }
-__device__ __forceinline__ float top_unscale(uint32_t bits) { return __uint_as_float((top_exponent(bits) - 14u) << 23); }
-__device__ __forceinline__ uint32_t abs_bits4(float4 v) {
-    const uint32_t all = 0x7FFFFFFFu;
-    return max(max(__float_as_uint(v.x) & all, __float_as_uint(v.y) & all), max(__float_as_uint(v.z) & all, __float_as_uint(v.w) & all));
-}
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // byte offset of element e (0 .. 63) of row r inside a swizzled tile of 128-byte rows
 __device__ __forceinline__ uint32_t swz_at(int r, int e) { return swz(r, e >> 3) + 2 * (e & 7); }
 
-// SCALED: top[kv head, key tile] holds the bits of the largest absolute key and value of the tile (attn_top_kernel). Keys and
-// values of a head share a power of two each, every query vector has its own, the softmax weights have kAtProb. Kv heads with
-// an infinity or a NaN are left to the f32 kernel.
-template <int ATOMS, int NV, bool SCALED>
-__global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn a, const uint2 *__restrict__ top, int all_tiles, int *status) {
+template <int ATOMS, int NV>
+__global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn a, int *status) {
     extern __shared__ __align__(1024) uint8_t at_smem_raw[];
     uint8_t *smem = at_smem_raw + (-smem_u32(at_smem_raw) & 1023u);   // (stays an address in shared memory to the compiler)
     __shared__ __align__(8) uint64_t bars[6];   // kv_full[2], kv_empty[2], s_full, p_full
     __shared__ uint32_t tmem_s;
-    __shared__ float q_unscale[SCALED ? kAtRows : 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t kvf = smem_u32(bars), kve = kvf + 16, sf = kvf + 32, pf = kvf + 40;
     // (the last rows first: under a wide window they see the most keys)
@@ -93,17 +57,6 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
     const int pos0 = a.span.pos0;
     const int first = max(0, pos0 + t0 / group - a.window + 1), last = pos0 + last_pair / group;   // keys some row sees
     const int tiles = (last - first) / kAtKeys + 1;
-    float k_scale = 1.0f, v_scale = 1.0f, k_unscale = 1.0f, v_unscale = 1.0f;
-    if (SCALED) {
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        const uint2 m = attn_largest(top + (size_t)kvh * all_tiles, all_tiles);
-        if (max(m.x, m.y) >= kNotFinite) return;
-        k_scale = top_scale(m.x);
-        v_scale = top_scale(m.y);
-        k_unscale = top_unscale(m.x);
-        v_unscale = top_unscale(m.y);
-    }
     uint8_t *q_s = smem, *kv_s = q_s + at_q_bytes(ATOMS), *p_s = kv_s + 2 * (at_k_bytes(ATOMS) + at_v_bytes(NV));
     const int kv_stage = at_k_bytes(ATOMS) + at_v_bytes(NV);
 
@@ -135,15 +88,8 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
         for (int i = 0; i < QN; i++) {
             const int u = tid + kAtThreads * i, r = u / (16 * ATOMS), d = 4 * (u % (16 * ATOMS));
             uint2 hi, lo;
-            float scale = 1.0f;
-            if (SCALED) {   // a warp holds one vector of 128
-                static_assert(!SCALED || ATOMS == 2, "a warp per vector");
-                const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, abs_bits4(v[i]));
-                scale = top_scale(m);
-                if (lane == 0) q_unscale[r] = top_unscale(m);
-            }
-            split2_as<SCALED>(v[i].x, v[i].y, scale, hi.x, lo.x);
-            split2_as<SCALED>(v[i].z, v[i].w, scale, hi.y, lo.y);
+            split2(v[i].x, v[i].y, hi.x, lo.x);
+            split2(v[i].z, v[i].w, hi.y, lo.y);
             uint8_t *dst = q_s + (d >> 6) * kAtQAtom + swz_at(r, d & 63);
             *reinterpret_cast<uint2 *>(dst) = hi;
             *reinterpret_cast<uint2 *>(dst + ATOMS * kAtQAtom) = lo;
@@ -160,7 +106,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
         // ---------------- softmax ----------------
         const int row = (t0 + tid) / group;                           // (rows past the end are not stored)
         const int my_hi = pos0 + row, my_lo = my_hi - a.window + 1;   // keys this vector sees
-        const float c = SCALED ? a.scale * kLog2E * q_unscale[tid] * k_unscale : a.scale * kLog2E;
+        const float c = a.scale * kLog2E;
         const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
         float acc[NV * 32];
 #pragma unroll
@@ -206,9 +152,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
                 for (int e = 0; e < 4; e++) {
                     const int i = ch * 8 + 2 * e;
                     const float x0 = __uint_as_float(s[i >> 5][i & 31]) - base, x1 = __uint_as_float(s[i >> 5][(i & 31) + 1]) - base;
-                    const float p0 = SCALED ? ex2(x0) : exp2f(x0), p1 = SCALED ? ex2(x1) : exp2f(x1);
+                    const float p0 = exp2f(x0), p1 = exp2f(x1);
                     sum += p0 + p1;
-                    split2_as<SCALED>(p0, p1, kAtProb, hp[e], lp[e]);
+                    split2(p0, p1, hp[e], lp[e]);
                 }
                 *reinterpret_cast<uint4 *>(p_s + swz(tid, ch)) = h;
                 *reinterpret_cast<uint4 *>(p_s + kAtQAtom + swz(tid, ch)) = lw;
@@ -221,7 +167,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
         }
         if (ok && t0 + tid <= last_pair) {
             const int head = kvh * group + (t0 + tid) % group;
-            const float inv = SCALED ? v_unscale * (1.0f / kAtProb) / l : 1.0f / l;
+            const float inv = 1.0f / l;
             const float *g = a.ffn.proj + (size_t)row * a.ffn.in_cols + a.c_g + head * a.vdim;
             const size_t at = (size_t)row * a.ffn.out_k + head * a.vdim;
             if (a.ffn.act_dt == NNQ_BF16 && (a.vdim & 7) == 0) {
@@ -279,8 +225,8 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
                 const int u = lt + LT * (b * KB + i), key = u / (16 * ATOMS), d = 4 * (u % (16 * ATOMS));
                 if (u >= KU) continue;
                 uint2 hi, lo;
-                split2_as<SCALED>(v[i].x, v[i].y, k_scale, hi.x, lo.x);
-                split2_as<SCALED>(v[i].z, v[i].w, k_scale, hi.y, lo.y);
+                split2(v[i].x, v[i].y, hi.x, lo.x);
+                split2(v[i].z, v[i].w, hi.y, lo.y);
                 uint8_t *dst = k_s + (d >> 6) * kAtKAtom + swz_at(key, d & 63);
                 *reinterpret_cast<uint2 *>(dst) = hi;
                 *reinterpret_cast<uint2 *>(dst + ATOMS * kAtKAtom) = lo;
@@ -308,7 +254,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     uint32_t hi, lo;
-                    split2_as<SCALED>(xv[e], yv[e], v_scale, hi, lo);
+                    split2(xv[e], yv[e], hi, lo);
                     uint8_t *dst = v_s + swz_at(d + e, j);
                     *reinterpret_cast<uint32_t *>(dst) = hi;
                     *reinterpret_cast<uint32_t *>(dst + NV * 32 * 128) = lo;
@@ -338,7 +284,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
         }
     } else if (lane == 0) {
         // ---------------- MMA issuer ----------------
-        constexpr uint32_t ab = SCALED ? 0u : (1u << 7) | (1u << 10);   // both operands f16, or both bf16
+        constexpr uint32_t ab = (1u << 7) | (1u << 10);   // both operands bf16
         const uint32_t id_s = (1u << 4) | ab | ((uint32_t)(kAtKeys >> 3) << 17) | ((128u >> 4) << 24);
         const uint32_t id_o = (1u << 4) | ab | ((uint32_t)(NV * 32 >> 3) << 17) | ((128u >> 4) << 24);
         const uint32_t qa = smem_u32(q_s), pa = smem_u32(p_s);
@@ -346,8 +292,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
             const uint32_t ka = smem_u32(kv_s + (t & 1) * kv_stage);
             bool add = false;
 #pragma unroll 1
-            for (int i = 0; i < 3; i++) {   // hi hi, hi lo, lo hi; SCALED: hi hi last, so that the small sums are rounded at their size
-                const int x = SCALED ? 2 - i : i;
+            for (int x = 0; x < 3; x++) {   // hi hi, hi lo, lo hi
                 const uint32_t qo = qa + (x == 2 ? ATOMS * kAtQAtom : 0), ko = ka + (x == 1 ? ATOMS * kAtKAtom : 0);
                 for (int at = 0; at < ATOMS; at++) {
                     const uint64_t dq = smem_desc(qo + at * kAtQAtom), dk = smem_desc(ko + at * kAtKAtom);
@@ -371,11 +316,10 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
             tc_fence_after();
             const uint32_t va = smem_u32(kv_s + (t & 1) * kv_stage) + at_k_bytes(ATOMS);
 #pragma unroll 1
-            for (int i = 0; i < 3; i++) {
-                const int x = SCALED ? 2 - i : i;
+            for (int x = 0; x < 3; x++) {
                 const uint64_t dp = smem_desc(pa + (x == 2 ? kAtQAtom : 0)), dv = smem_desc(va + (x == 1 ? NV * 32 * 128 : 0));
 #pragma unroll
-                for (int k = 0; k < 4; k++) umma_bf16(o_tmem, dp + 2 * k, dv + 2 * k, id_o, (i | k) != 0);
+                for (int k = 0; k < 4; k++) umma_bf16(o_tmem, dp + 2 * k, dv + 2 * k, id_o, (x | k) != 0);
             }
             umma_commit(kve + 8 * (t & 1));
             if (t + 1 < tiles) {
@@ -404,48 +348,18 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const WindowAttn
     }
 }
 
-// The bits of the largest absolute key and value of every tile of 64 keys, [kv heads, tiles]; a NaN is above an infinity.
-__global__ void __launch_bounds__(256) attn_top_kernel(const float *__restrict__ kcache, const float *__restrict__ vcache, int cap, int keys, uint2 *__restrict__ top) {
-    __shared__ uint32_t m[2];
-    const int tid = threadIdx.x, key0 = blockIdx.x * kAtKeys, have = min(kAtKeys, keys - key0);
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (tid < 2) m[tid] = 0;
-    __syncthreads();
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const size_t at = ((size_t)blockIdx.y * cap + key0) * 128;
-    uint32_t k = 0, v = 0;
-#pragma unroll
-    for (int i = 0; i < kAtKeys * 32 / 256; i++) {
-        const int u = tid + 256 * i;
-        if (u < have * 32) {
-            k = max(k, abs_bits4(reinterpret_cast<const float4 *>(kcache + at)[u]));
-            v = max(v, abs_bits4(reinterpret_cast<const float4 *>(vcache + at)[u]));
-        }
-    }
-    k = __reduce_max_sync(0xFFFFFFFFu, k);
-    v = __reduce_max_sync(0xFFFFFFFFu, v);
-    if ((tid & 31) == 0) {
-        atomicMax(&m[0], k);
-        atomicMax(&m[1], v);
-    }
-    __syncthreads();
-    if (tid == 0) top[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = make_uint2(m[0], m[1]);
-}
-
 // Enough query vectors to fill a good part of a tile, heads of at most 128, bf16 decoders (an f32 decoder
 // keeps f32 products).
 bool attn_tc_supported(const WindowAttn &a) {
     return a.ffn.act_dt == NNQ_BF16 && a.dim <= 128 && a.vdim <= 128 && a.span.n * (a.heads / a.kv_heads) >= 32;
 }
 
-template <int ATOMS, int NV, bool SCALED = false>
-static nnq_status at_go(nnq_ctx *ctx, const WindowAttn &a, cudaStream_t st, const uint2 *top = nullptr, int tiles = 0) {
+template <int ATOMS, int NV>
+static nnq_status at_go(nnq_ctx *ctx, const WindowAttn &a, cudaStream_t st) {
     const int smem = at_smem_bytes(ATOMS, NV), pairs = a.span.n * (a.heads / a.kv_heads);
-    nnq_status s = check_cuda(ctx, cudaFuncSetAttribute(attn_tc_kernel<ATOMS, NV, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "attention shared memory");
+    nnq_status s = check_cuda(ctx, cudaFuncSetAttribute(attn_tc_kernel<ATOMS, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "attention shared memory");
     if (s != NNQ_OK) return s;
-    const dim3 grid(a.kv_heads, (pairs + kAtRows - 1) / kAtRows);
-    if (SCALED) launch_pdl_smem(attn_tc_kernel<ATOMS, NV, SCALED>, grid, dim3(kAtThreads), smem, st, a, top, tiles, ctx->d_status);
-    else attn_tc_kernel<ATOMS, NV, SCALED><<<grid, kAtThreads, smem, st>>>(a, top, tiles, ctx->d_status);
+    attn_tc_kernel<ATOMS, NV><<<dim3(a.kv_heads, (pairs + kAtRows - 1) / kAtRows), kAtThreads, smem, st>>>(a, ctx->d_status);
     ctx->launches++;
     return check_cuda(ctx, cudaGetLastError(), "tensor-core attention launch");
 }
@@ -458,21 +372,6 @@ nnq_status launch_attn_tc(nnq_ctx *ctx, const WindowAttn &a, cudaStream_t st) {
         case 3: return two ? at_go<2, 3>(ctx, a, st) : at_go<1, 3>(ctx, a, st);
         default: return two ? at_go<2, 4>(ctx, a, st) : at_go<1, 4>(ctx, a, st);
     }
-}
-
-int attn_tiles(int keys) { return (keys + kAtKeys - 1) / kAtKeys; }
-
-// Heads of 128, no window: operands as two f16 terms hold 22 to 24 bits of every value that is at most 2^16 below the largest of
-// its query vector, or of the head's keys or values (2^-39 of that largest below). Error of the outputs against 64 bits, f32
-// kernel / this / two bf16 terms: 4.8e-7 / 1.6e-7 / 1.7e-6 for 2048 rows of normal values, 1.2e-6 / 5.7e-7 / 9.5e-6 with four
-// times the queries, 7.8e-7 / 3.6e-7 / 4.3e-6 for 4000 rows, 2.1e-7 / 1.8e-7 / 4.0e-6 for 9 rows behind 20. Time as with bf16 terms
-// (288 us for 2048 rows), 10 us for the launches before and behind it. top: [kv_heads, attn_tiles(cap)].
-nnq_status launch_attn_tc_scaled(nnq_ctx *ctx, const WindowAttn &a, uint2 *top, cudaStream_t st) {
-    const int keys = a.span.pos0 + a.span.n, tiles = attn_tiles(keys);
-    launch_pdl(attn_top_kernel, dim3(tiles, a.kv_heads), dim3(256), st, a.kcache, a.vcache, a.cap, keys, top);
-    ctx->launches++;
-    nnq_status s = check_cuda(ctx, cudaGetLastError(), "largest keys and values launch");
-    return s != NNQ_OK ? s : at_go<2, 4, true>(ctx, a, st, top, tiles);
 }
 
 }  // namespace nnq

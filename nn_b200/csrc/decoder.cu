@@ -63,7 +63,9 @@ struct nnq_decoder {
     float *pf_h, *pf_delta, *pf_q, *pf_k, *pf_v, *pf_qrot, *pf_g, *pf_u;
     void *pf_xn, *pf_attn, *pf_mid;
     int *pf_tokens;
-    uint2 *pf_top;              // largest keys and values of every 64 positions, [lkv, max_seq / 64] (attn_tc.cu)
+    uint2 *pf_top;              // largest keys and values of every 64 positions, [lkv, max_seq / 64] (attn_split.cu)
+    uint8_t *pf_images;         // keys and values of one layer as operand tiles, of pf_image_keys positions
+    int pf_image_keys;
     int *pf_want;               // rows of a block whose logits are asked for, [pf_rows]
     float *d_want_logits;       // [kWantRows, vocab], allocated by the first nnq_decoder_extend that asks for any
     int embed_ld, xn_ld;        // row strides of the embedding table and of the normed rows
@@ -1689,6 +1691,23 @@ static void norm_rows(nnq_decoder *d, const float *delta, const __nv_bfloat16 *e
     else dec_norm_rows_kernel<<<n, 256, 0, st>>>(d->pf_h, delta, embed, tokens, w, eps, d->pf_xn, d->act_dt, hidden);
 }
 
+// The operand tiles of a layer's keys and values (as many bytes as they have in the cache of one layer), twice as many as before
+// when a longer context comes.
+static bool image_buffer(nnq_decoder *d, int keys) {
+    if (keys <= d->pf_image_keys) return true;
+    const int want = std::min(d->cfg.max_seq, std::max(2 * d->pf_image_keys, (keys + 2047) / 2048 * 2048));
+    cudaFree(d->pf_images);   // (waits for the kernels that use it)
+    d->pf_images = nullptr;
+    d->pf_image_keys = 0;
+    if (cudaMalloc((void **)&d->pf_images, attn_image_bytes(d->lkv, want)) != cudaSuccess) {
+        cudaGetLastError();
+        d->pf_images = nullptr;
+        return false;
+    }
+    d->pf_image_keys = want;
+    return true;
+}
+
 static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
     nnq_ctx *ctx = d->ctx;
     const nnq_decoder_config &c = d->cfg;
@@ -1711,11 +1730,11 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         else
             dec_qk_rope_rows_kernel<<<dim3(lh + 2 * lkv, n), hd, 0, st>>>(d->pf_q, d->pf_k, d->pf_v, L.q_norm, L.k_norm, d->d_cos, d->d_sin, pos0,
                                                                      c.rms_eps, d->pf_qrot, kc, vc, lh, lkv, hd, c.max_seq);
-        // bf16 decoders: on the tensor cores (attn_tc.cu, two f16 terms per operand) from 32 query vectors per key / value head and
-        // 64 keys on. Its three launches take 23 us on the fewest rows and keys, the f32 kernel 0.42 us more per key: in us, f32 /
-        // tensor cores, 16.9 / 24.6 at 32 rows, 31.1 / 25.0 at 64, 37.1 / 26.9 at 8 rows behind 64, 2328 / 287 at 2048 rows of the
+        // bf16 decoders: on the tensor cores (attn_split.cu, two f16 terms per operand) from 32 query vectors per key / value head and
+        // 64 keys on. Its launches take 23 us on the fewest rows and keys, the f32 kernel 0.42 us more per key: in us, f32 /
+        // tensor cores, 16.9 / 24.6 at 32 rows, 31.1 / 25.0 at 64, 37.1 / 26.9 at 8 rows behind 64, 2328 / 130 at 2048 rows of the
         // Qwen3-8B shape. f32 decoders keep f32 products, and so do the kv heads with an infinity or a NaN: which other rows
-        // those reach stays as in the f32 kernel.
+        // those reach stays as in the f32 kernel. Without memory for the operand tiles the f32 kernel takes all heads.
         WindowAttn wa = {};
         wa.span = {n, pos0, nullptr};
         wa.heads = lh;
@@ -1729,8 +1748,8 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         wa.ffn.act = d->pf_attn;
         wa.ffn.act_dt = d->act_dt;
         wa.ffn.out_k = lh * hd;
-        const bool tc = attn_tc_supported(wa) && pos0 + n >= 64;
-        if (tc && (s = launch_attn_tc_scaled(ctx, wa, d->pf_top, st)) != NNQ_OK) return s;
+        const bool tc = attn_split_supported(wa) && pos0 + n >= 64 && image_buffer(d, pos0 + n);
+        if (tc && (s = launch_attn_split(ctx, wa, d->pf_top, d->pf_images, st)) != NNQ_OK) return s;
         const uint2 *top = tc ? d->pf_top : nullptr;
         const int tiles = attn_tiles(pos0 + n);
         // 16 query vectors per warp: R = 16 / G rows share each key / value row
@@ -2017,6 +2036,7 @@ void nnq_decoder_destroy(nnq_decoder *d) {
     cudaFree(d->pf_mem); cudaFree(d->d_want_logits);
     cudaFree(d->d_final_norm); cudaFree(d->d_cos); cudaFree(d->d_sin); cudaFree(d->d_kcache); cudaFree(d->d_vcache);
     cudaFree(d->d_h); cudaFree(d->d_delta); cudaFree(d->d_q); cudaFree(d->d_k); cudaFree(d->d_v); cudaFree(d->d_qrot);
+    cudaFree(d->pf_images);
     cudaFree(d->d_g); cudaFree(d->d_u); cudaFree(d->d_logits); cudaFree(d->d_part); cudaFree(d->d_arrived); cudaFree(d->d_xn); cudaFree(d->d_attn);
     cudaFree(d->d_mid); cudaFree(d->d_state); cudaFree(d->d_tokens);
     if (!d->pf_mem) {   // of a block decoder
