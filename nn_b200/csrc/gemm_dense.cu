@@ -145,18 +145,20 @@ dequant_bf16_kernel(const uint8_t *__restrict__ src, const uint8_t *__restrict__
 }
 
 // nn-gptoss expert tensors [E, K, N] (MXFP4, 32-weight blocks along N, the even column in the high
-// nibble) -> bf16 [E, N, K]: a CTA turns a 64 x 64 tile through shared memory. Reads are whole sectors
-// (32 bytes of a k row), writes 128 contiguous bytes per output row. Bound by the decode, which looks four magnitudes up at a
-// time and stores pairs of k: the 4096-token block of 32 experts of 2880, one code at a time / this: 1.82 / 1.74 ms. half_rows > 0 interleaves the output
-// rows of every expert (row j -> 2j, row half_rows + j -> 2j + 1), as the fused SwiGLU epilogue wants.
+// nibble) -> bf16 [E, N, K]: a CTA turns a tile of 64 KT (k) x 64 (n)
+// through shared memory. Reads are whole sectors (32 bytes of a k row), writes 128 KT contiguous bytes per output row. Bound by the
+// decode, which looks four magnitudes up at a time and stores pairs of k, then by the stores: both weights of 32 experts of 2880,
+// KT = 1 / 3: 504 / 467 us (KT = 3 where K is a multiple of 192). half_rows > 0 interleaves the output rows of every expert (row j ->
+// 2j, row half_rows + j -> 2j + 1), as the fused SwiGLU epilogue wants.
 constexpr int kKnTile = 64;
-__global__ void __launch_bounds__(128)
+template <int KT>
+__global__ void __launch_bounds__(128 * KT)
 dequant_kn_bf16_kernel(const uint8_t *__restrict__ data, const uint8_t *__restrict__ scales, __nv_bfloat16 *__restrict__ dst,
                        int K, int N, int half_rows) {
-    __shared__ __align__(16) uint16_t tile[kKnTile][kKnTile + 8];   // [n][k]; 144-byte rows keep 16-byte reads aligned
-    const int e = blockIdx.z, k0 = blockIdx.y * kKnTile, n0 = blockIdx.x * kKnTile;
+    __shared__ __align__(16) uint16_t tile[kKnTile][kKnTile * KT + 8];   // [n][k]; the odd 16 bytes keep 16-byte reads aligned
+    const int e = blockIdx.z, k0 = blockIdx.y * kKnTile * KT, n0 = blockIdx.x * kKnTile;
     // this thread's pair of k rows and 16 of the 64 columns: it makes the pairs (k, k + 1) that lie side by side in the copy
-    const int pair = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const int pair = (threadIdx.x & 31) + 32 * (threadIdx.x >> 7), part = (threadIdx.x >> 5) & 3;
     const size_t row = (size_t)e * K + k0 + 2 * pair;
     const uint2 qa = __ldg(reinterpret_cast<const uint2 *>(data + row * (size_t)(N / 2) + n0 / 2 + part * 8));
     const uint2 qb = __ldg(reinterpret_cast<const uint2 *>(data + (row + 1) * (size_t)(N / 2) + n0 / 2 + part * 8));
@@ -183,8 +185,8 @@ dequant_kn_bf16_kernel(const uint8_t *__restrict__ data, const uint8_t *__restri
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kKnTile * 8; i += 128) {
-        const int r = i >> 3, c = i & 7, n = n0 + r;
+    for (int i = threadIdx.x; i < kKnTile * 8 * KT; i += 128 * KT) {
+        const int r = i / (8 * KT), c = i - r * (8 * KT), n = n0 + r;
         const int nn = half_rows > 0 ? (n < half_rows ? 2 * n : 2 * (n - half_rows) + 1) : n;
         *reinterpret_cast<uint4 *>(dst + ((size_t)e * N + nn) * K + k0 + c * 8) = *reinterpret_cast<const uint4 *>(&tile[r][c * 8]);
     }
@@ -226,12 +228,6 @@ __device__ __forceinline__ void dg_tma_2d_pair(uint32_t dst, const CUtensorMap *
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 
-// Grouped mode (expert products): the rows of x are sorted by expert (offsets[e] .. offsets[e+1]
-// on the device), expert e multiplies its rows with rows [e * N, (e + 1) * N) of the decoded
-// weights and adds bias + e * N. Row tiles are numbered expert by expert; rows of the next expert
-// inside a tile are computed but not stored. offsets == NULL: a plain product.
-constexpr int kDgMaxGroups = 256;
-
 // A pair of CTAs (CG = 2) holds 128 rows of the activation tile and BN / 2 rows of the weight tile each: the tensor cores
 // read both halves, so an operand byte is brought to shared memory and read from it once per 256 x 256 products instead of
 // once per 128 x 256. With one CTA the two (48 KB in, 48 KB out per 64-wide k step of 512 tensor-core clocks) exceed what
@@ -242,7 +238,7 @@ template <int BN, int CG>
 __global__ void __launch_bounds__(kDgThreads, 1)
 gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                   const float *__restrict__ bias, void *__restrict__ y, int M, int N, int K, int y_dt, int *status,
-                  const int *__restrict__ offsets, int groups, __nv_bfloat16 *__restrict__ h_out, float swiglu_limit, int gate_kind) {
+                  __nv_bfloat16 *__restrict__ h_out, int gate_kind) {
     constexpr int kDgBN = BN, kDgStageBytes = dg_stage_bytes(BN, CG), kDgStages = dg_stages(BN, CG), kDgRows = kDgBM * CG;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + (-smem_u32(smem_raw) & 1023u);   // (stays an address in shared memory to the compiler)
@@ -254,36 +250,12 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     const uint32_t accf_s = empty_s + 8 * kDgStages, acce_s = accf_s + 16, done_s = acce_s + 16;
     const int rank = CG == 2 ? (int)cluster_rank() : 0;
     const int unit = blockIdx.x / CG, units = gridDim.x / CG;   // a unit multiplies one tile at a time
-    __shared__ int tile_begin[kDgMaxGroups + 1], row_begin[kDgMaxGroups + 1];
-    if (tid == 0) {
-        if (offsets) {
-            int acc = 0;
-            for (int e = 0; e < groups; e++) {
-                tile_begin[e] = acc;
-                row_begin[e] = offsets[e];
-                acc += (offsets[e + 1] - offsets[e] + kDgRows - 1) / kDgRows;
-            }
-            tile_begin[groups] = acc;
-            row_begin[groups] = offsets[groups];
-        } else {
-            tile_begin[0] = 0;
-            tile_begin[1] = (M + kDgRows - 1) / kDgRows;
-            row_begin[0] = 0;
-            row_begin[1] = M;
-        }
-    }
-    __syncthreads();
-    const int ngroups = offsets ? groups : 1;
-    const int m_tiles = tile_begin[ngroups], n_tiles = (N + kDgBN - 1) / kDgBN;
+    const int m_tiles = (M + kDgRows - 1) / kDgRows, n_tiles = (N + kDgBN - 1) / kDgBN;
     const int tiles = m_tiles * n_tiles;
     const int nkb = K / kDgBK;
-    // tile t -> (group, this CTA's first row, end of the group's rows, first weight row)
-    auto locate = [&](int t, int &e, int &m0, int &m_end, int &n0) {
-        const int mt = t % m_tiles;
-        e = 0;
-        while (e + 1 < ngroups && mt >= tile_begin[e + 1]) e++;
-        m0 = row_begin[e] + (mt - tile_begin[e]) * kDgRows + rank * kDgBM;
-        m_end = row_begin[e + 1];
+    // tile t -> this CTA's first row, first weight row
+    auto locate = [&](int t, int &m0, int &n0) {
+        m0 = t % m_tiles * kDgRows + rank * kDgBM;
         n0 = (t / m_tiles) * kDgBN;
     };
 
@@ -323,9 +295,9 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
             uint32_t phase = 0;
             long long filled = 0;
             for (int t = unit; t < tiles && ok; t += units) {
-                int e, m0, m_end, n0;
-                locate(t, e, m0, m_end, n0);
-                const int w0 = e * N + n0 + rank * (BN / CG);   // weight rows of this group in the decoded [groups * N, K] matrix
+                int m0, n0;
+                locate(t, m0, n0);
+                const int w0 = n0 + rank * (BN / CG);
                 for (int kb = 0; kb < nkb; kb++) {
                     if (filled >= kDgStages && !mbar_wait_fast(empty_s + 8 * slot, phase ^ 1u)) {
                         ok = false;
@@ -410,9 +382,8 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
         int it = 0;
         for (int t = unit; t < tiles && ok; t += units, it++) {
             const int a = it & 1;
-            int e, m0, m_end, n0;
-            locate(t, e, m0, m_end, n0);
-            const float *gbias = bias ? bias + (size_t)e * N : nullptr;
+            int m0, n0;
+            locate(t, m0, n0);
             if (!mbar_wait_fast(accf_s + 8 * a, (uint32_t)((it >> 1) & 1))) {
                 ok = false;
                 break;
@@ -425,10 +396,9 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                 tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * kDgBN + cc * 32), v);
                 const int col0 = n0 + cc * 32;
                 if (h_out) {
-                    // interleaved gate / up columns (2j, 2j + 1): h[row, j] = clamp(f(g), +-limit) * u in bf16, f silu or gelu,
-                    // the input of the second expert product; the bias of column c is the gate bias of c / 2 for
-                    // even c and the up bias (second half of the expert's bias row) for odd c
-                    if (row < m_end && col0 < N) {
+                    // interleaved gate / up columns (2j, 2j + 1): h[row, j] = f(g) * u in bf16, f silu or gelu; the bias of column c
+                    // is the gate bias of c / 2 for even c and the up bias (second half of the bias row) for odd c
+                    if (row < M && col0 < N) {
                         const int I = N >> 1;
                         uint32_t packed[8];
 #pragma unroll
@@ -438,17 +408,15 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                             for (int q2 = 0; q2 < 2; q2++) {
                                 const int j = (col0 >> 1) + p + q2;
                                 float gv = __uint_as_float(v[2 * (p + q2)]), uv = __uint_as_float(v[2 * (p + q2) + 1]);
-                                if (gbias && j < I) {
-                                    gv += __ldg(gbias + j);
-                                    uv += __ldg(gbias + I + j);
+                                if (bias && j < I) {
+                                    gv += __ldg(bias + j);
+                                    uv += __ldg(bias + I + j);
                                 }
                                 // fast exponential and division (2^-22 relative): far below the bf16 rounding of h,
                                 // and cheap enough for the epilogue to stay hidden behind the next tile's MMAs
                                 // (the tanh form of gelu is x sigmoid(2 sqrt(2 / pi) (x + 0.044715 x^3)))
                                 const float sx = gate_kind == NNQ_ACT_GELU_TANH ? 1.5957691216057308f * fmaf(0.044715f * gv * gv, gv, gv) : gv;
-                                float sv = __fdividef(gv, 1.0f + __expf(-sx));
-                                sv = fminf(fmaxf(sv, -swiglu_limit), swiglu_limit);
-                                hv[q2] = sv * uv;
+                                hv[q2] = __fdividef(gv, 1.0f + __expf(-sx)) * uv;
                             }
                             __nv_bfloat162 b2 = __floats2bfloat162_rn(hv[0], hv[1]);
                             packed[p >> 1] = *reinterpret_cast<uint32_t *>(&b2);
@@ -463,10 +431,10 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                                 if ((col0 >> 1) + i < I) dstp[i] = pk[i];
                         }
                     }
-                } else if (row < m_end && col0 < N) {
+                } else if (row < M && col0 < N) {
                     float f[32];
 #pragma unroll
-                    for (int i = 0; i < 32; i++) f[i] = __uint_as_float(v[i]) + (gbias && col0 + i < N ? __ldg(gbias + col0 + i) : 0.0f);
+                    for (int i = 0; i < 32; i++) f[i] = __uint_as_float(v[i]) + (bias && col0 + i < N ? __ldg(bias + col0 + i) : 0.0f);
                     if (col0 + 32 <= N && (N & 7) == 0) {
                         if (y_dt == NNQ_F32) {
                             float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(y) + (size_t)row * N + col0);
@@ -595,21 +563,11 @@ static DgShape dg_pick(const nnq_ctx *ctx, int64_t m, int64_t n, int64_t k, bool
     if (decoded && waves == 1 && (m + n) * k * 2 <= 60ll << 20) return {256, 1};
     return 16 * pair_waves <= (k >= 2048 ? 18 : 17) * waves ? DgShape{256, 2} : DgShape{256, 1};
 }
-// Experts: the last row tile of each is filled by half on average, so tiles of 128 rows. (32 experts, 16384 routed rows: single
-// CTAs 572 + 328 us, pairs 564 + 322 when only they run, 1.855 against 1.879 ms for the block.)
-static DgShape dg_pick_grouped(const nnq_ctx *ctx, int64_t rows, int experts, int64_t n) {
-    const int64_t m_tiles = rows / kDgBM + experts;   // at most
-    return {2 * m_tiles * ((n + 255) / 256) <= ctx->sm_count ? 128 : 256, 1};
-}
-
 struct DgArgs {
     const float *bias;
     void *y;
     int m, n, k, y_dt;
-    const int *offsets;
-    int groups;
     __nv_bfloat16 *h_out;
-    float swiglu_limit;
     int gate_kind;
 };
 
@@ -636,8 +594,7 @@ static nnq_status dg_launch(nnq_ctx *ctx, const CUtensorMap &xmap, const CUtenso
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = CG == 2 ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_dense_kernel<BN, CG>, xmap, wmap, a.bias, a.y, a.m, a.n, a.k, a.y_dt, ctx->d_status, a.offsets, a.groups,
-                                             a.h_out, a.swiglu_limit, a.gate_kind);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_dense_kernel<BN, CG>, xmap, wmap, a.bias, a.y, a.m, a.n, a.k, a.y_dt, ctx->d_status, a.h_out, a.gate_kind);
     ctx->launches++;
     return check_cuda(ctx, e, "bf16 GEMM launch");
 }
@@ -647,50 +604,51 @@ static nnq_status dg_launch_shape(nnq_ctx *ctx, DgShape shape, const CUtensorMap
     return shape.bn == 256 ? dg_launch<256, 1>(ctx, xmap, wmap, a, tiles, stream) : dg_launch<128, 1>(ctx, xmap, wmap, a, tiles, stream);
 }
 
-// The GEMM alone: w_bf16 is a bf16 [n, k] weight in device memory (16-byte aligned). h_out: see launch_gemm_dense_pairs.
-static nnq_status dense_bf16(nnq_ctx *ctx, const void *w_bf16, const TcArgs &a, __nv_bfloat16 *h_out, int gate_kind, cudaStream_t stream) {
+// The GEMM alone: w_bf16 is a bf16 [n, k] weight in device memory (16-byte aligned), decoded: just before. h_out: see
+// launch_gemm_dense_pairs.
+static nnq_status dense_bf16(nnq_ctx *ctx, const void *w_bf16, const TcArgs &a, __nv_bfloat16 *h_out, int gate_kind, bool decoded, cudaStream_t stream) {
     CUtensorMap xmap, wmap;
     memset(&xmap, 0, sizeof(xmap));
     memset(&wmap, 0, sizeof(wmap));
-    const DgShape shape = dg_pick(ctx, a.m, a.n, a.k, w_bf16 == ctx->d_dense);
+    const DgShape shape = dg_pick(ctx, a.m, a.n, a.k, decoded);
     if (!make_map(a.x, a.m, a.k, kDgBM, &xmap) || !make_map(w_bf16, a.n, a.k, shape.bn / shape.cg, &wmap))
         return fail(ctx, NNQ_ERR_DISPATCH_FAILED, "tensor map creation failed");
-    const DgArgs d = {a.bias, a.y, (int)a.m, (int)a.n, (int)a.k, a.y_dt, nullptr, 0, h_out, INFINITY, gate_kind};
+    const DgArgs d = {a.bias, a.y, (int)a.m, (int)a.n, (int)a.k, a.y_dt, h_out, gate_kind};
     const int64_t rows = kDgBM * shape.cg, tiles = (a.m + rows - 1) / rows * ((a.n + shape.bn - 1) / shape.bn);
     return dg_launch_shape(ctx, shape, xmap, wmap, d, tiles, stream);
 }
 
-nnq_status launch_gemm_dense_bf16(nnq_ctx *ctx, const void *w_bf16, const TcArgs &a, cudaStream_t stream) { return dense_bf16(ctx, w_bf16, a, nullptr, 0, stream); }
+nnq_status launch_gemm_dense_bf16(nnq_ctx *ctx, const void *w_bf16, const TcArgs &a, cudaStream_t stream) { return dense_bf16(ctx, w_bf16, a, nullptr, 0, w_bf16 == ctx->d_dense, stream); }
 
 nnq_status launch_gemm_dense_pairs(nnq_ctx *ctx, const TcArgs &a, __nv_bfloat16 *h_out, int gate_kind, cudaStream_t stream) {
-    return dense_bf16(ctx, a.w, a, h_out, gate_kind, stream);
+    return dense_bf16(ctx, a.w, a, h_out, gate_kind, false, stream);
 }
 
-nnq_status launch_gemm_dense(nnq_ctx *ctx, const TcArgs &a, cudaStream_t stream) {
-    // a bf16 weight is its own decoded form
-    if (a.fmt == NNQ_BF16_DENSE && !((uintptr_t)a.w & 15u)) return launch_gemm_dense_bf16(ctx, a.w, a, stream);
-    Geometry g = geometry(a.fmt);
-    const int64_t nchunks = a.n * (a.k / g.elems) * (g.elems / 32);
-    cudaError_t e;
-    switch (a.fmt) {
-#define NNQ_DB(F) case F: e = launch_dequant_bf16<F>(a.w, a.scales, nchunks, ctx->d_dense, ctx->sm_count, stream); break
+static cudaError_t decode_bf16(nnq_ctx *ctx, int fmt, const uint8_t *w, const uint8_t *scales, int64_t nchunks, void *dst, cudaStream_t stream, int cpr = 1, int half_rows = 0) {
+    ctx->launches++;
+    switch (fmt) {
+#define NNQ_DB(F) case F: return launch_dequant_bf16<F>(w, scales, nchunks, dst, ctx->sm_count, stream, cpr, half_rows)
         NNQ_DB(NNQ_Q4_0); NNQ_DB(NNQ_Q4_1); NNQ_DB(NNQ_Q8_0); NNQ_DB(NNQ_Q4_K); NNQ_DB(NNQ_Q4_K_GGML); NNQ_DB(NNQ_Q6_K);
         NNQ_DB(NNQ_MXFP4_CORE); NNQ_DB(NNQ_MXFP4_SPLIT); NNQ_DB(NNQ_MXFP4_GPTOSS); NNQ_DB(NNQ_Q5_0); NNQ_DB(NNQ_Q5_1);
         NNQ_DB(NNQ_Q2_K); NNQ_DB(NNQ_Q3_K); NNQ_DB(NNQ_Q5_K);
         NNQ_DB(NNQ_F32_DENSE); NNQ_DB(NNQ_BF16_DENSE);
 #undef NNQ_DB
-        default: return fail(ctx, NNQ_ERR_INVALID_ARG, "unknown format %d", a.fmt);
+        default: return cudaErrorInvalidValue;
     }
-    ctx->launches++;
-    nnq_status s = check_cuda(ctx, e, "bf16 decode launch");
-    if (s != NNQ_OK) return s;
-    return launch_gemm_dense_bf16(ctx, ctx->d_dense, a, stream);
+}
+
+nnq_status launch_gemm_dense(nnq_ctx *ctx, const TcArgs &a, cudaStream_t stream) {
+    // a bf16 weight is its own decoded form
+    if (a.fmt == NNQ_BF16_DENSE && !((uintptr_t)a.w & 15u)) return launch_gemm_dense_bf16(ctx, a.w, a, stream);
+    const Geometry g = geometry(a.fmt);
+    nnq_status s = check_cuda(ctx, decode_bf16(ctx, a.fmt, a.w, a.scales, a.n * (a.k / g.elems) * (g.elems / 32), ctx->d_dense, stream), "bf16 decode launch");
+    return s != NNQ_OK ? s : launch_gemm_dense_bf16(ctx, ctx->d_dense, a, stream);
 }
 
 bool gemm_dense_grouped_supported(const nnq_ctx *ctx, const TcGroupArgs &g) {
     if (g.kn && (g.fmt != NNQ_MXFP4_GPTOSS || g.n % kKnTile || g.k % kKnTile || ((uintptr_t)g.w & 15u))) return false;
     const bool room = g.pairs || (ctx->d_dense && (size_t)g.experts * (size_t)g.n * (size_t)g.k * 2 <= ctx->dense_bytes);
-    return room && g.k >= kDgBK && g.k % kDgBK == 0 && g.experts >= 1 && g.experts <= kDgMaxGroups && g.rows_upper >= 1 && g.rows_upper < (1ll << 30) &&
+    return room && g.k >= kDgBK && g.k % kDgBK == 0 && g.experts >= 1 && g.experts <= kGeMaxGroups && g.rows_upper >= 1 && g.rows_upper < (1ll << 30) &&
            (int64_t)g.experts * g.n < (1ll << 31) && encode_fn() != nullptr;
 }
 
@@ -712,30 +670,19 @@ nnq_status launch_gemm_dense_grouped(nnq_ctx *ctx, const TcGroupArgs &g, cudaStr
     if (g.pairs) {
         // bf16 experts are multiplied where they are
     } else if (g.kn) {
-        dequant_kn_bf16_kernel<<<dim3((unsigned)(g.n / kKnTile), (unsigned)(g.k / kKnTile), (unsigned)g.experts), 128, 0, stream>>>(
-            g.w, g.scales, static_cast<__nv_bfloat16 *>(ctx->d_dense), (int)g.k, (int)g.n, half);
+        const int kt = g.k % (3 * kKnTile) == 0 ? 3 : 1;
+        const dim3 grid((unsigned)(g.n / kKnTile), (unsigned)(g.k / (kt * kKnTile)), (unsigned)g.experts);
+        __nv_bfloat16 *dst = static_cast<__nv_bfloat16 *>(ctx->d_dense);
+        if (kt == 3) dequant_kn_bf16_kernel<3><<<grid, 384, 0, stream>>>(g.w, g.scales, dst, (int)g.k, (int)g.n, half);
+        else dequant_kn_bf16_kernel<1><<<grid, 128, 0, stream>>>(g.w, g.scales, dst, (int)g.k, (int)g.n, half);
         e = cudaGetLastError();
-    } else
-    switch (g.fmt) {
-#define NNQ_DB(F) case F: e = launch_dequant_bf16<F>(g.w, g.scales, nchunks, ctx->d_dense, ctx->sm_count, stream, cpr, half); break
-        NNQ_DB(NNQ_Q4_0); NNQ_DB(NNQ_Q4_1); NNQ_DB(NNQ_Q8_0); NNQ_DB(NNQ_Q4_K); NNQ_DB(NNQ_Q4_K_GGML); NNQ_DB(NNQ_Q6_K);
-        NNQ_DB(NNQ_MXFP4_CORE); NNQ_DB(NNQ_MXFP4_SPLIT); NNQ_DB(NNQ_MXFP4_GPTOSS); NNQ_DB(NNQ_Q5_0); NNQ_DB(NNQ_Q5_1);
-        NNQ_DB(NNQ_Q2_K); NNQ_DB(NNQ_Q3_K); NNQ_DB(NNQ_Q5_K);
-        NNQ_DB(NNQ_F32_DENSE); NNQ_DB(NNQ_BF16_DENSE);
-#undef NNQ_DB
-        default: return fail(ctx, NNQ_ERR_INVALID_ARG, "unknown format %d", g.fmt);
+        ctx->launches++;
+    } else {
+        e = decode_bf16(ctx, g.fmt, g.w, g.scales, nchunks, ctx->d_dense, stream, cpr, half);
     }
-    if (!g.pairs) ctx->launches++;
     nnq_status s = check_cuda(ctx, e, "bf16 decode launch");
     if (s != NNQ_OK) return s;
-    CUtensorMap xmap, wmap;
-    memset(&xmap, 0, sizeof(xmap));
-    memset(&wmap, 0, sizeof(wmap));
-    const DgShape shape = dg_pick_grouped(ctx, g.rows_upper, g.experts, g.n);
-    if (!make_map(g.x_bf16, g.rows_upper, g.k, kDgBM, &xmap) || !make_map(w_bf16, (int64_t)g.experts * g.n, g.k, shape.bn / shape.cg, &wmap))
-        return fail(ctx, NNQ_ERR_DISPATCH_FAILED, "tensor map creation failed");
-    const DgArgs d = {g.bias, g.y, (int)g.rows_upper, (int)g.n, (int)g.k, NNQ_F32, g.offsets, g.experts, fuse ? g.h_out : nullptr, g.swiglu_limit, NNQ_ACT_SILU};
-    return dg_launch_shape(ctx, shape, xmap, wmap, d, ctx->sm_count, stream);   // (the number of tiles is known on the device only)
+    return launch_gemm_experts(ctx, g, w_bf16, fuse ? g.h_out : nullptr, stream);
 }
 
 }  // namespace nnq

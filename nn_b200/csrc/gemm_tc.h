@@ -63,6 +63,10 @@ nnq_status launch_gemm_ts(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int x_
 bool encode_map_2d(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64_t inner, int64_t rows, int64_t row_bytes, uint32_t box_inner,
                    uint32_t box_rows, CUtensorMapSwizzle swizzle);
 
+// The grouped product of decoded weights [experts, n, k] (gemm_experts.cu); h_out given: the gated activation instead of g.y.
+constexpr int kGeMaxGroups = 256;
+nnq_status launch_gemm_experts(nnq_ctx *ctx, const TcGroupArgs &g, const void *w_bf16, __nv_bfloat16 *h_out, cudaStream_t stream);
+
 // Large prefill (M >= 256, bf16 activations, K a multiple of 64): decode the weight to bf16 in the
 // context's scratch, then a persistent TMA + tcgen05 GEMM (gemm_dense.cu).
 bool gemm_dense_supported(const nnq_ctx *ctx, const nnq_weight *w, int64_t m, int x_dt);

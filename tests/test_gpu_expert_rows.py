@@ -1,5 +1,5 @@
-"""Expert products with chosen numbers of routed rows per expert: a reduction too long for the decode-sized kernel to
-hold its activations at once. Against float64 of the
+"""Expert products with chosen numbers of routed rows per expert: none, one, the edges of the 32-column steps and of the 256-row tiles of
+the prefill-sized product, and a reduction too long for the decode-sized kernel to hold its activations at once. Against float64 of the
 oracle's weights; the bound counts the roundings: gate and up sums carry 2^-20 of their magnitudes (exact weights: MXFP4 in bf16) or
 2^-8 (weights rounded to bf16 or f16 digits of their scales), |d silu| <= 1.1, h is rounded to bf16 (2^-8 with the rounding of the
 down product's operands) and the second product adds as the first."""
@@ -46,6 +46,12 @@ def _check(layout, fmt, counts, H, I, dtype, limit=7.0):
         bound = eh @ wd.abs() + exact * (h.abs() @ wd.abs()) + 1e-6
         err = ((got[torch.from_numpy(rows).cuda()] - want).abs() / bound).max().item()
         assert err <= 1.0, (e, rows.size, err)
+
+
+@pytest.mark.parametrize("layout,fmt", [(moe.LAYOUT_NK, Q.MXFP4_SPLIT), (moe.LAYOUT_KN_GPTOSS, Q.MXFP4_GPTOSS), (moe.LAYOUT_NK, Q.Q4_0)])
+@pytest.mark.parametrize("counts", [[0, 1, 31, 32, 33, 255, 256, 257, 700, 513, 0], [2050], [0, 0, 640, 1]])
+def test_rows_of_prefill_sized_products(layout, fmt, counts):
+    _check(layout, fmt, counts, 320, 192, torch.bfloat16)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
