@@ -64,6 +64,8 @@ struct nnq_decoder {
     void *pf_xn, *pf_attn, *pf_mid;
     int *pf_tokens;
     uint2 *pf_top;              // largest keys and values of every 64 positions, [lkv, max_seq / 64] (attn_split.cu)
+    void *d_pair;               // a layer's gate and up weights as bf16 for the prompt pass
+    size_t pair_bytes;
     uint8_t *pf_images;         // keys and values of one layer as operand tiles, of pf_image_keys positions
     int pf_image_keys;
     int *pf_want;               // rows of a block whose logits are asked for, [pf_rows]
@@ -856,6 +858,14 @@ nnq_status nnq_decoder_set_layer(nnq_decoder *d, int layer, const nnq_weight *q,
     if (s != NNQ_OK) return s;
     nnq_decoder::Layer &L = d->layers[layer];
     L.q = q; L.k = k; L.v = v; L.o = o; L.gate = gate; L.up = up; L.down = down;
+    const size_t pair = d->act_dt == NNQ_BF16 ? gemm_dense_gate_up_bytes(gate, up) : 0;
+    if (pair > d->pair_bytes) {   // (without room for it the prompt takes the two products one by one)
+        cudaFree(d->d_pair);
+        d->d_pair = nullptr;
+        d->pair_bytes = 0;
+        if (cudaMalloc(&d->d_pair, pair) == cudaSuccess) d->pair_bytes = pair;
+        else { cudaGetLastError(); d->d_pair = nullptr; }
+    }
     s = check_cuda(ctx, cudaMemcpy(L.in_norm, in_norm, (size_t)c.hidden * 4, cudaMemcpyDefault), "norm weight");
     if (s == NNQ_OK) s = check_cuda(ctx, cudaMemcpy(L.post_norm, post_norm, (size_t)c.hidden * 4, cudaMemcpyDefault), "norm weight");
     if (s == NNQ_OK) s = check_cuda(ctx, cudaMemcpy(L.q_norm, q_norm, (size_t)c.head_dim * 4, cudaMemcpyDefault), "norm weight");
@@ -1767,9 +1777,16 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         const nnq_weight *w2[2] = {L.gate, L.up};
         const void *x2[2] = {d->pf_xn, d->pf_xn};
         void *y2[2] = {d->pf_g, d->pf_u};
-        if ((s = nnq_linear_batch(ctx, 2, w2, x2, adt, n, nullptr, y2, NNQ_F32, st)) != NNQ_OK) return s;
+        // (from 513 rows on, where the products decode their weights once anyway)
+        const size_t pair = gemm_dense_gate_up_bytes(L.gate, L.up);
+        const bool gate_up = n > 512 && ctx->path == NNQ_PATH_AUTO && pair > 0 && pair <= d->pair_bytes && gemm_dense_shape_ok(ctx, n, 2 * L.gate->n, L.gate->k, d->act_dt);
+        if (gate_up) s = launch_gemm_dense_gate_up(ctx, L.gate, L.up, d->d_pair, d->pf_xn, n, (__nv_bfloat16 *)d->pf_mid, NNQ_ACT_SILU, st);
+        else s = nnq_linear_batch(ctx, 2, w2, x2, adt, n, nullptr, y2, NNQ_F32, st);
+        if (s != NNQ_OK) return s;
         const int64_t total = (int64_t)n * lffn;
-        if (lffn % 4 == 0) {
+        if (gate_up) {
+            // the products' kernel has formed the activation
+        } else if (lffn % 4 == 0) {
             launch_silu_mul_rows(ctx, d->pf_g, d->pf_u, d->pf_mid, d->act_dt, total, st);
         } else {
             const int64_t some = 1 << 30;   // (the kernel counts in 32 bits)
@@ -2036,6 +2053,7 @@ void nnq_decoder_destroy(nnq_decoder *d) {
     cudaFree(d->pf_mem); cudaFree(d->d_want_logits);
     cudaFree(d->d_final_norm); cudaFree(d->d_cos); cudaFree(d->d_sin); cudaFree(d->d_kcache); cudaFree(d->d_vcache);
     cudaFree(d->d_h); cudaFree(d->d_delta); cudaFree(d->d_q); cudaFree(d->d_k); cudaFree(d->d_v); cudaFree(d->d_qrot);
+    cudaFree(d->d_pair);
     cudaFree(d->pf_images);
     cudaFree(d->d_g); cudaFree(d->d_u); cudaFree(d->d_logits); cudaFree(d->d_part); cudaFree(d->d_arrived); cudaFree(d->d_xn); cudaFree(d->d_attn);
     cudaFree(d->d_mid); cudaFree(d->d_state); cudaFree(d->d_tokens);

@@ -67,7 +67,13 @@ __device__ __forceinline__ void mx_chunk_bf16(const uint4 q, uint32_t e, uint4 *
 template <int FMT>
 __global__ void __launch_bounds__(kDbThreads)
 dequant_bf16_kernel(const uint8_t *__restrict__ src, const uint8_t *__restrict__ scales, int64_t nchunks,
-                    uint4 *__restrict__ dst, int cpr, int half_rows) {
+                    uint4 *__restrict__ dst, int cpr, int half_rows, int pair) {
+    // pair >= 0: row j goes to row 2j + pair (one of two weights whose rows alternate; nchunks < 2^31)
+    const int shift = (cpr & (cpr - 1)) == 0 ? __ffs(cpr) - 1 : -1;
+    auto paired = [&](int64_t c) {
+        const uint32_t row = shift >= 0 ? (uint32_t)c >> shift : (uint32_t)c / (uint32_t)cpr;
+        return (int64_t)(2 * row + (uint32_t)pair) * cpr + ((uint32_t)c - row * (uint32_t)cpr);
+    };
     if (FMT == NNQ_MXFP4_SPLIT || FMT == NNQ_MXFP4_GPTOSS) {
         // a thread owns one 32-weight chunk: 64 contiguous output bytes (two whole 32-byte sectors), written
         // with four 16-byte stores -- the integer decode needs no staging (measured: 366 -> 320 us for the
@@ -94,7 +100,9 @@ dequant_bf16_kernel(const uint8_t *__restrict__ src, const uint8_t *__restrict__
             // rows) is written interleaved, gate row j to row 2j and up row j to row 2j + 1, so that a GEMM
             // tile holds both halves of an output column pair (the fused SwiGLU epilogue)
             int64_t oc = c;
-            if (half_rows > 0) {   // nchunks < 2^31 here (checked by the launcher): 32-bit divisions
+            if (pair >= 0) {
+                oc = paired(c);
+            } else if (half_rows > 0) {   // nchunks < 2^31 here (checked by the launcher): 32-bit divisions
                 const uint32_t c32 = (uint32_t)c, row = c32 / (uint32_t)cpr, cin = c32 - row * (uint32_t)cpr;
                 const uint32_t ex = row / (2u * half_rows), r = row - ex * 2u * half_rows;
                 const uint32_t r2 = r < (uint32_t)half_rows ? 2u * r : 2u * (r - half_rows) + 1u;
@@ -139,7 +147,11 @@ dequant_bf16_kernel(const uint8_t *__restrict__ src, const uint8_t *__restrict__
         const int64_t remaining = nchunks - base;
         const int live = remaining < kDbThreads ? (int)remaining : kDbThreads;
         uint4 *out = dst + base * 4;
-        for (int idx = threadIdx.x; idx < live * 4; idx += kDbThreads) out[idx] = tile[(idx & ~3) | ((idx & 3) ^ ((idx >> 3) & 3))];
+        if (pair >= 0) out = dst + (paired(base + (threadIdx.x >> 2)) - (threadIdx.x >> 2)) * 4;
+        for (int idx = threadIdx.x; idx < live * 4; idx += kDbThreads) {
+            out[idx] = tile[(idx & ~3) | ((idx & 3) ^ ((idx >> 3) & 3))];
+            if (pair >= 0 && idx + kDbThreads < live * 4) out = dst + (paired(base + ((idx + kDbThreads) >> 2)) - ((idx + kDbThreads) >> 2)) * 4;
+        }
         __syncthreads();
     }
 }
@@ -194,12 +206,12 @@ dequant_kn_bf16_kernel(const uint8_t *__restrict__ data, const uint8_t *__restri
 
 template <int FMT>
 static cudaError_t launch_dequant_bf16(const uint8_t *src, const uint8_t *scales, int64_t nchunks, void *dst, int sm_count,
-                                       cudaStream_t stream, int cpr = 1, int half_rows = 0) {
+                                       cudaStream_t stream, int cpr = 1, int half_rows = 0, int pair = -1) {
     const int64_t want = (nchunks + kDbThreads - 1) / kDbThreads;
     const int64_t cap = (int64_t)sm_count * 16;
     int grid = (int)(want < cap ? want : cap);
     if (grid < 1) grid = 1;
-    dequant_bf16_kernel<FMT><<<grid, kDbThreads, 0, stream>>>(src, scales, nchunks, reinterpret_cast<uint4 *>(dst), cpr, half_rows);
+    dequant_bf16_kernel<FMT><<<grid, kDbThreads, 0, stream>>>(src, scales, nchunks, reinterpret_cast<uint4 *>(dst), cpr, half_rows, pair);
     return cudaGetLastError();
 }
 
@@ -624,10 +636,11 @@ nnq_status launch_gemm_dense_pairs(nnq_ctx *ctx, const TcArgs &a, __nv_bfloat16 
     return dense_bf16(ctx, a.w, a, h_out, gate_kind, false, stream);
 }
 
-static cudaError_t decode_bf16(nnq_ctx *ctx, int fmt, const uint8_t *w, const uint8_t *scales, int64_t nchunks, void *dst, cudaStream_t stream, int cpr = 1, int half_rows = 0) {
+static cudaError_t decode_bf16(nnq_ctx *ctx, int fmt, const uint8_t *w, const uint8_t *scales, int64_t nchunks, void *dst, cudaStream_t stream, int cpr = 1, int half_rows = 0,
+                               int pair = -1) {
     ctx->launches++;
     switch (fmt) {
-#define NNQ_DB(F) case F: return launch_dequant_bf16<F>(w, scales, nchunks, dst, ctx->sm_count, stream, cpr, half_rows)
+#define NNQ_DB(F) case F: return launch_dequant_bf16<F>(w, scales, nchunks, dst, ctx->sm_count, stream, cpr, half_rows, pair)
         NNQ_DB(NNQ_Q4_0); NNQ_DB(NNQ_Q4_1); NNQ_DB(NNQ_Q8_0); NNQ_DB(NNQ_Q4_K); NNQ_DB(NNQ_Q4_K_GGML); NNQ_DB(NNQ_Q6_K);
         NNQ_DB(NNQ_MXFP4_CORE); NNQ_DB(NNQ_MXFP4_SPLIT); NNQ_DB(NNQ_MXFP4_GPTOSS); NNQ_DB(NNQ_Q5_0); NNQ_DB(NNQ_Q5_1);
         NNQ_DB(NNQ_Q2_K); NNQ_DB(NNQ_Q3_K); NNQ_DB(NNQ_Q5_K);
@@ -643,6 +656,26 @@ nnq_status launch_gemm_dense(nnq_ctx *ctx, const TcArgs &a, cudaStream_t stream)
     const Geometry g = geometry(a.fmt);
     nnq_status s = check_cuda(ctx, decode_bf16(ctx, a.fmt, a.w, a.scales, a.n * (a.k / g.elems) * (g.elems / 32), ctx->d_dense, stream), "bf16 decode launch");
     return s != NNQ_OK ? s : launch_gemm_dense_bf16(ctx, ctx->d_dense, a, stream);
+}
+
+// Gate and up products of one input and the activation in one GEMM over the two weights decoded to alternating rows of the
+// caller's buffer: the f32 products are neither written nor read, and no kernel multiplies them. Prompt of 2048
+// tokens through eight layers of the Qwen3-8B shape (gate and up of 12288 x 4096), apart / together: 8.80 / 8.17 ms.
+size_t gemm_dense_gate_up_bytes(const nnq_weight *gate, const nnq_weight *up) {
+    if (!gate || !up || gate->fmt != up->fmt || gate->n != up->n || gate->k != up->k || gate->fmt == NNQ_BF16_DENSE || !gate->d_raw || !up->d_raw) return 0;
+    return gate->n % 8 == 0 && gate->k >= kDgBK && gate->k % kDgBK == 0 && gate->n * (gate->k / 32) < (1ll << 30) ? (size_t)gate->n * (size_t)gate->k * 4 : 0;
+}
+nnq_status launch_gemm_dense_gate_up(nnq_ctx *ctx, const nnq_weight *gate, const nnq_weight *up, void *w_bf16, const void *x, int64_t m, __nv_bfloat16 *h_out, int gate_kind,
+                                     cudaStream_t stream) {
+    const Geometry g = geometry(gate->fmt);
+    const int64_t nchunks = gate->n * (gate->k / g.elems) * (g.elems / 32);
+    const nnq_weight *w[2] = {gate, up};
+    for (int i = 0; i < 2; i++) {
+        nnq_status s = check_cuda(ctx, decode_bf16(ctx, w[i]->fmt, w[i]->d_raw, w[i]->d_scales, nchunks, w_bf16, stream, (int)(gate->k / 32), 0, i), "bf16 decode launch");
+        if (s != NNQ_OK) return s;
+    }
+    const TcArgs a = {nullptr, nullptr, x, nullptr, nullptr, m, 2 * gate->n, gate->k, NNQ_BF16_DENSE, NNQ_BF16, NNQ_BF16};
+    return dense_bf16(ctx, w_bf16, a, h_out, gate_kind, true, stream);
 }
 
 bool gemm_dense_grouped_supported(const nnq_ctx *ctx, const TcGroupArgs &g) {
