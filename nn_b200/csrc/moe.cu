@@ -57,7 +57,18 @@ moe_router_kernel(const XT *__restrict__ x, const float *__restrict__ rw, const 
     const int tok0 = blockIdx.x * TOK;
     if (tok0 >= T) return;
     const int ntok = min(TOK, T - tok0);
-    for (int i = threadIdx.x; i < ntok * H; i += 256) xs[i] = ld_act<XT>(x, (int64_t)tok0 * H + i);
+    if (sizeof(XT) == 2 && (H & 7) == 0 && ((uintptr_t)x & 15u) == 0) {   // bf16 rows of whole 16-byte units
+        const uint4 *p = reinterpret_cast<const uint4 *>(x + (int64_t)tok0 * H);
+#pragma unroll 4
+        for (int i = threadIdx.x; i < ntok * H / 8; i += 256) {
+            const uint4 v = __ldg(p + i);
+            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) *reinterpret_cast<float2 *>(xs + 8 * i + 2 * j) = make_float2(__uint_as_float(u[j] << 16), __uint_as_float(u[j] & 0xFFFF0000u));
+        }
+    } else {
+        for (int i = threadIdx.x; i < ntok * H; i += 256) xs[i] = ld_act<XT>(x, (int64_t)tok0 * H + i);
+    }
     for (int i = ntok * H + threadIdx.x; i < TOK * H; i += 256) xs[i] = 0.0f;
     __syncthreads();
     constexpr int EB = 4;
@@ -70,15 +81,25 @@ moe_router_kernel(const XT *__restrict__ x, const float *__restrict__ rw, const 
         for (int t = 0; t < TOK; t++)
 #pragma unroll
             for (int j = 0; j < EB; j++) acc[t][j] = 0.0f;
-        for (int h = lane; h < H; h += 32) {
-            float wv[EB];
+        // (the weights of several turns are under way at a time: with those of one in flight the kernel waited for them, 65 us at 4096
+        // tokens of 2880 and 32 experts; this and the 16-byte loads of x: 50)
+        constexpr int U = 5;
+        for (int h0 = lane; h0 < H; h0 += 32 * U) {
+            float wv[U][EB];
 #pragma unroll
-            for (int j = 0; j < EB; j++) wv[j] = __ldg(w[j] + h);
+            for (int u = 0; u < U; u++)
 #pragma unroll
-            for (int t = 0; t < TOK; t++) {
-                const float xv = xs[t * H + h];
+                for (int j = 0; j < EB; j++) wv[u][j] = h0 + 32 * u < H ? __ldg(w[j] + h0 + 32 * u) : 0.0f;
 #pragma unroll
-                for (int j = 0; j < EB; j++) acc[t][j] = fmaf(xv, wv[j], acc[t][j]);
+            for (int u = 0; u < U; u++) {
+                const int h = h0 + 32 * u;
+                if (h >= H) break;
+#pragma unroll
+                for (int t = 0; t < TOK; t++) {
+                    const float xv = xs[t * H + h];
+#pragma unroll
+                    for (int j = 0; j < EB; j++) acc[t][j] = fmaf(xv, wv[u][j], acc[t][j]);
+                }
             }
         }
 #pragma unroll
@@ -151,28 +172,40 @@ moe_group_kernel(const int *__restrict__ idx, int total, int *__restrict__ count
                  int *__restrict__ rowtok, int *__restrict__ pos, int pass, int e_begin) {
     const int el = blockIdx.x;          // local expert (this device holds experts e_begin .. e_begin + gridDim.x)
     const int e = e_begin + el;
-    __shared__ int warp_sums[2][8];     // double-buffered: one barrier per 256 assignments
+    // pieces of 256 assignments per barrier, their loads under way together (both passes over 16384 assignments, one piece / eight
+    // pieces: 45 / 18.5 us)
+    constexpr int U = 8;
+    __shared__ __align__(16) int warp_sums[2][U][8];     // double-buffered
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int base = 0;                       // assignments of this expert before `start` (the same in every thread)
-    for (int start = 0, it = 0; start < total; start += 256, it++) {
-        int i = start + threadIdx.x;
-        bool hit = i < total && idx[i] == e;
-        unsigned ballot = __ballot_sync(0xFFFFFFFFu, hit);
-        if (lane == 0) warp_sums[it & 1][warp] = __popc(ballot);
-        __syncthreads();
-        int before = 0, tot = 0;
+    int base = 0;                       // assignments of this expert before the piece (the same in every thread)
+    for (int start = 0, it = 0; start < total; start += 256 * U, it++) {
+        int v[U];
+        unsigned ballot[U];
 #pragma unroll
-        for (int w = 0; w < 8; w++) {
-            const int v = warp_sums[it & 1][w];
-            tot += v;
-            if (w < warp) before += v;
+        for (int u = 0; u < U; u++) v[u] = start + 256 * u + (int)threadIdx.x < total ? idx[start + 256 * u + threadIdx.x] : -1;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            ballot[u] = __ballot_sync(0xFFFFFFFFu, v[u] == e);
+            if (lane == 0) warp_sums[it & 1][u][warp] = __popc(ballot[u]);
         }
-        if (pass == 1 && hit) {
-            int row = offset[el] + base + before + __popc(ballot & ((1u << lane) - 1u));
-            rowtok[row] = i;
-            pos[i] = row;
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int4 a = *reinterpret_cast<const int4 *>(&warp_sums[it & 1][u][0]), b = *reinterpret_cast<const int4 *>(&warp_sums[it & 1][u][4]);
+            const int n[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            int before = 0, tot = 0;
+#pragma unroll
+            for (int w = 0; w < 8; w++) {
+                tot += n[w];
+                if (w < warp) before += n[w];
+            }
+            if (pass == 1 && v[u] == e) {
+                const int i = start + 256 * u + threadIdx.x, row = offset[el] + base + before + __popc(ballot[u] & ((1u << lane) - 1u));
+                rowtok[row] = i;
+                pos[i] = row;
+            }
+            base += tot;
         }
-        base += tot;
     }
     if (pass == 0 && threadIdx.x == 0) count[el] = base;
 }
