@@ -408,6 +408,27 @@ static bool takes_gemm_ts(const nnq_ctx *ctx, const nnq_weight *w, int64_t m, in
     return m > (x_dt == NNQ_BF16 ? 32 : 16) && (x_dt == NNQ_F32 || m <= 512);
 }
 
+// Up to twice the rows the token-column kernel takes at once: two passes over the weight (the second one mostly from L2), which round
+// no weight. Products of one format in a batch make each pass together: prompt of 32 rows through eight layers of the Qwen3-8B shape,
+// a launch per product and pass / per batch and pass: 1.83 / 1.61 ms.
+static int64_t pass_rows(nnq_dtype x_dt) { return x_dt == NNQ_BF16 ? 16 : 8; }
+static bool takes_two_passes(const nnq_weight *w, int64_t m, nnq_dtype x_dt) {
+    const int64_t cols = pass_rows(x_dt);
+    return m > cols && m <= 2 * cols && !skinny_supported(w, m, x_dt) && skinny_supported(w, cols, x_dt) && skinny_supported(w, m - cols, x_dt);
+}
+static nnq_status launch_two_passes(nnq_ctx *ctx, const SkinnyJob *jobs, int count, nnq_dtype x_dt, int64_t m, nnq_dtype y_dt, cudaStream_t stream) {
+    const int64_t cols = pass_rows(x_dt);
+    const size_t xe = x_dt == NNQ_BF16 ? 2 : 4, ye = y_dt == NNQ_BF16 ? 2 : 4;
+    nnq_status s = launch_skinny(ctx, jobs, count, x_dt, cols, y_dt, stream);
+    if (s != NNQ_OK) return s;
+    SkinnyJob hi[kSkinnyMaxJobs];
+    for (int i = 0; i < count; i++) {
+        const SkinnyJob &j = jobs[i];
+        hi[i] = {j.w, static_cast<const uint8_t *>(j.x) + (size_t)cols * j.w->k * xe, j.bias, static_cast<uint8_t *>(j.y) + (size_t)cols * j.w->n * ye};
+    }
+    return launch_skinny(ctx, hi, count, x_dt, m - cols, y_dt, stream);
+}
+
 static nnq_status linear_dispatch(nnq_ctx *ctx, const nnq_weight *w, const void *x_dev, nnq_dtype x_dt,
                                   int64_t m, const float *bias_dev, void *y_dev, nnq_dtype y_dt,
                                   cudaStream_t stream) {
@@ -421,18 +442,9 @@ static nnq_status linear_dispatch(nnq_ctx *ctx, const nnq_weight *w, const void 
     if (path == NNQ_PATH_SKINNY && !skinny_ok)
         return fail(ctx, NNQ_ERR_UNSUPPORTED, "skinny path does not cover format %d, N=%lld, K=%lld, M=%lld",
                     w->fmt, (long long)w->n, (long long)w->k, (long long)m);
-    // Up to twice the rows the token-column kernel takes at once: two passes over the weight (the second
-    // one mostly from L2) are still ahead of the tensor path, which decodes a 128-row tile for them
-    // (Q4_K 4096 x 4096 at 32 rows: 2 x 7 us against 25 us; 12288 x 4096: 2 x 18 against 46).
-    const int64_t cols = x_dt == NNQ_BF16 ? 16 : 8;
-    if (path == NNQ_PATH_AUTO && !skinny_ok && m > cols && m <= 2 * cols && skinny_supported(w, cols, x_dt) &&
-        skinny_supported(w, m - cols, x_dt)) {
-        const size_t xe = x_dt == NNQ_BF16 ? 2 : 4, ye = y_dt == NNQ_BF16 ? 2 : 4;
-        SkinnyJob lo = {w, x_dev, bias_dev, y_dev};
-        SkinnyJob hi = {w, static_cast<const uint8_t *>(x_dev) + (size_t)cols * w->k * xe, bias_dev,
-                        static_cast<uint8_t *>(y_dev) + (size_t)cols * w->n * ye};
-        nnq_status s = launch_skinny(ctx, &lo, 1, x_dt, cols, y_dt, stream);
-        return s != NNQ_OK ? s : launch_skinny(ctx, &hi, 1, x_dt, m - cols, y_dt, stream);
+    if (path == NNQ_PATH_AUTO && takes_two_passes(w, m, x_dt)) {
+        const SkinnyJob job = {w, x_dev, bias_dev, y_dev};
+        return launch_two_passes(ctx, &job, 1, x_dt, m, y_dt, stream);
     }
     if (path == NNQ_PATH_AUTO && dense_gemv_supported(w, m, x_dt)) {
         TcArgs a = {w->d_raw, w->d_scales, x_dev, bias_dev, y_dev, m, w->n, w->k, w->fmt, x_dt, y_dt};
@@ -479,13 +491,14 @@ nnq_status nnq_linear_batch(nnq_ctx *ctx, int count, const nnq_weight *const *w,
     if (!ctx) return NNQ_ERR_INVALID_ARG;
     if (count < 0 || (count && (!w || !x_dev || !y_dev))) return fail(ctx, NNQ_ERR_INVALID_ARG, "bad batch arguments");
     nnq_status s;
-    bool all_ts = count > 1 && count <= kSkinnyMaxJobs;
+    bool all_ts = count > 1 && count <= kSkinnyMaxJobs, all_two = all_ts && ctx->path == NNQ_PATH_AUTO;
     bool all_skinny = count > 0 && ctx->path != NNQ_PATH_GENERIC && ctx->path != NNQ_PATH_TENSOR && ctx->path != NNQ_PATH_F32;
     for (int i = 0; i < count; i++) {
         s = linear_checked(ctx, w[i], x_dev[i], x_dt, m, bias_dev ? bias_dev[i] : nullptr, y_dev[i], y_dt);
         if (s != NNQ_OK) return s;
         all_skinny = all_skinny && skinny_supported(w[i], m, x_dt) && w[i]->fmt == w[0]->fmt;
         all_ts = all_ts && takes_gemm_ts(ctx, w[i], m, x_dt);
+        all_two = all_two && takes_two_passes(w[i], m, x_dt) && w[i]->fmt == w[0]->fmt;
     }
     if ((s = set_device(ctx)) != NNQ_OK) return s;
     if (m == 0) return NNQ_OK;
@@ -493,6 +506,11 @@ nnq_status nnq_linear_batch(nnq_ctx *ctx, int count, const nnq_weight *const *w,
         SkinnyJob jobs[kSkinnyMaxJobs];
         for (int i = 0; i < count; i++) jobs[i] = {w[i], x_dev[i], bias_dev ? bias_dev[i] : nullptr, y_dev[i]};
         return launch_skinny(ctx, jobs, count, x_dt, m, y_dt, (cudaStream_t)stream);
+    }
+    if (all_two) {
+        SkinnyJob jobs[kSkinnyMaxJobs];
+        for (int i = 0; i < count; i++) jobs[i] = {w[i], x_dev[i], bias_dev ? bias_dev[i] : nullptr, y_dev[i]};
+        return launch_two_passes(ctx, jobs, count, x_dt, m, y_dt, (cudaStream_t)stream);
     }
     if (all_ts) {
         SkinnyJob jobs[kSkinnyMaxJobs];
