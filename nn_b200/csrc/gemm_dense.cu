@@ -156,6 +156,122 @@ dequant_bf16_kernel(const uint8_t *__restrict__ src, const uint8_t *__restrict__
     }
 }
 
+// Formats whose blocks are not aligned: Q6_K, Q8_0, Q4_0. Read byte by byte from global memory they are bound by L1 (88 % busy), so a
+// warp brings 64 chunks, whole 16-byte units of any of them, to its own shared memory with asynchronous copies, the next 64 while
+// it decodes; a lane makes a chunk from halfwords, 32 at a time, and they are stored through a tile in whole lines. Bound by memory
+// then. 12288 x 4096, byte by byte / this, in us: Q6_K 32.6 / 27.0, Q8_0 39.4 / 22.7, Q4_0 28.8 / 21.1; 25600 x 5120 Q6_K 80.6 / 66.0
+// (5.6 TB/s).
+template <int FMT>
+__host__ __device__ constexpr int staged_bytes() {   // of 64 chunks
+    return FMT == NNQ_Q6_K ? 1680 : FMT == NNQ_Q8_0 ? 2176 : 1152;
+}
+template <int FMT>
+__device__ __forceinline__ void staged_chunk(const uint8_t *raw, int c, float (&o)[32]) {
+    if constexpr (FMT == NNQ_Q8_0) {
+        Decode<NNQ_Q8_0>::chunk_halfwords(reinterpret_cast<const uint16_t *>(raw + 34 * c), o);
+    } else if constexpr (FMT == NNQ_Q4_0) {
+        // two weights (a byte) per step: the high nibble stays where it is, d / 16 (exact) is its factor
+        const uint16_t *p = reinterpret_cast<const uint16_t *>(raw + 18 * c);
+        const float d = f16_bits_to_f32(p[0]);
+        const float2 unbias = make_float2(-(8388608.0f + 8.0f), -(8388608.0f + 128.0f)), d2 = make_float2(d, __fmul_rn(d, 0.0625f));
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t t = p[1 + i];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t b = t >> (8 * h);
+                const float2 v = __fmul2_rn(__fadd2_rn(make_float2(__uint_as_float((b & 0x0Fu) | 0x4B000000u), __uint_as_float((b & 0xF0u) | 0x4B000000u)), unbias), d2);
+                o[4 * i + 2 * h] = v.x;
+                o[4 * i + 2 * h + 1] = v.y;
+            }
+        }
+    } else {
+        // four weights per step: the two of a byte's low (high) nibbles side by side, q and 256 q'
+        const uint16_t *p = reinterpret_cast<const uint16_t *>(raw + 210 * (c >> 3));
+        const int j = c & 7;
+        const float d = f16_bits_to_f32(p[104]);
+        const uint32_t sc = p[96 + j];
+        const float s[2] = {__fmul_rn(d, s8_to_f(sc & 0xFFu)), __fmul_rn(d, s8_to_f(sc >> 8))};
+        const float2 unbias = make_float2(-(8388608.0f + 32.0f), -(8388608.0f + 8192.0f));
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t ql = p[8 * j + i], qh = (uint32_t)p[64 + 4 * j + (i >> 1)] >> (8 * (i & 1));
+            const uint32_t a = (ql & 0x0F0Fu) | ((qh << 4) & 0x30u) | ((qh << 8) & 0x3000u);
+            const uint32_t b = ((ql >> 4) & 0x0F0Fu) | ((qh << 2) & 0x30u) | ((qh << 6) & 0x3000u);
+            const float2 s2 = make_float2(s[i >> 2], __fmul_rn(s[i >> 2], 0.00390625f));
+            const float2 u = __fmul2_rn(__fadd2_rn(make_float2(__uint_as_float((a & 0xFFu) | 0x4B000000u), __uint_as_float((a & 0xFF00u) | 0x4B000000u)), unbias), s2);
+            const float2 v = __fmul2_rn(__fadd2_rn(make_float2(__uint_as_float((b & 0xFFu) | 0x4B000000u), __uint_as_float((b & 0xFF00u) | 0x4B000000u)), unbias), s2);
+            o[4 * i] = u.x;
+            o[4 * i + 1] = v.x;
+            o[4 * i + 2] = u.y;
+            o[4 * i + 3] = v.y;
+        }
+    }
+}
+
+constexpr int kDbResident = 8;   // CTAs per SM (registers, shared memory)
+template <int FMT>
+__global__ void __launch_bounds__(kDbThreads, kDbResident)
+dequant_staged_kernel(const uint8_t *__restrict__ src, int64_t nchunks, uint4 *__restrict__ dst, int cpr, int pair) {
+    constexpr int UB = staged_bytes<FMT>(), W = kDbThreads / 32;
+    __shared__ __align__(16) uint8_t raw[W][2][UB];
+    __shared__ uint4 tile[W][128];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, shift = (cpr & (cpr - 1)) == 0 ? __ffs(cpr) - 1 : -1;
+    const int64_t units = (nchunks + 63) / 64, total = nchunks * UB / 64, stride = (int64_t)gridDim.x * W;
+    auto bring = [&](int64_t u, int buf) {
+        if (u < units) {
+            const int64_t off = u * UB;
+            const int bytes = total - off < UB ? (int)(total - off) : UB;
+            const uint32_t to = smem_u32(raw[warp][buf]);
+#pragma unroll
+            for (int i = 0; i < (UB / 16 + 31) / 32; i++)
+                if (16 * (i * 32 + lane) + 16 <= bytes)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16 * (i * 32 + lane)), "l"(src + off + 16 * (i * 32 + lane)) : "memory");
+            const int at = (bytes & ~15) + lane;   // what is left of the last unit
+            if (lane < (bytes & 15)) raw[warp][buf][at] = __ldg(src + off + at);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int buf = 0;
+    int64_t u = (int64_t)blockIdx.x * W + warp;
+    bring(u, 0);
+    for (; u < units; u += stride, buf ^= 1) {
+        bring(u + stride, buf ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+            const int64_t base = u * 64 + 32 * h;
+            if (base + lane < nchunks) {
+                float o[32];
+                staged_chunk<FMT>(raw[warp][buf], 32 * h + lane, o);   // the bit-exact decode, then round to nearest even
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    uint32_t p[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) p[i] = pack_bf16(o[8 * j + 2 * i], o[8 * j + 2 * i + 1]);
+                    tile[warp][lane * 4 + (j ^ ((lane >> 1) & 3))] = make_uint4(p[0], p[1], p[2], p[3]);   // (swizzle: as below)
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int idx = 32 * i + lane;
+                const int64_t c = base + (idx >> 2);
+                if (c < nchunks) {
+                    int64_t oc = c;
+                    if (pair >= 0) {   // row j goes to row 2j + pair (nchunks < 2^30 here)
+                        const uint32_t row = shift >= 0 ? (uint32_t)c >> shift : (uint32_t)c / (uint32_t)cpr;
+                        oc = (int64_t)(2 * row + (uint32_t)pair) * cpr + ((uint32_t)c - row * (uint32_t)cpr);
+                    }
+                    dst[oc * 4 + (idx & 3)] = tile[warp][(idx & ~3) | ((idx & 3) ^ ((idx >> 3) & 3))];
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
 // nn-gptoss expert tensors [E, K, N] (MXFP4, 32-weight blocks along N, the even column in the high
 // nibble) -> bf16 [E, N, K]: a CTA turns a tile of 64 KT (k) x 64 (n)
 // through shared memory. Reads are whole sectors (32 bytes of a k row), writes 128 KT contiguous bytes per output row. Bound by the
@@ -207,6 +323,17 @@ dequant_kn_bf16_kernel(const uint8_t *__restrict__ data, const uint8_t *__restri
 template <int FMT>
 static cudaError_t launch_dequant_bf16(const uint8_t *src, const uint8_t *scales, int64_t nchunks, void *dst, int sm_count,
                                        cudaStream_t stream, int cpr = 1, int half_rows = 0, int pair = -1) {
+    if constexpr (FMT == NNQ_Q6_K || FMT == NNQ_Q8_0 || FMT == NNQ_Q4_0) {
+        // From a unit for every resident warp on; below, the copy in between is one more wait (1024 x 5120 Q6_K, directly / staged:
+        // 6.2 / 6.5 us). Persistent, every warp with the same number of units.
+        constexpr int W = kDbThreads / 32;
+        const int64_t units = (nchunks + 63) / 64, most = (int64_t)sm_count * kDbResident * W, rounds = (units + most - 1) / most;
+        if (half_rows == 0 && units >= most && ((uintptr_t)src & 15u) == 0) {
+            const int64_t ctas = (units + W * rounds - 1) / (W * rounds);
+            dequant_staged_kernel<FMT><<<(int)ctas, kDbThreads, 0, stream>>>(src, nchunks, reinterpret_cast<uint4 *>(dst), cpr, pair);
+            return cudaGetLastError();
+        }
+    }
     const int64_t want = (nchunks + kDbThreads - 1) / kDbThreads;
     const int64_t cap = (int64_t)sm_count * 16;
     int grid = (int)(want < cap ? want : cap);
