@@ -517,7 +517,26 @@ nnq_status nnq_linear_batch(nnq_ctx *ctx, int count, const nnq_weight *const *w,
         for (int i = 0; i < count; i++) jobs[i] = {w[i], x_dev[i], bias_dev ? bias_dev[i] : nullptr, y_dev[i]};
         return launch_gemm_ts(ctx, jobs, count, x_dt, m, y_dt, (cudaStream_t)stream);
     }
+    // neighbours with one input, where each would be decoded to bf16 by itself
+    const bool dense = ctx->path == NNQ_PATH_AUTO && x_dt == NNQ_BF16 && m > 512;
     for (int i = 0; i < count; i++) {
+        if (dense) {
+            SkinnyJob jobs[kSkinnyMaxJobs];
+            int n = 0;
+            while (n < kSkinnyMaxJobs && i + n < count) {
+                jobs[n] = {w[i + n], x_dev[i + n], bias_dev ? bias_dev[i + n] : nullptr, y_dev[i + n]};
+                n++;
+                if (n > 1 && !gemm_dense_batch_supported(ctx, jobs, n, m, x_dt)) {
+                    n--;
+                    break;
+                }
+            }
+            if (n > 1) {
+                if ((s = launch_gemm_dense_batch(ctx, jobs, n, m, y_dt, (cudaStream_t)stream)) != NNQ_OK) return s;
+                i += n - 1;
+                continue;
+            }
+        }
         s = linear_dispatch(ctx, w[i], x_dev[i], x_dt, m, bias_dev ? bias_dev[i] : nullptr, y_dev[i], y_dt,
                             (cudaStream_t)stream);
         if (s != NNQ_OK) return s;

@@ -77,6 +77,9 @@ nnq_status launch_gemm_dense_bf16(nnq_ctx *ctx, const void *w_bf16, const TcArgs
 // gate / up product of a bf16 weight with alternating gate and up rows (n = 2 * width): h_out[m, width] = f(gate) * up in
 // bf16, f = gate_kind (nnq_gate_act); gemm_dense_supported tells whether it runs, a.y is not written
 nnq_status launch_gemm_dense_pairs(nnq_ctx *ctx, const TcArgs &a, __nv_bfloat16 *h_out, int gate_kind, cudaStream_t stream);
+// products of one x with several weights of one format, decoded one behind the other into the context's scratch
+bool gemm_dense_batch_supported(const nnq_ctx *ctx, const SkinnyJob *jobs, int count, int64_t m, int x_dt);
+nnq_status launch_gemm_dense_batch(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int64_t m, int y_dt, cudaStream_t stream);
 // h_out[m, n] = f(x gate^T) * (x up^T) in bf16 for two weights of one format, decoded first into w_bf16: gemm_dense_gate_up_bytes of
 // it (0 where the two cannot be taken together); gemm_dense_shape_ok(m, 2 n, k) has to hold
 size_t gemm_dense_gate_up_bytes(const nnq_weight *gate, const nnq_weight *up);
