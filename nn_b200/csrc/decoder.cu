@@ -1747,9 +1747,9 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
             dec_qk_rope_rows_kernel<<<dim3(lh + 2 * lkv, n), hd, 0, st>>>(d->pf_q, d->pf_k, d->pf_v, L.q_norm, L.k_norm, d->d_cos, d->d_sin, pos0,
                                                                      c.rms_eps, d->pf_qrot, kc, vc, lh, lkv, hd, c.max_seq);
         // bf16 decoders: on the tensor cores (attn_split.cu, two f16 terms per operand) from 32 query vectors per key / value head and
-        // 64 keys on. Its launches take 23 us on the fewest rows and keys, the f32 kernel 0.42 us more per key: in us, f32 /
-        // tensor cores, 16.9 / 24.6 at 32 rows, 31.1 / 25.0 at 64, 37.1 / 26.9 at 8 rows behind 64, 2328 / 130 at 2048 rows of the
-        // Qwen3-8B shape. f32 decoders keep f32 products, and so do the kv heads with an infinity or a NaN: which other rows
+        // 64 keys on: below, its launches in front take as long as the f32 kernel. Prompts through eight layers of the Qwen3-8B shape,
+        // f32 / tensor cores, in us: 1843 / 1860 with 32 rows, 1391 / 1264 with 64, 1145 / 883 with 8 rows behind 56, 4478 / 2637 with
+        // 512; 2328 / 130 a layer with 2048. f32 decoders keep f32 products, and so do the kv heads with an infinity or a NaN: which other rows
         // those reach stays as in the f32 kernel. Without memory for the operand tiles the f32 kernel takes all heads.
         WindowAttn wa = {};
         wa.span = {n, pos0, nullptr};

@@ -405,7 +405,7 @@ __device__ __forceinline__ void issue_tile(uint32_t dst, const void *src, uint32
 // STEP: 1 x is a residual row to be normed, 2 also the activation of a pair of jobs (StepPart; KS = 8, a CTA takes a row tile of
 // both jobs in turn, the same warp finishes both). What it saves are launches and their waits: five kernels of a decoder layer instead
 // of nine, with the sums added to the residual row by the products in front and the rotation in the attention kernel. A
-// Qwen3-8B-shaped token (36 layers behind 2048 positions) 2545 -> 1926 us, its logits 1.9e-2 -> 1.1e-2 off 64 bits (one rounding to
+// Qwen3-8B-shaped token (36 layers behind 2048 positions) 2545 -> 1953 us, its logits 1.9e-2 -> 1.1e-2 off 64 bits (one rounding to
 // bf16 less per normed row).
 template <bool F32X, int KS, bool FUSED = false, int STEP = 0>
 __global__ void __launch_bounds__(kWarps * 32, 2)
