@@ -1791,7 +1791,7 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         // (from 513 rows on, where the products decode their weights once anyway)
         const size_t pair = gemm_dense_gate_up_bytes(L.gate, L.up);
         const bool gate_up = n > 512 && ctx->path == NNQ_PATH_AUTO && pair > 0 && pair <= d->pair_bytes && gemm_dense_shape_ok(ctx, n, 2 * L.gate->n, L.gate->k, d->act_dt);
-        if (gate_up) s = launch_gemm_dense_gate_up(ctx, L.gate, L.up, d->d_pair, d->pf_xn, n, (__nv_bfloat16 *)d->pf_mid, NNQ_ACT_SILU, st);
+        if (gate_up) s = launch_gemm_dense_gate_up(ctx, L.gate, L.up, d->d_pair, d->pf_xn, n, (__nv_bfloat16 *)d->pf_mid, st);
         else s = nnq_linear_batch(ctx, 2, w2, x2, adt, n, nullptr, y2, NNQ_F32, st);
         if (s != NNQ_OK) return s;
         const int64_t total = (int64_t)n * lffn;

@@ -351,6 +351,7 @@ static cudaError_t launch_dequant_bf16(const uint8_t *src, const uint8_t *scales
 constexpr int kDgBM = 128, kDgBK = 64;
 constexpr int kDgABytes = kDgBM * 128;
 constexpr int kDgMaxOuts = 4;
+constexpr int kDgSilu = 16;   // gate_kind: silu by expf and a rounded division
 constexpr int kDgThreads = 192;
 __host__ __device__ constexpr int dg_stage_bytes(int bn, int cg) { return kDgABytes + bn / cg * 128; }
 __host__ __device__ constexpr int dg_stages(int, int cg) { return cg == 1 ? 4 : 6; }
@@ -565,11 +566,15 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                                     gv += __ldg(bias + j);
                                     uv += __ldg(bias + I + j);
                                 }
-                                // fast exponential and division (2^-22 relative): far below the bf16 rounding of h,
-                                // and cheap enough for the epilogue to stay hidden behind the next tile's MMAs
-                                // (the tanh form of gelu is x sigmoid(2 sqrt(2 / pi) (x + 0.044715 x^3)))
-                                const float sx = gate_kind == NNQ_ACT_GELU_TANH ? 1.5957691216057308f * fmaf(0.044715f * gv * gv, gv, gv) : gv;
-                                hv[q2] = __fdividef(gv, 1.0f + __expf(-sx)) * uv;
+                                // kDgSilu: the numbers of the activation's own kernel (prompt_rows.cu). The others have the fast
+                                // exponential and division, whose error grows with the argument (2^-22 relative near zero, 2^-20
+                                // at -16; h is rounded to 2^-9). (The tanh form of gelu is x sigmoid(2 sqrt(2 / pi) (x + 0.044715 x^3)).)
+                                if (gate_kind == kDgSilu) {
+                                    hv[q2] = gv / (1.0f + expf(-gv)) * uv;
+                                } else {
+                                    const float sx = gate_kind == NNQ_ACT_GELU_TANH ? 1.5957691216057308f * fmaf(0.044715f * gv * gv, gv, gv) : gv;
+                                    hv[q2] = __fdividef(gv, 1.0f + __expf(-sx)) * uv;
+                                }
                             }
                             __nv_bfloat162 b2 = __floats2bfloat162_rn(hv[0], hv[1]);
                             packed[p >> 1] = *reinterpret_cast<uint32_t *>(&b2);
@@ -845,8 +850,7 @@ size_t gemm_dense_gate_up_bytes(const nnq_weight *gate, const nnq_weight *up) {
     if (!gate || !up || gate->fmt != up->fmt || gate->n != up->n || gate->k != up->k || gate->fmt == NNQ_BF16_DENSE || !gate->d_raw || !up->d_raw) return 0;
     return gate->n % 8 == 0 && gate->k >= kDgBK && gate->k % kDgBK == 0 && gate->n * (gate->k / 32) < (1ll << 30) ? (size_t)gate->n * (size_t)gate->k * 4 : 0;
 }
-nnq_status launch_gemm_dense_gate_up(nnq_ctx *ctx, const nnq_weight *gate, const nnq_weight *up, void *w_bf16, const void *x, int64_t m, __nv_bfloat16 *h_out, int gate_kind,
-                                     cudaStream_t stream) {
+nnq_status launch_gemm_dense_gate_up(nnq_ctx *ctx, const nnq_weight *gate, const nnq_weight *up, void *w_bf16, const void *x, int64_t m, __nv_bfloat16 *h_out, cudaStream_t stream) {
     const Geometry g = geometry(gate->fmt);
     const int64_t nchunks = gate->n * (gate->k / g.elems) * (g.elems / 32);
     const nnq_weight *w[2] = {gate, up};
@@ -855,7 +859,7 @@ nnq_status launch_gemm_dense_gate_up(nnq_ctx *ctx, const nnq_weight *gate, const
         if (s != NNQ_OK) return s;
     }
     const TcArgs a = {nullptr, nullptr, x, nullptr, nullptr, m, 2 * gate->n, gate->k, NNQ_BF16_DENSE, NNQ_BF16, NNQ_BF16};
-    return dense_bf16(ctx, w_bf16, a, h_out, gate_kind, true, stream);
+    return dense_bf16(ctx, w_bf16, a, h_out, kDgSilu, true, stream);
 }
 
 bool gemm_dense_grouped_supported(const nnq_ctx *ctx, const TcGroupArgs &g) {

@@ -80,11 +80,10 @@ nnq_status launch_gemm_dense_pairs(nnq_ctx *ctx, const TcArgs &a, __nv_bfloat16 
 // products of one x with several weights of one format, decoded one behind the other into the context's scratch
 bool gemm_dense_batch_supported(const nnq_ctx *ctx, const SkinnyJob *jobs, int count, int64_t m, int x_dt);
 nnq_status launch_gemm_dense_batch(nnq_ctx *ctx, const SkinnyJob *jobs, int count, int64_t m, int y_dt, cudaStream_t stream);
-// h_out[m, n] = f(x gate^T) * (x up^T) in bf16 for two weights of one format, decoded first into w_bf16: gemm_dense_gate_up_bytes of
+// h_out[m, n] = silu(x gate^T) * (x up^T) in bf16 for two weights of one format, decoded first into w_bf16: gemm_dense_gate_up_bytes of
 // it (0 where the two cannot be taken together); gemm_dense_shape_ok(m, 2 n, k) has to hold
 size_t gemm_dense_gate_up_bytes(const nnq_weight *gate, const nnq_weight *up);
-nnq_status launch_gemm_dense_gate_up(nnq_ctx *ctx, const nnq_weight *gate, const nnq_weight *up, void *w_bf16, const void *x, int64_t m, __nv_bfloat16 *h_out, int gate_kind,
-                                     cudaStream_t stream);
+nnq_status launch_gemm_dense_gate_up(nnq_ctx *ctx, const nnq_weight *gate, const nnq_weight *up, void *w_bf16, const void *x, int64_t m, __nv_bfloat16 *h_out, cudaStream_t stream);
 // dense_gemv.cu: one to four bf16 rows against an unquantized bf16 weight
 bool dense_gemv_supported(const nnq_weight *w, int64_t m, int x_dt);
 nnq_status launch_dense_gemv(nnq_ctx *ctx, const TcArgs &a, cudaStream_t stream);

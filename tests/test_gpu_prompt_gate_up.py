@@ -14,6 +14,42 @@ from nn_b200.formats import QuantFormat as Q
 pytestmark = pytest.mark.gpu
 
 
+def _model(fmt, hidden, ffn, max_seq=720):
+    b, rng = api.gpu_backend(), np.random.default_rng(hidden)
+    dec = decoder.Decoder(b, decoder.DecoderConfig(hidden=hidden, n_heads=2, n_kv_heads=1, ffn=ffn, n_layers=2, vocab=320, max_seq=max_seq, act_dtype=api.BF16))
+
+    def weight(n, k, f=fmt):
+        return api.DeviceWeight.from_device(b, f, torch.from_numpy(F.gen_weight(f, int(rng.integers(1 << 30)), n, k)[0]).cuda(), n, k)
+
+    norm = lambda n: (1.0 + 0.1 * rng.standard_normal(n)).astype(np.float32)  # noqa: E731
+    for i in range(2):
+        ws = [weight(*s) for s in ((256, hidden), (128, hidden), (128, hidden))]
+        dec.set_layer(i, *ws, weight(hidden, 256), weight(ffn, hidden), weight(ffn, hidden), weight(hidden, ffn, Q.Q8_0), norm(hidden), norm(hidden), norm(128), norm(128))
+    dec.set_head(torch.from_numpy(rng.standard_normal((320, hidden)).astype(np.float32)).to(torch.bfloat16).cuda(), norm(hidden), weight(320, hidden))
+    return dec
+
+
+@pytest.mark.parametrize("fmt,hidden,ffn", [(Q.Q4_K_GGML, 1280, 768), (Q.Q8_0, 576, 704)])
+def test_same_bits_as_separate_products(fmt, hidden, ffn):
+    """Both routes form every sum in the same order, round the same values and take the same activation: keys and values of the
+    second layer, behind the first one's activation, have the same bits."""
+    dec, b = _model(fmt, hidden, ffn), api.gpu_backend()
+    tokens = [int(t) for t in np.random.default_rng(3).integers(0, 320, 700)]
+    got = []
+    for path in (api.PATH_AUTO, api.PATH_TENSOR):
+        b.set_path(path)
+        try:
+            dec.prefill(tokens)
+        finally:
+            b.set_path(api.PATH_AUTO)
+        torch.cuda.synchronize()
+        b.device_status()
+        got.append([c[1, :, :700].clone() for c in dec.buffers()[:2]])
+    for one, other in zip(*got):
+        assert torch.isfinite(one).all() and torch.equal(one, other)
+    dec.release()
+
+
 @pytest.mark.parametrize("fmt,hidden,ffn", [(Q.Q4_K_GGML, 1280, 768), (Q.Q6_K, 512, 1280), (Q.Q8_0, 576, 704), (Q.Q4_0, 1024, 1088)])
 @pytest.mark.parametrize("count", [513, 700])
 def test_against_separate_products(fmt, hidden, ffn, count):
