@@ -338,7 +338,7 @@ constexpr int kGqMmaWarps = 8;
 template <int W, int NT>
 __global__ void __launch_bounds__(kGqMmaWarps * 32)
 gq_mma_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ scale, const float *__restrict__ zpf, int64_t groups, int gsteps, uint32_t flip, float off,
-              const __nv_bfloat16 *__restrict__ x, const float *__restrict__ bias, void *__restrict__ y, int y_dt, int64_t m, int64_t n, int64_t k) {
+              const __nv_bfloat16 *x, const float *__restrict__ bias, void *__restrict__ y, int y_dt, int64_t m, int64_t n, int64_t k) {
     __shared__ float part[kGqMmaWarps][16][8 * NT + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int64_t row0 = (int64_t)blockIdx.x * 16;
@@ -406,7 +406,7 @@ gq_mma_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ scale
 #pragma unroll
                 for (int i = 0; i < NT; i++) {
                     uint4 v = make_uint4(0, 0, 0, 0);
-                    if (live[i]) v = __ldg(reinterpret_cast<const uint4 *>(xr[i] + (int64_t)(st + r) * 32 * W + 8 * j));
+                    if (live[i]) v = __ldcg(reinterpret_cast<const uint4 *>(xr[i] + (int64_t)(st + r) * 32 * W + 8 * j));   // (written while this grid is resident)
                     gq_mma(d[i], a[0], b[0], a[1], b[1], __byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632));
                     gq_mma(d[i], a[2], b[2], a[3], b[3], __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
                 }

@@ -319,7 +319,7 @@ __device__ __forceinline__ void stage_x_block(const float (&xv)[8], int kb, uint
 }
 
 // This lane's 8 activations of super-block kb. FRESH = true reads with loads that bypass L1
-// (ld.global.cg): for a kernel that stages activations another CTA of the same launch has just written.
+// (ld.global.cg): for activations that are written while the grid runs, by another CTA or by the launch in front of it.
 template <bool F32X, bool FRESH>
 __device__ __forceinline__ void load_x_block(const void *x, int kb, int lane, float (&xv)[8]) {
     const int i = kb * 256 + lane * 8;
@@ -376,7 +376,7 @@ __device__ __forceinline__ float stage_normed_warp(const float *x, const float *
 #pragma unroll 2
     for (int kb = kb_begin; kb < kb_end; kb++) {
         float xv[8], wv[8];
-        load_x_block<true, false>(x, kb, lane, xv);
+        load_x_block<true, true>(x, kb, lane, xv);   // (the product in front writes the row while this grid is resident)
         load_x_block<true, false>(w, kb, lane, wv);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
