@@ -207,13 +207,13 @@ static cudaError_t launch_ks(int ksplit, const SkinnyParams &P, int grid, int sm
                         : launch_ks_f<F32X, false>(ksplit, P, grid, smem_bytes, stream);
 }
 
-template <int FMT, int SB, int NT, bool F32X>
+template <int FMT, int SB, int NT, bool F32X, bool STEP = false>
 static cudaError_t launch_mn(const SkinnyParams &P, int grid, int smem_bytes, cudaStream_t stream) {
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(skinny_mn_kernel<FMT, SB, NT, F32X>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        cudaError_t e = cudaFuncSetAttribute(skinny_mn_kernel<FMT, SB, NT, F32X, STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
         if (e != cudaSuccess) return e;
         configured[dev] = true;
     }
@@ -227,11 +227,12 @@ static cudaError_t launch_mn(const SkinnyParams &P, int grid, int smem_bytes, cu
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, skinny_mn_kernel<FMT, SB, NT, F32X>, P);
+    return cudaLaunchKernelEx(&cfg, skinny_mn_kernel<FMT, SB, NT, F32X, STEP>, P);
 }
 
 template <int FMT, int SB = 8>
-static cudaError_t launch_mn_fmt(const SkinnyParams &P, int nt, bool f32x, int grid, int smem_bytes, cudaStream_t stream) {
+static cudaError_t launch_mn_fmt(const SkinnyParams &P, bool step, int nt, bool f32x, int grid, int smem_bytes, cudaStream_t stream) {
+    if (step) return launch_mn<FMT, SB, 1, false, true>(P, grid, smem_bytes, stream);   // (one bf16 token)
     if (f32x) return launch_mn<FMT, SB, 1, true>(P, grid, smem_bytes, stream);
     return nt == 1 ? launch_mn<FMT, SB, 1, false>(P, grid, smem_bytes, stream) : launch_mn<FMT, SB, 2, false>(P, grid, smem_bytes, stream);
 }
@@ -314,13 +315,13 @@ static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, i
         int grid = tiles < ctx->sm_count * per_sm ? tiles : ctx->sm_count * per_sm;
         share_next(P, grid);
         cudaError_t e;
-        if (layout == kTiledQ4K) e = launch_mn_fmt<NNQ_Q4_K>(P, nt, f32x, grid, smem_bytes, stream);
-        else if (layout == kTiledQ8_0) e = launch_mn_fmt<NNQ_Q8_0>(P, nt, f32x, grid, smem_bytes, stream);
-        else if (layout == kTiledQ6K) e = launch_mn_fmt<NNQ_Q6_K>(P, nt, f32x, grid, smem_bytes, stream);
-        else if (layout == kTiledQ4_0) e = launch_mn_fmt<NNQ_Q4_0>(P, nt, f32x, grid, smem_bytes, stream);
-        else if (layout == kTiledQ4_1) e = launch_mn_fmt<NNQ_Q4_1>(P, nt, f32x, grid, smem_bytes, stream);
-        else if (tile_sb == 8) e = launch_mn_fmt<NNQ_MXFP4_SPLIT, 8>(P, nt, f32x, grid, smem_bytes, stream);
-        else e = launch_mn_fmt<NNQ_MXFP4_SPLIT, 6>(P, nt, f32x, grid, smem_bytes, stream);
+        if (layout == kTiledQ4K) e = launch_mn_fmt<NNQ_Q4_K>(P, step != nullptr, nt, f32x, grid, smem_bytes, stream);
+        else if (layout == kTiledQ8_0) e = launch_mn_fmt<NNQ_Q8_0>(P, step != nullptr, nt, f32x, grid, smem_bytes, stream);
+        else if (layout == kTiledQ6K) e = launch_mn_fmt<NNQ_Q6_K>(P, step != nullptr, nt, f32x, grid, smem_bytes, stream);
+        else if (layout == kTiledQ4_0) e = launch_mn_fmt<NNQ_Q4_0>(P, step != nullptr, nt, f32x, grid, smem_bytes, stream);
+        else if (layout == kTiledQ4_1) e = launch_mn_fmt<NNQ_Q4_1>(P, step != nullptr, nt, f32x, grid, smem_bytes, stream);
+        else if (tile_sb == 8) e = launch_mn_fmt<NNQ_MXFP4_SPLIT, 8>(P, step != nullptr, nt, f32x, grid, smem_bytes, stream);
+        else e = launch_mn_fmt<NNQ_MXFP4_SPLIT, 6>(P, step != nullptr, nt, f32x, grid, smem_bytes, stream);
         ctx->launches++;
         return check_cuda(ctx, e, "skinny launch");
     }
