@@ -288,7 +288,8 @@ static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, i
     int64_t job_tiles = 0;
     for (int i = 0; i < count; i++) job_tiles += (jobs[i].w->n + 15) / 16;
     const int64_t tokcol_limit = env_tc ? atoi(env_tc) : 2 * ctx->sm_count;
-    const bool token_columns = m > 1 || layout != kTiledQ4K || (!f32x && !fr && !norm && job_tiles <= tokcol_limit);
+    // (a step's rows of fewer super-blocks than warps too: the M = 1 kernel adds to y where its warps share a row tile)
+    const bool token_columns = m > 1 || layout != kTiledQ4K || (!f32x && !fr && !norm && (job_tiles <= tokcol_limit || (step && jobs[0].w->k < 256 * kWarps)));
     if (!token_columns) pick_stages(P.kblocks, f32x, &P.stages, &ctas_per_sm);
     else P.stages = 2;
     if (fr && ctas_per_sm > 2) ctas_per_sm = 2;   // register budget of the fused variant
@@ -351,6 +352,7 @@ static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, i
     share_next(P, grid);
     cudaError_t e;
     if (norm) e = step->pair ? launch_kernel<false, kWarps, false, 2>(P, grid, smem_bytes, stream) : launch_kernel<false, kWarps, false, 1>(P, grid, smem_bytes, stream);
+    else if (step) e = launch_kernel<false, kWarps, false, 3>(P, grid, smem_bytes, stream);
     else e = f32x ? launch_ks<true>(ksplit, P, grid, smem_bytes, stream) : launch_ks<false>(ksplit, P, grid, smem_bytes, stream);
     ctx->launches++;
     return check_cuda(ctx, e, "skinny launch");

@@ -402,8 +402,8 @@ __device__ __forceinline__ void issue_tile(uint32_t dst, const void *src, uint32
 // unit and on the (w % KS)-th part of K, streaming its tiles through a private ring of bulk
 // copies; with KS > 1 the partial sums of a row tile meet in shared memory and one of the KS
 // warps (in turn) writes the 16 outputs while the others already work on the next unit.
-// STEP: 1 x is a residual row to be normed, 2 also the activation of a pair of jobs (StepPart; KS = 8, a CTA takes a row tile of
-// both jobs in turn, the same warp finishes both). What it saves are launches and their waits: five kernels of a decoder layer instead
+// STEP (StepPart; KS = 8): 1 x is a residual row to be normed, 2 also the activation of a pair of jobs (a CTA takes a row tile of
+// both jobs in turn, the same warp finishes both), 3 rows as they are, added to y. All three ask for the next weights. What it saves are launches and their waits: five kernels of a decoder layer instead
 // of nine, with the sums added to the residual row by the products in front and the rotation in the attention kernel. A
 // Qwen3-8B-shaped token (36 layers behind 2048 positions) 2545 -> 1953 us, its logits 1.9e-2 -> 1.1e-2 off 64 bits (one rounding to
 // bf16 less per normed row).
@@ -531,7 +531,7 @@ skinny_q4k_m1_kernel(const __grid_constant__ SkinnyParams P) {
         ar_limit = comm_spin_limit(P.fr.peers[P.fr.rank]);
     }
 
-    if (STEP > 0) {
+    if (STEP == 1 || STEP == 2) {
         float ss = stage_normed_warp(reinterpret_cast<const float *>(P.x), P.step.norm_w, kb_lo, kb_hi, xs, tab, xinv, lane);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
@@ -602,7 +602,7 @@ skinny_q4k_m1_kernel(const __grid_constant__ SkinnyParams P) {
         }
         if (lane < 16 && row < J.n) {
             if (J.bias) v += __ldg(J.bias + row);
-            if (P.step.add) v += reinterpret_cast<const float *>(J.y)[row];
+            if (STEP == 3 && P.step.add) v += reinterpret_cast<const float *>(J.y)[row];
             if (P.y_dt == NNQ_F32) reinterpret_cast<float *>(J.y)[row] = v;
             else reinterpret_cast<__nv_bfloat16 *>(J.y)[row] = __float2bfloat16_rn(v);
         }
@@ -624,7 +624,7 @@ skinny_q4k_m1_kernel(const __grid_constant__ SkinnyParams P) {
 #pragma unroll
                 for (int w = 0; w < KS; w++) v += part[(b * kWarps + rsub * KS + w) * 16 + lane];
             }
-            if (STEP > 0) {
+            if (STEP == 1 || STEP == 2) {
                 if (rms == 0.0f) {
 #pragma unroll
                     for (int w = 0; w < kWarps; w++) rms += ssq[w];

@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 HIDDEN, FFN, VOCAB = 2048, 2304, 320
 
 
-def _model(heads, kv, layers, max_seq):
+def _model(heads, kv, layers, max_seq, HIDDEN=HIDDEN):
     b, rng = api.gpu_backend(), np.random.default_rng(heads + kv)
     dec = decoder.Decoder(b, decoder.DecoderConfig(hidden=HIDDEN, n_heads=heads, n_kv_heads=kv, ffn=FFN, n_layers=layers, vocab=VOCAB, max_seq=max_seq,
                                                    act_dtype=api.BF16))
@@ -62,4 +62,31 @@ def test_against_separate_kernels(heads, kv):
         assert got[0][0] < got[1][0]   # (the fused step is what ran)
         for one, other in zip(got[0][1:], got[1][1:]):
             assert float((one - other).norm() / other.norm()) < 1e-2, at
+    dec.release()
+
+
+@pytest.mark.parametrize("heads,kv", [(16, 8), (8, 2)])
+def test_wide_rows(heads, kv):
+    """More row tiles than the token-column kernel takes for o and down: the one-row kernel adds them to the residual row, from
+    eight super-blocks of K on (o of 16 heads), below that the token-column kernel (o of 8 heads)."""
+    dec, b, at, got = _model(heads, kv, 2, 64, 4864), api.gpu_backend(), 40, []
+    keys, values, logits = dec.buffers()[:3]
+    g = torch.Generator(device="cuda").manual_seed(3)
+    past = [torch.randn(keys.shape, device="cuda", generator=g) for _ in range(2)]
+    for path in (api.PATH_AUTO, api.PATH_SKINNY):
+        keys[:], values[:] = past
+        b.set_path(path)
+        try:
+            dec.reset(7, at)
+            before = b.launch_count()
+            dec.step()
+            launches = b.launch_count() - before
+        finally:
+            b.set_path(api.PATH_AUTO)
+        torch.cuda.synchronize()
+        b.device_status()
+        got.append((launches, logits[:].clone(), keys[:, :, at].clone(), values[:, :, at].clone()))
+    assert got[0][0] < got[1][0]
+    for one, other in zip(got[0][1:], got[1][1:]):
+        assert float((one - other).norm() / other.norm()) < 1e-2
     dec.release()
