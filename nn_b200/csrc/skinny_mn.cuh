@@ -132,8 +132,8 @@ struct MnSharedX {
 // The same from global memory (L1 / L2 resident), the sums by a second MMA with ones in place of the weights. HALVES: a lane has
 // four elements of each half of a block.
 template <int NT_, bool HALVES>
-struct MnGlobalX {
-    const uint8_t *row[NT_];
+struct MnGlobalX {   // (made for each tile, the rows by reference: as an object kept over the loop 3 % more time for Q4_K at 16 rows)
+    const uint8_t *const (&row)[NT_];
     int koff;   // the tile's first element
     template <int NT, bool F32X>
     __device__ __forceinline__ XB<F32X> frag(int block, int nt, int t) const {
@@ -623,6 +623,9 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
     using TF = TileFmt<FMT, SB>;
     constexpr int TB = TF::kBytes;
     constexpr int TE = TF::kElems;   // weights per tile row
+    // timed / untimed waits in us: Q8_0 4096 x 4096 at 16 rows 9.9 / 9.1, Q6_K at 8 f32 rows 10.5 / 10.8, Q4_0 4096 x 12288 at 9 rows
+    // 14.9 / 15.6, Q4_K 4096 x 12288 at 16 rows 16.8 / 17.0
+    constexpr bool kTimed = FMT != NNQ_Q8_0;
     extern __shared__ __align__(128) uint8_t smem[];
     const MnPlan L = mn_plan(TB, P.stages, NT);
     const int tid = threadIdx.x, lane = tid & 31;
@@ -696,11 +699,11 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // activations of this lane's token column(s); a column beyond M reads token 0 and is never stored
-    MnGlobalX<NT, TF::kSums == 2> x;
+    const uint8_t *xrow[NT];
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) {
         const int tok = nt * 8 + g;
-        x.row[nt] = reinterpret_cast<const uint8_t *>(P.x) + (size_t)(tok < P.m ? tok : 0) * P.kblocks * TE * (F32X ? 4 : 2);
+        xrow[nt] = reinterpret_cast<const uint8_t *>(P.x) + (size_t)(tok < P.m ? tok : 0) * P.kblocks * TE * (F32X ? 4 : 2);
     }
     MnConsts K;
     K.init();
@@ -722,7 +725,7 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
     // the warp whose turn it is adds the 8 partial tiles of the unit and writes the outputs
     auto finish = [&](int unit) {
         const int b = unit & 1;
-        if (!mbar_wait_fast(full_s + 8 * b, (unit >> 1) & 1u)) {
+        if (!mbar_wait_fast<kTimed>(full_s + 8 * b, (unit >> 1) & 1u)) {
             failed = true;
             return;
         }
@@ -757,9 +760,8 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
         bool ok = true;
 #pragma unroll 1
         for (int k = 0; k < nkb; k++) {
-            ok &= mbar_wait_fast(bar_s + 8 * slot, phase);
-            x.koff = (kb_lo + k) * TE;
-            TF::template tile<NT, F32X>(ring + slot * TB, sct4, x, lane, g, t, K, y);
+            ok &= mbar_wait_fast<kTimed>(bar_s + 8 * slot, phase);
+            TF::template tile<NT, F32X>(ring + slot * TB, sct4, MnGlobalX<NT, TF::kSums == 2>{xrow, (kb_lo + k) * TE}, lane, g, t, K, y);
             consumed++;
             if (++slot == stages) {
                 slot = 0;
@@ -773,7 +775,7 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
             break;
         }
         const int b = unit & 1;
-        if (unit >= 2 && !mbar_wait_fast(empty_s + 8 * b, ((unit >> 1) - 1) & 1u)) {
+        if (unit >= 2 && !mbar_wait_fast<kTimed>(empty_s + 8 * b, ((unit >> 1) - 1) & 1u)) {
             failed = true;
             break;
         }

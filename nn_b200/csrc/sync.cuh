@@ -27,8 +27,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
 }
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    // (suspends the thread until the phase ends, some microseconds at most; with a time of its own the instruction becomes a loop
-    // that polls and sleeps: 129 instead of 99 clocks from an arrival to the waiting warp, and a tenth more issue slots in gemm_ts.cu)
     asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
@@ -42,17 +40,24 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 }
 
 
-// Bounded wait written as one PTX loop: try, leave on success, else count down.
+// Bounded wait written as one PTX loop: try, leave on success, else count down. TIMED: each try may suspend the thread for 2 us at
+// most, without it as long as the machine likes. A probe measured 129 / 99 clocks from an arrival to the waiting warp with / without;
+// which form a kernel is ahead with is not that alone, and stands at the kernel.
+#define NNQ_WAIT(TIME)                                                                                    \
+    asm volatile(                                                                                         \
+        "{\n .reg .pred p;\n .reg .u32 n;\n mov.u32 n, %3;\n"                                             \
+        "W_%=:\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2" TIME ";\n @p bra D_%=;\n"          \
+        " sub.u32 n, n, 1;\n setp.ne.u32 p, n, 0;\n @p bra W_%=;\n mov.u32 %0, 0;\n bra E_%=;\n"          \
+        "D_%=:\n mov.u32 %0, 1;\nE_%=:\n}"                                                                \
+        : "=r"(ok) : "r"(bar), "r"(parity), "r"(kWaitSpins) : "memory")
+template <bool TIMED = false>
 __device__ __forceinline__ bool mbar_wait_fast(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n .reg .u32 n;\n mov.u32 n, %3;\n"
-        "W_%=:\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n @p bra D_%=;\n"
-        " sub.u32 n, n, 1;\n setp.ne.u32 p, n, 0;\n @p bra W_%=;\n mov.u32 %0, 0;\n bra E_%=;\n"
-        "D_%=:\n mov.u32 %0, 1;\nE_%=:\n}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "r"(kWaitSpins) : "memory");
+    if constexpr (TIMED) NNQ_WAIT(", 2000");
+    else NNQ_WAIT("");
     return ok != 0;
 }
+#undef NNQ_WAIT
 
 // the address of a shared-memory object at this offset in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
