@@ -406,7 +406,7 @@ gq_mma_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ scale
 #pragma unroll
                 for (int i = 0; i < NT; i++) {
                     uint4 v = make_uint4(0, 0, 0, 0);
-                    if (live[i]) v = __ldcg(reinterpret_cast<const uint4 *>(xr[i] + (int64_t)(st + r) * 32 * W + 8 * j));   // (written while this grid is resident)
+                    if (live[i]) v = *reinterpret_cast<const uint4 *>(xr[i] + (int64_t)(st + r) * 32 * W + 8 * j);   // (written while this grid is resident)
                     gq_mma(d[i], a[0], b[0], a[1], b[1], __byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632));
                     gq_mma(d[i], a[2], b[2], a[3], b[3], __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
                 }
