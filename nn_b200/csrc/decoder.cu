@@ -630,103 +630,196 @@ dec_qk_rope_rows_kernel(const float *__restrict__ q, const float *__restrict__ k
     else kcache[((size_t)(head - n_heads) * max_seq + pos) * hd + d] = y;
 }
 
-constexpr unsigned kLeftRows = 64;
 // Causal attention of a block of query rows over the cache: one warp per (kv head, R consecutive
 // rows) serves the G query heads of the group for all R rows (G * R = 16 query vectors in shared
 // memory), so that a key / value row is read once per R rows; row r sees keys 0 .. pos0 + r (the mask
 // of the reference's prompt pass: crates/nn-core/src/layers/attention/sdpa.rs:118-141). Same
 // batch-of-32-keys scheme as the decode kernel, normalised output written directly.
-// LEFT: behind the tensor-core kernel (top: its largest values), which leaves the kv heads that hold an infinity or a NaN to this one. Blocks of rows
-// are then dealt to at most kLeftRows CTAs of a kv head: as a rule they all return at once, and 4096 of them took 14 us to do so.
-template <int G, int R, bool LEFT>
+// top: not NULL behind the tensor-core kernel, which leaves the kv heads that hold an infinity or a NaN to this one.
+template <int G, int R>
 __global__ void __launch_bounds__(32)
 dec_attn_rows_kernel(const float *__restrict__ qrot, const float *__restrict__ kcache, const float *__restrict__ vcache, int pos0,
                      int n, float scale, void *__restrict__ out, int act_dt, int n_heads, int hd, int max_seq, const uint2 *top, int tiles) {
     constexpr int P = G * R;   // pair p = r * G + g
     __shared__ __align__(16) float qs[P][128];
     pdl_prologue();
-    if (LEFT) {
+    if (top) {
         const uint2 t = attn_largest(top + (size_t)blockIdx.x * tiles, tiles);
         if (max(t.x, t.y) < kNotFinite) return;
     }
-    const int kvh = blockIdx.x, lane = threadIdx.x;
-    for (int r0 = blockIdx.y * R; r0 < n; r0 += gridDim.y * R) {
-        const int rows = min(R, n - r0);
-        const int jmax = pos0 + r0 + rows;   // keys the last row of this block sees
+    const int kvh = blockIdx.x, r0 = blockIdx.y * R, lane = threadIdx.x;
+    const int rows = min(R, n - r0);
+    const int jmax = pos0 + r0 + rows;   // keys the last row of this block sees
 #pragma unroll
-        for (int p = 0; p < P; p++) {
-            const int row = r0 + min(p / G, rows - 1);   // rows past the end repeat the last one; not stored
-            *reinterpret_cast<float4 *>(&qs[p][4 * lane]) =
-                *reinterpret_cast<const float4 *>(qrot + (size_t)row * n_heads * hd + (kvh * G + p % G) * hd + 4 * lane);
-        }
-        __syncwarp();
-        float m[P], l[P];
-        float4 acc[P];
+    for (int p = 0; p < P; p++) {
+        const int row = r0 + min(p / G, rows - 1);   // rows past the end repeat the last one; not stored
+        *reinterpret_cast<float4 *>(&qs[p][4 * lane]) =
+            *reinterpret_cast<const float4 *>(qrot + (size_t)row * n_heads * hd + (kvh * G + p % G) * hd + 4 * lane);
+    }
+    __syncwarp();
+    float m[P], l[P];
+    float4 acc[P];
 #pragma unroll
-        for (int p = 0; p < P; p++) {
-            m[p] = -INFINITY;
-            l[p] = 0.0f;
-            acc[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-        const float *kb = kcache + (size_t)kvh * max_seq * hd, *vb = vcache + (size_t)kvh * max_seq * hd;
-        for (int b0 = 0; b0 < jmax; b0 += 32) {
-            const int j = b0 + lane;
-            const float4 *krow = reinterpret_cast<const float4 *>(kb + (size_t)(j < jmax ? j : b0) * hd);
-            float dot[P];
+    for (int p = 0; p < P; p++) {
+        m[p] = -INFINITY;
+        l[p] = 0.0f;
+        acc[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    const float *kb = kcache + (size_t)kvh * max_seq * hd, *vb = vcache + (size_t)kvh * max_seq * hd;
+    for (int b0 = 0; b0 < jmax; b0 += 32) {
+        const int j = b0 + lane;
+        const float4 *krow = reinterpret_cast<const float4 *>(kb + (size_t)(j < jmax ? j : b0) * hd);
+        float dot[P];
 #pragma unroll
-            for (int p = 0; p < P; p++) dot[p] = 0.0f;
+        for (int p = 0; p < P; p++) dot[p] = 0.0f;
 #pragma unroll 8
-            for (int d4 = 0; d4 < 32; d4++) {
-                const float4 kv = krow[d4];
-#pragma unroll
-                for (int p = 0; p < P; p++) {
-                    const float4 qv = *reinterpret_cast<const float4 *>(&qs[p][4 * d4]);
-                    dot[p] = fmaf(qv.x, kv.x, fmaf(qv.y, kv.y, fmaf(qv.z, kv.z, fmaf(qv.w, kv.w, dot[p]))));
-                }
-            }
+        for (int d4 = 0; d4 < 32; d4++) {
+            const float4 kv = krow[d4];
 #pragma unroll
             for (int p = 0; p < P; p++) {
-                // key j is visible to row r0 + p / G up to position pos0 + row; the first batch holds key 0
-                // for every row, so the running maximum is finite from then on
-                const bool valid = j <= pos0 + r0 + min(p / G, rows - 1);
-                const float sc = valid ? dot[p] * scale : -INFINITY;
-                float bm = sc;
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, off));
-                const float mn = fmaxf(m[p], bm);
-                const float corr = expf(m[p] - mn);
-                dot[p] = expf(sc - mn);   // the probability, kept in place of the score
-                float ps = dot[p];
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) ps += __shfl_xor_sync(0xFFFFFFFFu, ps, off);
-                l[p] = l[p] * corr + ps;
-                acc[p].x *= corr; acc[p].y *= corr; acc[p].z *= corr; acc[p].w *= corr;
-                m[p] = mn;
-            }
-            const int nb = min(32, jmax - b0);
-            for (int jj = 0; jj < nb; jj++) {
-                const float4 vv = *reinterpret_cast<const float4 *>(vb + (size_t)(b0 + jj) * hd + 4 * lane);
-#pragma unroll
-                for (int p = 0; p < P; p++) {
-                    const float pj = __shfl_sync(0xFFFFFFFFu, dot[p], jj);
-                    acc[p].x = fmaf(pj, vv.x, acc[p].x);
-                    acc[p].y = fmaf(pj, vv.y, acc[p].y);
-                    acc[p].z = fmaf(pj, vv.z, acc[p].z);
-                    acc[p].w = fmaf(pj, vv.w, acc[p].w);
-                }
+                const float4 qv = *reinterpret_cast<const float4 *>(&qs[p][4 * d4]);
+                dot[p] = fmaf(qv.x, kv.x, fmaf(qv.y, kv.y, fmaf(qv.z, kv.z, fmaf(qv.w, kv.w, dot[p]))));
             }
         }
 #pragma unroll
         for (int p = 0; p < P; p++) {
-            if (p / G >= rows) continue;
-            char *orow = reinterpret_cast<char *>(out) + (size_t)(r0 + p / G) * n_heads * hd * (act_dt == NNQ_F32 ? 4 : 2);
-            const int base = (kvh * G + p % G) * hd + 4 * lane;
-            store_act(orow, act_dt, base, acc[p].x / l[p]);
-            store_act(orow, act_dt, base + 1, acc[p].y / l[p]);
-            store_act(orow, act_dt, base + 2, acc[p].z / l[p]);
-            store_act(orow, act_dt, base + 3, acc[p].w / l[p]);
+            // key j is visible to row r0 + p / G up to position pos0 + row; the first batch holds key 0
+            // for every row, so the running maximum is finite from then on
+            const bool valid = j <= pos0 + r0 + min(p / G, rows - 1);
+            const float sc = valid ? dot[p] * scale : -INFINITY;
+            float bm = sc;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, off));
+            const float mn = fmaxf(m[p], bm);
+            const float corr = expf(m[p] - mn);
+            dot[p] = expf(sc - mn);   // the probability, kept in place of the score
+            float ps = dot[p];
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) ps += __shfl_xor_sync(0xFFFFFFFFu, ps, off);
+            l[p] = l[p] * corr + ps;
+            acc[p].x *= corr; acc[p].y *= corr; acc[p].z *= corr; acc[p].w *= corr;
+            m[p] = mn;
         }
-        if (!LEFT) break;   // (one block of rows)
+        const int nb = min(32, jmax - b0);
+        for (int jj = 0; jj < nb; jj++) {
+            const float4 vv = *reinterpret_cast<const float4 *>(vb + (size_t)(b0 + jj) * hd + 4 * lane);
+#pragma unroll
+            for (int p = 0; p < P; p++) {
+                const float pj = __shfl_sync(0xFFFFFFFFu, dot[p], jj);
+                acc[p].x = fmaf(pj, vv.x, acc[p].x);
+                acc[p].y = fmaf(pj, vv.y, acc[p].y);
+                acc[p].z = fmaf(pj, vv.z, acc[p].z);
+                acc[p].w = fmaf(pj, vv.w, acc[p].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        if (p / G >= rows) continue;
+        char *orow = reinterpret_cast<char *>(out) + (size_t)(r0 + p / G) * n_heads * hd * (act_dt == NNQ_F32 ? 4 : 2);
+        const int base = (kvh * G + p % G) * hd + 4 * lane;
+        store_act(orow, act_dt, base, acc[p].x / l[p]);
+        store_act(orow, act_dt, base + 1, acc[p].y / l[p]);
+        store_act(orow, act_dt, base + 2, acc[p].z / l[p]);
+        store_act(orow, act_dt, base + 3, acc[p].w / l[p]);
+    }
+}
+
+template <int G, int R>
+__device__ __forceinline__ void attend_rows(float (*qs)[128], const float *__restrict__ qrot, const float *__restrict__ kcache, const float *__restrict__ vcache, int pos0, int n,
+                                            float scale, void *__restrict__ out, int act_dt, int n_heads, int hd, int max_seq, int kvh, int r0, int lane) {
+    constexpr int P = G * R;   // pair p = r * G + g
+    const int rows = min(R, n - r0);
+    const int jmax = pos0 + r0 + rows;   // keys the last row of this block sees
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        const int row = r0 + min(p / G, rows - 1);   // rows past the end repeat the last one; not stored
+        *reinterpret_cast<float4 *>(&qs[p][4 * lane]) =
+            *reinterpret_cast<const float4 *>(qrot + (size_t)row * n_heads * hd + (kvh * G + p % G) * hd + 4 * lane);
+    }
+    __syncwarp();
+    float m[P], l[P];
+    float4 acc[P];
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        m[p] = -INFINITY;
+        l[p] = 0.0f;
+        acc[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    const float *kb = kcache + (size_t)kvh * max_seq * hd, *vb = vcache + (size_t)kvh * max_seq * hd;
+    for (int b0 = 0; b0 < jmax; b0 += 32) {
+        const int j = b0 + lane;
+        const float4 *krow = reinterpret_cast<const float4 *>(kb + (size_t)(j < jmax ? j : b0) * hd);
+        float dot[P];
+#pragma unroll
+        for (int p = 0; p < P; p++) dot[p] = 0.0f;
+#pragma unroll 8
+        for (int d4 = 0; d4 < 32; d4++) {
+            const float4 kv = krow[d4];
+#pragma unroll
+            for (int p = 0; p < P; p++) {
+                const float4 qv = *reinterpret_cast<const float4 *>(&qs[p][4 * d4]);
+                dot[p] = fmaf(qv.x, kv.x, fmaf(qv.y, kv.y, fmaf(qv.z, kv.z, fmaf(qv.w, kv.w, dot[p]))));
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            // key j is visible to row r0 + p / G up to position pos0 + row; the first batch holds key 0
+            // for every row, so the running maximum is finite from then on
+            const bool valid = j <= pos0 + r0 + min(p / G, rows - 1);
+            const float sc = valid ? dot[p] * scale : -INFINITY;
+            float bm = sc;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, off));
+            const float mn = fmaxf(m[p], bm);
+            const float corr = expf(m[p] - mn);
+            dot[p] = expf(sc - mn);   // the probability, kept in place of the score
+            float ps = dot[p];
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) ps += __shfl_xor_sync(0xFFFFFFFFu, ps, off);
+            l[p] = l[p] * corr + ps;
+            acc[p].x *= corr; acc[p].y *= corr; acc[p].z *= corr; acc[p].w *= corr;
+            m[p] = mn;
+        }
+        const int nb = min(32, jmax - b0);
+        for (int jj = 0; jj < nb; jj++) {
+            const float4 vv = *reinterpret_cast<const float4 *>(vb + (size_t)(b0 + jj) * hd + 4 * lane);
+#pragma unroll
+            for (int p = 0; p < P; p++) {
+                const float pj = __shfl_sync(0xFFFFFFFFu, dot[p], jj);
+                acc[p].x = fmaf(pj, vv.x, acc[p].x);
+                acc[p].y = fmaf(pj, vv.y, acc[p].y);
+                acc[p].z = fmaf(pj, vv.z, acc[p].z);
+                acc[p].w = fmaf(pj, vv.w, acc[p].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        if (p / G >= rows) continue;
+        char *orow = reinterpret_cast<char *>(out) + (size_t)(r0 + p / G) * n_heads * hd * (act_dt == NNQ_F32 ? 4 : 2);
+        const int base = (kvh * G + p % G) * hd + 4 * lane;
+        store_act(orow, act_dt, base, acc[p].x / l[p]);
+        store_act(orow, act_dt, base + 1, acc[p].y / l[p]);
+        store_act(orow, act_dt, base + 2, acc[p].z / l[p]);
+        store_act(orow, act_dt, base + 3, acc[p].w / l[p]);
+    }
+}
+
+// The same behind the tensor-core kernel for many blocks of rows. As a rule all CTAs return at once, and 4096 of one warp took 14 us
+// to do so: four warps in each, a block of rows per warp, and no more CTAs for a kv head than the GPU holds at a time.
+constexpr int kLeftWarps = 4, kLeftBlocks = 64;
+template <int G, int R>
+__global__ void __launch_bounds__(kLeftWarps * 32)
+dec_attn_left_kernel(const float *__restrict__ qrot, const float *__restrict__ kcache, const float *__restrict__ vcache, int pos0,
+                     int n, float scale, void *__restrict__ out, int act_dt, int n_heads, int hd, int max_seq, const uint2 *top, int tiles) {
+    __shared__ __align__(16) float qs[kLeftWarps][G * R][128];
+    pdl_prologue();
+    const uint2 t = attn_largest(top + (size_t)blockIdx.x * tiles, tiles);
+    if (max(t.x, t.y) < kNotFinite) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int r0 = (blockIdx.y * kLeftWarps + warp) * R; r0 < n; r0 += gridDim.y * kLeftWarps * R) {
+        attend_rows<G, R>(qs[warp], qrot, kcache, vcache, pos0, n, scale, out, act_dt, n_heads, hd, max_seq, blockIdx.x, r0, lane);
         __syncwarp();   // the query vectors have been read
     }
 }
@@ -1766,19 +1859,18 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         wa.ffn.out_k = lh * hd;
         const bool tc = attn_split_supported(wa) && pos0 + n >= 64 && image_buffer(d, pos0 + n);
         if (tc && (s = launch_attn_split(ctx, wa, d->pf_top, d->pf_images, st)) != NNQ_OK) return s;
-        const uint2 *top = tc ? d->pf_top : nullptr;
-        const int tiles = attn_tiles(pos0 + n);
         // 16 query vectors per warp: R = 16 / G rows share each key / value row
         auto attend = [&](auto all, auto left, int rows) {
-            const unsigned blocks = (unsigned)((n + rows - 1) / rows);
-            launch_pdl(tc ? left : all, dim3(lkv, tc ? std::min(blocks, kLeftRows) : blocks), dim3(32), st, d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq,
-                       top, tiles);
+            const int blocks = (n + rows - 1) / rows, ctas = std::min((blocks + kLeftWarps - 1) / kLeftWarps, 2 * ctx->sm_count);
+            if (tc && blocks > kLeftBlocks) launch_pdl(left, dim3(lkv, ctas), dim3(kLeftWarps * 32), st, d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq, d->pf_top, attn_tiles(pos0 + n));
+            else launch_pdl(all, dim3(lkv, blocks), dim3(32), st, d->pf_qrot, kc, vc, pos0, n, scale, d->pf_attn, d->act_dt, lh, hd, c.max_seq, tc ? d->pf_top : nullptr,
+                            attn_tiles(pos0 + n));
         };
         switch (group) {
-            case 1: attend(dec_attn_rows_kernel<1, 16, false>, dec_attn_rows_kernel<1, 16, true>, 16); break;
-            case 2: attend(dec_attn_rows_kernel<2, 8, false>, dec_attn_rows_kernel<2, 8, true>, 8); break;
-            case 4: attend(dec_attn_rows_kernel<4, 4, false>, dec_attn_rows_kernel<4, 4, true>, 4); break;
-            case 8: attend(dec_attn_rows_kernel<8, 2, false>, dec_attn_rows_kernel<8, 2, true>, 2); break;
+            case 1: attend(dec_attn_rows_kernel<1, 16>, dec_attn_left_kernel<1, 16>, 16); break;
+            case 2: attend(dec_attn_rows_kernel<2, 8>, dec_attn_left_kernel<2, 8>, 8); break;
+            case 4: attend(dec_attn_rows_kernel<4, 4>, dec_attn_left_kernel<4, 4>, 4); break;
+            case 8: attend(dec_attn_rows_kernel<8, 2>, dec_attn_left_kernel<8, 2>, 2); break;
             default: return fail(ctx, NNQ_ERR_UNSUPPORTED, "query heads per key/value head must be 1, 2, 4 or 8");
         }
         s = d->comm ? nnq_comm_linear(d->comm, L.o, d->pf_attn, adt, n, nullptr, d->pf_delta, NNQ_F32, st)
