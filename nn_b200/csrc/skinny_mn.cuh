@@ -57,7 +57,7 @@ __device__ __forceinline__ void split_bf16(float a, float b, uint32_t &hi, uint3
     lo = *reinterpret_cast<uint32_t *>(&l);
 }
 
-// elements [e0, e0+4) and [e1, e1+4) of the token row x (element offsets); FRESH: see load_x_block
+// elements [e0, e0+4) and [e1, e1+4) of the token row x (element offsets); FRESH: not through the read-only path
 template <bool F32X, bool FRESH = false>
 __device__ __forceinline__ XB<F32X> load_xb(const void *x, int e0, int e1) {
     auto ld = [](auto *p) { return FRESH ? __ldcg(p) : __ldg(p); };
