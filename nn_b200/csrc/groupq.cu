@@ -331,11 +331,11 @@ gq_linear_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ sc
 // add in f32, and one scale is applied per group (12288 x 4096, groups of 128: 1 row 20.2 -> 16.4 us per call, 8 rows 67 -> 19, 16
 // rows 133 -> 25). Lane 4g + t holds 8 * W consecutive weights of rows g and g + 8 (one load of
 // 4 * W bytes each); pair i of a word is (e_i, e_i+4), the activations are paired alike. A step of 32 * W weights lies inside a
-// group. The eight warps' sums meet in shared memory and are added in warp order. What is left is memory latency: a warp has four steps
-// at K = 4096, so the codes, scales and zero points of four are asked for at once, the first ones while the kernel in front still
-// runs (six such weights one after the other 98.3 -> 84.7 us; with registers for three CTAs per SM 88.4).
+// group. The eight warps' sums meet in shared memory and are added in warp order. What is left is memory latency: the codes, scales and
+// zero points of B steps are asked for ahead, the first ones while the kernel in front still runs (six such weights of 12288 x 4096 one
+// after the other 98.3 -> 84.7 us). ROLL: a step's place is filled again as soon as it is used, else all B when all are used.
 constexpr int kGqMmaWarps = 8;
-template <int W, int NT>
+template <int W, int NT, int B, bool ROLL>
 __global__ void __launch_bounds__(kGqMmaWarps * 32)
 gq_mma_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ scale, const float *__restrict__ zpf, int64_t groups, int gsteps, uint32_t flip, float off,
               const __nv_bfloat16 *x, const float *__restrict__ bias, void *__restrict__ y, int y_dt, int64_t m, int64_t n, int64_t k) {
@@ -353,7 +353,6 @@ gq_mma_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ scale
         live[j] = 8 * j + g < m;
         xr[j] = x + (live[j] ? 8 * j + g : 0) * k + 8 * W * t;
     }
-    constexpr int B = W == 1 ? 8 : 4;   // steps of a batch
     float acc[NT][4] = {};
     auto words = [&](const uint8_t *p, uint32_t (&q)[W]) {
         if (W == 4) {
@@ -378,18 +377,16 @@ gq_mma_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ scale
     // its predecessor (the weight is older than either)
     uint32_t q0[B][W], q1[B][W];
     float s0[B], s1[B], zp0[B], zp1[B];
-    auto fetch = [&](int st) {
-#pragma unroll
-        for (int i = 0; i < B; i++) {
-            if (st + i >= hi) break;
-            words(w0 + (int64_t)(st + i) * 16 * W, q0[i]);
-            words(w1 + (int64_t)(st + i) * 16 * W, q1[i]);
-            const int gi = (st + i) / gsteps;
-            s0[i] = __ldg(sc0 + gi); s1[i] = __ldg(sc1 + gi);
-            zp0[i] = __ldg(z0 + gi); zp1[i] = __ldg(z1 + gi);
-        }
+    auto fetch = [&](int i, int st) {
+        if (st >= hi) return;
+        words(w0 + (int64_t)st * 16 * W, q0[i]);
+        words(w1 + (int64_t)st * 16 * W, q1[i]);
+        const int gi = st / gsteps;
+        s0[i] = __ldg(sc0 + gi); s1[i] = __ldg(sc1 + gi);
+        zp0[i] = __ldg(z0 + gi); zp1[i] = __ldg(z1 + gi);
     };
-    fetch(lo);
+#pragma unroll
+    for (int i = 0; i < B; i++) fetch(i, lo + i);
     pdl_release();
     pdl_prologue();
     for (int st = lo; st < hi; st += B) {
@@ -418,8 +415,12 @@ gq_mma_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ scale
                 acc[i][2] = fmaf(s1[r], d[i][2], acc[i][2]);
                 acc[i][3] = fmaf(s1[r], d[i][3], acc[i][3]);
             }
+            if (ROLL) fetch(r, st + r + B);
         }
-        fetch(st + B);
+        if (!ROLL) {
+#pragma unroll
+            for (int i = 0; i < B; i++) fetch(i, st + B + i);
+        }
     }
 #pragma unroll
     for (int i = 0; i < NT; i++) {
@@ -615,17 +616,29 @@ bool gq_mma_takes(const nnq_gq_weight *w, int x_dt, int64_t m) {
     return w->bits == 4 && w->exact16 && x_dt == NNQ_BF16 && m <= 16 && !stream && w->group_size % 32 == 0 && w->n <= (1ll << 31) && w->k < (1ll << 31);
 }
 
-template <int W>
-void launch_mma(nnq_gq_weight *w, const void *x, const float *bias, void *y, int y_dt, int64_t m, cudaStream_t st) {
-    const unsigned grid = (unsigned)((w->n + 15) / 16);
+// Steps ahead: where every SM has two CTAs at most (weights of up to 4736 rows on 148 SMs) many, as registers allow; where CTAs
+// queue for the SMs few, so that more of them are resident. In us at 1 row, one form for all (four steps ahead, eight of one word) / this
+// / without steps ahead and without programmatic launch: groups of 64, 4096 x 12800 23.1 / 15.2 / 20.2, 4096 x 4096 8.2 / 6.6 / 8.4; of
+// 128, 20000 x 2048 13.1 / 10.8 / 11.7, 12288 x 4096 14.6 / 13.4 / 14.7; of 32 at 9 rows, 12288 x 4096 36.1 / 30.6 / 31.7; of 32 at 1
+// row, 1024 x 4096 7.7 / 6.9 / 7.0, 4096 x 12800 26.6 / 26.1 / 25.5. Groups of 128 and 64 on few CTAs are ahead without ROLL (4096 x 12800
+// 14.9 / 13.9 and 16.8 / 15.2).
+template <int W, int NT, int B, bool ROLL>
+void launch_mma_form(nnq_gq_weight *w, const void *x, const float *bias, void *y, int y_dt, int64_t m, cudaStream_t st) {
     const uint32_t flip = w->is_signed ? 0x88888888u : 0u;
     const float off = w->is_signed ? 136.0f : 128.0f;
-#define NNQ_GQ(NT) launch_pdl(gq_mma_kernel<W, NT>, dim3(grid), dim3(kGqMmaWarps * 32), st, w->codes, w->scale, w->zpf, w->groups, w->group_size / (32 * W), flip, off, \
-                              (const __nv_bfloat16 *)x, bias, y, y_dt, m, w->n, w->k)
-    if (m <= 8) NNQ_GQ(1);
-    else NNQ_GQ(2);
-#undef NNQ_GQ
+    launch_pdl(gq_mma_kernel<W, NT, B, ROLL>, dim3((unsigned)((w->n + 15) / 16)), dim3(kGqMmaWarps * 32), st, w->codes, w->scale, w->zpf, w->groups, w->group_size / (32 * W), flip,
+               off, (const __nv_bfloat16 *)x, bias, y, y_dt, m, w->n, w->k);
     w->ctx->launches++;
+}
+template <int W, int NT>
+void launch_mma_rows(nnq_gq_weight *w, const void *x, const float *bias, void *y, int y_dt, int64_t m, cudaStream_t st) {
+    if ((w->n + 15) / 16 <= 2 * w->ctx->sm_count) launch_mma_form<W, NT, W == 4 ? 4 : W == 2 ? 8 : 12, W == 1>(w, x, bias, y, y_dt, m, st);
+    else launch_mma_form<W, NT, W == 1 ? 4 : 2, true>(w, x, bias, y, y_dt, m, st);
+}
+template <int W>
+void launch_mma(nnq_gq_weight *w, const void *x, const float *bias, void *y, int y_dt, int64_t m, cudaStream_t st) {
+    if (m <= 8) launch_mma_rows<W, 1>(w, x, bias, y, y_dt, m, st);
+    else launch_mma_rows<W, 2>(w, x, bias, y, y_dt, m, st);
 }
 
 }  // namespace

@@ -296,3 +296,11 @@ def test_int4_products_in_several_batches_of_steps(n, k, g, m):
     w64, x64 = wq.dequantize(qt).double().cpu().numpy(), x.double().cpu().numpy()
     y = wq.quantized_matmul(x, qt).double().cpu().numpy()
     assert np.all(np.abs(y - x64 @ w64.T) <= (k + 2) * 2.0 ** -24 * (np.abs(x64) @ np.abs(w64).T))
+
+
+@pytest.mark.parametrize("m", [1, 16])
+@pytest.mark.parametrize("n,k,g", [(4750, 1152, 128), (4750, 2688, 128), (4740, 2240, 64), (4740, 1376, 32), (24, 8768, 64), (24, 6496, 32)])
+def test_int4_products_with_few_and_many_steps_ahead(n, k, g, m):
+    """Weights whose CTAs queue for the SMs (from 4737 rows on 148 SMs on): fewer steps ahead, places filled again at once; and long
+    rows of the others. The bound of the test above."""
+    test_int4_products_in_several_batches_of_steps(n, k, g, m)
