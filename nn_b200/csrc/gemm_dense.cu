@@ -64,11 +64,12 @@ __device__ __forceinline__ void mx_chunk_bf16(const uint4 q, uint32_t e, uint4 *
     }
 }
 
-template <int FMT>
+template <int FMT, bool PAIR>
 __global__ void __launch_bounds__(kDbThreads)
 dequant_bf16_kernel(const uint8_t *__restrict__ src, const uint8_t *__restrict__ scales, int64_t nchunks,
                     uint4 *__restrict__ dst, int cpr, int half_rows, int pair) {
-    // pair >= 0: row j goes to row 2j + pair (one of two weights whose rows alternate; nchunks < 2^31)
+    // PAIR: row j goes to row 2j + pair (one of two weights whose rows alternate; nchunks < 2^31). Kernels of their own: as a branch this
+    // took registers from the others (MXFP4: 87 -> 72 and spills)
     const int shift = (cpr & (cpr - 1)) == 0 ? __ffs(cpr) - 1 : -1;
     auto paired = [&](int64_t c) {
         const uint32_t row = shift >= 0 ? (uint32_t)c >> shift : (uint32_t)c / (uint32_t)cpr;
@@ -100,7 +101,7 @@ dequant_bf16_kernel(const uint8_t *__restrict__ src, const uint8_t *__restrict__
             // rows) is written interleaved, gate row j to row 2j and up row j to row 2j + 1, so that a GEMM
             // tile holds both halves of an output column pair (the fused SwiGLU epilogue)
             int64_t oc = c;
-            if (pair >= 0) {
+            if (PAIR) {
                 oc = paired(c);
             } else if (half_rows > 0) {   // nchunks < 2^31 here (checked by the launcher): 32-bit divisions
                 const uint32_t c32 = (uint32_t)c, row = c32 / (uint32_t)cpr, cin = c32 - row * (uint32_t)cpr;
@@ -147,10 +148,10 @@ dequant_bf16_kernel(const uint8_t *__restrict__ src, const uint8_t *__restrict__
         const int64_t remaining = nchunks - base;
         const int live = remaining < kDbThreads ? (int)remaining : kDbThreads;
         uint4 *out = dst + base * 4;
-        if (pair >= 0) out = dst + (paired(base + (threadIdx.x >> 2)) - (threadIdx.x >> 2)) * 4;
+        if (PAIR) out = dst + (paired(base + (threadIdx.x >> 2)) - (threadIdx.x >> 2)) * 4;
         for (int idx = threadIdx.x; idx < live * 4; idx += kDbThreads) {
             out[idx] = tile[(idx & ~3) | ((idx & 3) ^ ((idx >> 3) & 3))];
-            if (pair >= 0 && idx + kDbThreads < live * 4) out = dst + (paired(base + ((idx + kDbThreads) >> 2)) - ((idx + kDbThreads) >> 2)) * 4;
+            if (PAIR && idx + kDbThreads < live * 4) out = dst + (paired(base + ((idx + kDbThreads) >> 2)) - ((idx + kDbThreads) >> 2)) * 4;
         }
         __syncthreads();
     }
@@ -338,7 +339,8 @@ static cudaError_t launch_dequant_bf16(const uint8_t *src, const uint8_t *scales
     const int64_t cap = (int64_t)sm_count * 16;
     int grid = (int)(want < cap ? want : cap);
     if (grid < 1) grid = 1;
-    dequant_bf16_kernel<FMT><<<grid, kDbThreads, 0, stream>>>(src, scales, nchunks, reinterpret_cast<uint4 *>(dst), cpr, half_rows, pair);
+    if (pair >= 0) dequant_bf16_kernel<FMT, true><<<grid, kDbThreads, 0, stream>>>(src, scales, nchunks, reinterpret_cast<uint4 *>(dst), cpr, half_rows, pair);
+    else dequant_bf16_kernel<FMT, false><<<grid, kDbThreads, 0, stream>>>(src, scales, nchunks, reinterpret_cast<uint4 *>(dst), cpr, half_rows, pair);
     return cudaGetLastError();
 }
 
