@@ -64,7 +64,7 @@ struct nnq_decoder {
     void *pf_xn, *pf_attn, *pf_mid;
     int *pf_tokens;
     uint2 *pf_top;              // largest keys and values of every 64 positions, [lkv, max_seq / 64] (attn_split.cu)
-    void *d_pair;               // a layer's gate and up weights as bf16 for the prompt pass
+    void *d_pair;               // a layer's gate and up weights as bf16 for the prompt pass, where the context's scratch is smaller
     size_t pair_bytes;
     uint8_t *pf_images;         // keys and values of one layer as operand tiles, of pf_image_keys positions
     int pf_image_keys;
@@ -957,14 +957,6 @@ nnq_status nnq_decoder_set_layer(nnq_decoder *d, int layer, const nnq_weight *q,
     if (s != NNQ_OK) return s;
     nnq_decoder::Layer &L = d->layers[layer];
     L.q = q; L.k = k; L.v = v; L.o = o; L.gate = gate; L.up = up; L.down = down;
-    const size_t pair = d->act_dt == NNQ_BF16 ? gemm_dense_gate_up_bytes(gate, up) : 0;
-    if (pair > d->pair_bytes) {   // (without room for it the prompt takes the two products one by one)
-        cudaFree(d->d_pair);
-        d->d_pair = nullptr;
-        d->pair_bytes = 0;
-        if (cudaMalloc(&d->d_pair, pair) == cudaSuccess) d->pair_bytes = pair;
-        else { cudaGetLastError(); d->d_pair = nullptr; }
-    }
     s = check_cuda(ctx, cudaMemcpy(L.in_norm, in_norm, (size_t)c.hidden * 4, cudaMemcpyDefault), "norm weight");
     if (s == NNQ_OK) s = check_cuda(ctx, cudaMemcpy(L.post_norm, post_norm, (size_t)c.hidden * 4, cudaMemcpyDefault), "norm weight");
     if (s == NNQ_OK) s = check_cuda(ctx, cudaMemcpy(L.q_norm, q_norm, (size_t)c.head_dim * 4, cudaMemcpyDefault), "norm weight");
@@ -1817,6 +1809,27 @@ static bool image_buffer(nnq_decoder *d, int keys) {
     return true;
 }
 
+// Room for a layer's gate and up weights as bf16: the context's scratch, where the products decode theirs in turn, or, where no weight
+// of the context is as large as the two, memory of the decoder's own from the first prompt on that takes them together. NULL: none.
+static void *pair_room(nnq_decoder *d, size_t bytes) {
+    if (bytes <= d->ctx->dense_bytes) return d->ctx->d_dense;
+    return bytes <= d->pair_bytes ? d->d_pair : nullptr;
+}
+static void pair_reserve(nnq_decoder *d) {
+    size_t most = 0;
+    for (int l = 0; l < d->cfg.n_layers; l++) most = std::max(most, gemm_dense_gate_up_bytes(d->layers[l].gate, d->layers[l].up));
+    if (most <= std::max(d->ctx->dense_bytes, d->pair_bytes)) return;
+    cudaFree(d->d_pair);
+    d->d_pair = nullptr;
+    d->pair_bytes = 0;
+    if (cudaMalloc(&d->d_pair, most) == cudaSuccess) {
+        d->pair_bytes = most;
+    } else {   // the two products are taken one by one
+        cudaGetLastError();
+        d->d_pair = nullptr;
+    }
+}
+
 static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
     nnq_ctx *ctx = d->ctx;
     const nnq_decoder_config &c = d->cfg;
@@ -1826,6 +1839,9 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
     const size_t layer_cache = (size_t)lkv * c.max_seq * hd;
     const float scale = (float)(1.0 / sqrt((double)hd));
     const __nv_bfloat16 *embed = (const __nv_bfloat16 *)d->d_embed;
+    // gate and up in one GEMM: from 513 rows on, where the products decode their weights once anyway
+    const bool together = n > 512 && ctx->path == NNQ_PATH_AUTO && d->act_dt == NNQ_BF16;
+    if (together) pair_reserve(d);
     for (int l = 0; l < c.n_layers; l++) {
         const nnq_decoder::Layer &L = d->layers[l];
         float *kc = d->d_kcache + l * layer_cache, *vc = d->d_vcache + l * layer_cache;
@@ -1880,10 +1896,10 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         const nnq_weight *w2[2] = {L.gate, L.up};
         const void *x2[2] = {d->pf_xn, d->pf_xn};
         void *y2[2] = {d->pf_g, d->pf_u};
-        // (from 513 rows on, where the products decode their weights once anyway)
-        const size_t pair = gemm_dense_gate_up_bytes(L.gate, L.up);
-        const bool gate_up = n > 512 && ctx->path == NNQ_PATH_AUTO && pair > 0 && pair <= d->pair_bytes && gemm_dense_shape_ok(ctx, n, 2 * L.gate->n, L.gate->k, d->act_dt);
-        if (gate_up) s = launch_gemm_dense_gate_up(ctx, L.gate, L.up, d->d_pair, d->pf_xn, n, (__nv_bfloat16 *)d->pf_mid, st);
+        const size_t pair = together ? gemm_dense_gate_up_bytes(L.gate, L.up) : 0;
+        void *room = pair > 0 ? pair_room(d, pair) : nullptr;
+        const bool gate_up = room && gemm_dense_shape_ok(ctx, n, 2 * L.gate->n, L.gate->k, d->act_dt);
+        if (gate_up) s = launch_gemm_dense_gate_up(ctx, L.gate, L.up, room, d->pf_xn, n, (__nv_bfloat16 *)d->pf_mid, st);
         else s = nnq_linear_batch(ctx, 2, w2, x2, adt, n, nullptr, y2, NNQ_F32, st);
         if (s != NNQ_OK) return s;
         const int64_t total = (int64_t)n * lffn;
