@@ -20,6 +20,8 @@
 // CTA, the weights through shared memory and one place for each of S, P and O). Every wait is bounded.
 #include <math.h>
 
+#include <algorithm>
+
 #include "blocks.cuh"
 #include "pdl.cuh"
 #include "sync.cuh"
@@ -89,17 +91,18 @@ __global__ void __launch_bounds__(256) attn_top_kernel(const float *__restrict__
     if (tid == 0) top[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = make_uint2(m[0], m[1]);
 }
 
-// Images of the key tile (rows = keys: hi, lo of two 64-wide pieces) and the value tile (rows = dimensions: hi, lo), [kv heads, tiles].
-__global__ void __launch_bounds__(256) attn_image_kernel(const float *__restrict__ kcache, const float *__restrict__ vcache, int cap, int keys, const uint2 *__restrict__ top,
+// Images of the key tile (rows = keys: hi, lo of two 64-wide pieces) and the value tile (rows = dimensions: hi, lo), [kv heads from kv0 on, tiles].
+__global__ void __launch_bounds__(256) attn_image_kernel(const float *__restrict__ kcache, const float *__restrict__ vcache, int cap, int keys, int kv0, const uint2 *__restrict__ top,
                                                          uint8_t *__restrict__ images) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tiles = gridDim.x, key0 = blockIdx.x * kSpKeys, have = min(kSpKeys, keys - key0);
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     pdl_release();
     pdl_prologue();
-    const uint2 m = attn_largest(top + (size_t)blockIdx.y * tiles, tiles);
+    const int kvh = kv0 + blockIdx.y;
+    const uint2 m = attn_largest(top + (size_t)kvh * tiles, tiles);
     if (max(m.x, m.y) >= kNotFinite) return;
     const float k_scale = top_scale(m.x), v_scale = top_scale(m.y);
-    const float *kb = kcache + ((size_t)blockIdx.y * cap + key0) * 128, *vb = vcache + ((size_t)blockIdx.y * cap + key0) * 128;
+    const float *kb = kcache + ((size_t)kvh * cap + key0) * 128, *vb = vcache + ((size_t)kvh * cap + key0) * 128;
     uint8_t *dst = images + ((size_t)blockIdx.y * tiles + blockIdx.x) * (kSpK + kSpV);
     float4 k[8], x[4], y[4];
 #pragma unroll
@@ -141,7 +144,7 @@ __device__ __forceinline__ void sp_st8(uint32_t addr, const uint32_t (&v)[8]) {
                  ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(addr) : "memory");
 }
 
-__global__ void __launch_bounds__(kSpThreads, 1) attn_split_kernel(const WindowAttn a, const uint2 *__restrict__ top, int all_tiles, const uint8_t *__restrict__ images, int *status) {
+__global__ void __launch_bounds__(kSpThreads, 1) attn_split_kernel(const WindowAttn a, int kv0, const uint2 *__restrict__ top, int all_tiles, const uint8_t *__restrict__ images, int *status) {
     extern __shared__ __align__(1024) uint8_t sp_smem_raw[];
     uint8_t *smem = sp_smem_raw + (-smem_u32(sp_smem_raw) & 1023u);
     __shared__ __align__(8) uint64_t bars[14];   // k_full, k_empty, v_full, v_empty, s_full, p_full, o_full: two each
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) attn_split_kernel(const WindowA
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
     const uint32_t kf = smem_u32(bars), ke = kf + 16, vf = kf + 32, ve = kf + 48, sf = kf + 64, pf = kf + 80, of = kf + 96;
     // (the last rows first: they see the most keys)
-    const int kvh = blockIdx.x, group = a.heads / a.kv_heads, pairs = a.span.n * group, t0 = (gridDim.y - 1 - blockIdx.y) * kSpRows;
+    const int kvh = kv0 + blockIdx.x, group = a.heads / a.kv_heads, pairs = a.span.n * group, t0 = (gridDim.y - 1 - blockIdx.y) * kSpRows;
     const int last_pair = min(pairs, t0 + kSpRows) - 1, pos0 = a.span.pos0;
     const int tiles = (pos0 + last_pair / group) / kSpKeys + 1;
     pdl_release();
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) attn_split_kernel(const WindowA
     const uint2 m2 = attn_largest(top + (size_t)kvh * all_tiles, all_tiles);
     if (max(m2.x, m2.y) >= kNotFinite) return;
     uint8_t *k_s = smem + kSpQ, *v_s = k_s + 2 * kSpK;
-    const uint8_t *image = images + (size_t)kvh * all_tiles * (kSpK + kSpV);
+    const uint8_t *image = images + (size_t)blockIdx.x * all_tiles * (kSpK + kSpV);
 
     if (tid == 0) {
         for (int i = 0; i < 14; i++) mbar_init(kf + 8 * i, i >= 10 && i < 12 ? 4 : 1);
@@ -379,15 +382,19 @@ bool attn_split_supported(const WindowAttn &a) {
 // head's keys or values (2^-39 of that largest below). Error of the outputs against 64 bits, f32 kernel / this / two bf16 terms: 4.8e-7 /
 // 1.6e-7 / 1.7e-6 for 2048 rows of normal values, 1.2e-6 / 5.7e-7 / 9.5e-6 with four times the queries, 7.8e-7 / 3.6e-7 / 4.3e-6 for
 // 4000 rows, 2.1e-7 / 1.8e-7 / 4.0e-6 for 9 rows behind 20. Kv heads with an infinity or a NaN are left to the f32 kernel.
-// top: [kv_heads, attn_tiles(keys)], images: attn_image_bytes(kv_heads, keys).
-nnq_status launch_attn_split(nnq_ctx *ctx, const WindowAttn &a, uint2 *top, uint8_t *images, cudaStream_t st) {
+// top: [kv_heads, attn_tiles(keys)], images: attn_image_bytes(held, keys), of `held` kv heads at a time.
+nnq_status launch_attn_split(nnq_ctx *ctx, const WindowAttn &a, uint2 *top, uint8_t *images, int held, cudaStream_t st) {
     const int keys = a.span.pos0 + a.span.n, tiles = attn_tiles(keys), pairs = a.span.n * (a.heads / a.kv_heads);
     nnq_status s = check_cuda(ctx, cudaFuncSetAttribute(attn_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpSmem), "attention shared memory");
     if (s != NNQ_OK) return s;
     launch_pdl(attn_top_kernel, dim3(tiles, a.kv_heads), dim3(256), st, a.kcache, a.vcache, a.cap, keys, top);
-    launch_pdl(attn_image_kernel, dim3(tiles, a.kv_heads), dim3(256), st, a.kcache, a.vcache, a.cap, keys, top, images);
-    launch_pdl_smem(attn_split_kernel, dim3(a.kv_heads, (pairs + kSpRows - 1) / kSpRows), dim3(kSpThreads), kSpSmem, st, a, top, tiles, images, ctx->d_status);
-    ctx->launches += 3;
+    for (int kv0 = 0; kv0 < a.kv_heads; kv0 += held) {
+        const int heads = std::min(held, a.kv_heads - kv0);
+        launch_pdl(attn_image_kernel, dim3(tiles, heads), dim3(256), st, a.kcache, a.vcache, a.cap, keys, kv0, top, images);
+        launch_pdl_smem(attn_split_kernel, dim3(heads, (pairs + kSpRows - 1) / kSpRows), dim3(kSpThreads), kSpSmem, st, a, kv0, top, tiles, images, ctx->d_status);
+        ctx->launches += 2;
+    }
+    ctx->launches++;
     return check_cuda(ctx, cudaGetLastError(), "prompt attention launch");
 }
 

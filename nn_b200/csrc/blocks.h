@@ -105,7 +105,7 @@ nnq_status launch_attn_rows(nnq_ctx *ctx, const WindowAttn &a, cudaStream_t st);
 bool attn_tc_supported(const WindowAttn &a);                                           // attn_tc.cu: block of rows on the tensor cores
 nnq_status launch_attn_tc(nnq_ctx *ctx, const WindowAttn &a, cudaStream_t st);
 bool attn_split_supported(const WindowAttn &a);                                        // attn_split.cu: no window, f32-class accuracy
-nnq_status launch_attn_split(nnq_ctx *ctx, const WindowAttn &a, uint2 *top, uint8_t *images, cudaStream_t st);
+nnq_status launch_attn_split(nnq_ctx *ctx, const WindowAttn &a, uint2 *top, uint8_t *images, int held, cudaStream_t st);
 int attn_tiles(int keys);
 size_t attn_image_bytes(int kv_heads, int keys);
 nnq_status launch_attn_step(nnq_ctx *ctx, const WindowAttn &a, cudaStream_t st);       // one row, prologue and feed-forward part included

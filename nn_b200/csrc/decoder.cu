@@ -66,8 +66,8 @@ struct nnq_decoder {
     uint2 *pf_top;              // largest keys and values of every 64 positions, [lkv, max_seq / 64] (attn_split.cu)
     void *d_pair;               // a layer's gate and up weights as bf16 for the prompt pass, where the context's scratch is smaller
     size_t pair_bytes;
-    uint8_t *pf_images;         // keys and values of one layer as operand tiles, of pf_image_keys positions
-    int pf_image_keys;
+    uint8_t *pf_images;         // keys and values of one layer, or of some of its kv heads, as operand tiles
+    size_t pf_image_bytes;
     int *pf_want;               // rows of a block whose logits are asked for, [pf_rows]
     float *d_want_logits;       // [kWantRows, vocab], allocated by the first nnq_decoder_extend that asks for any
     int embed_ld, xn_ld;        // row strides of the embedding table and of the normed rows
@@ -1792,21 +1792,29 @@ static void norm_rows(nnq_decoder *d, const float *delta, const __nv_bfloat16 *e
     else dec_norm_rows_kernel<<<n, 256, 0, st>>>(d->pf_h, delta, embed, tokens, w, eps, d->pf_xn, d->act_dt, hidden);
 }
 
-// The operand tiles of a layer's keys and values (as many bytes as they have in the cache of one layer), twice as many as before
-// when a longer context comes.
-static bool image_buffer(nnq_decoder *d, int keys) {
-    if (keys <= d->pf_image_keys) return true;
-    const int want = std::min(d->cfg.max_seq, std::max(2 * d->pf_image_keys, (keys + 2047) / 2048 * 2048));
-    cudaFree(d->pf_images);   // (waits for the kernels that use it)
-    d->pf_images = nullptr;
-    d->pf_image_keys = 0;
-    if (cudaMalloc((void **)&d->pf_images, attn_image_bytes(d->lkv, want)) != cudaSuccess) {
-        cudaGetLastError();
+// Room for the operand tiles of a layer's keys and values (as many bytes as they have in the cache of one layer, twice as many as
+// before when a longer context comes): the kv heads whose tiles fit at a time. Where memory is short half of them, a quarter and so on
+// are taken in turn, without any (0) the f32 kernel takes all.
+static int image_heads(nnq_decoder *d, int keys) {
+    const size_t one = attn_image_bytes(1, keys);
+    if (d->lkv * one > d->pf_image_bytes) {
+        const int held = (int)std::min((size_t)d->cfg.max_seq, d->pf_image_bytes / attn_image_bytes(d->lkv, 64) * 64);
+        const int roomy = std::min(d->cfg.max_seq, std::max(2 * held, (keys + 2047) / 2048 * 2048));
+        cudaFree(d->pf_images);   // (waits for the kernels that use it)
         d->pf_images = nullptr;
-        return false;
+        d->pf_image_bytes = 0;
+        size_t bytes = attn_image_bytes(d->lkv, roomy);
+        int heads = d->lkv;
+        while (cudaMalloc((void **)&d->pf_images, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            d->pf_images = nullptr;
+            if (heads == 0) return 0;
+            bytes = heads * one;
+            heads /= 2;
+        }
+        d->pf_image_bytes = bytes;
     }
-    d->pf_image_keys = want;
-    return true;
+    return (int)std::min((size_t)d->lkv, d->pf_image_bytes / one);
 }
 
 // Room for a layer's gate and up weights as bf16: the context's scratch, where the products decode theirs in turn, or, where no weight
@@ -1842,6 +1850,7 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
     // gate and up in one GEMM: from 513 rows on, where the products decode their weights once anyway
     const bool together = n > 512 && ctx->path == NNQ_PATH_AUTO && d->act_dt == NNQ_BF16;
     if (together) pair_reserve(d);
+    int held = 0;   // kv heads that the prompt attention on the tensor cores takes at a time
     for (int l = 0; l < c.n_layers; l++) {
         const nnq_decoder::Layer &L = d->layers[l];
         float *kc = d->d_kcache + l * layer_cache, *vc = d->d_vcache + l * layer_cache;
@@ -1873,8 +1882,9 @@ static nnq_status rows_qwen3(nnq_decoder *d, int n, int pos0, cudaStream_t st) {
         wa.ffn.act = d->pf_attn;
         wa.ffn.act_dt = d->act_dt;
         wa.ffn.out_k = lh * hd;
-        const bool tc = attn_split_supported(wa) && pos0 + n >= 64 && image_buffer(d, pos0 + n);
-        if (tc && (s = launch_attn_split(ctx, wa, d->pf_top, d->pf_images, st)) != NNQ_OK) return s;
+        if (l == 0 && attn_split_supported(wa) && pos0 + n >= 64) held = image_heads(d, pos0 + n);
+        const bool tc = held > 0;
+        if (tc && (s = launch_attn_split(ctx, wa, d->pf_top, d->pf_images, held, st)) != NNQ_OK) return s;
         // 16 query vectors per warp: R = 16 / G rows share each key / value row
         auto attend = [&](auto all, auto left, int rows) {
             const int blocks = (n + rows - 1) / rows, ctas = std::min((blocks + kLeftWarps - 1) / kLeftWarps, 2 * ctx->sm_count);

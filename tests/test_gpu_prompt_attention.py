@@ -111,6 +111,51 @@ def test_a_value_that_is_no_number_reaches_no_earlier_block_of_rows():
     dec.release()
 
 
+def test_many_blocks_of_rows_of_a_head_with_a_value_that_is_no_number():
+    """More blocks of 16 / group rows than the f32 kernel has warps for a kv head at a time."""
+    group, count, at = 8, 2500, 2100
+    dec, model = _model(group, count)
+    ids = np.random.default_rng(5).integers(0, VOCAB - 1, count)
+    ids[at] = VOCAB - 1
+    want = _forward(model, ids)
+    bad = model["embed"].copy()
+    bad[VOCAB - 1] = np.nan
+    dec.set_head(torch.from_numpy(bad).to(torch.bfloat16).cuda(), model["final"], model["head_weight"])
+    got = dec.extend(ids, 0, list(range(count)))
+    assert np.all(np.isnan(got[at:]))
+    assert np.max(np.abs(got[:at] - want[:at])) <= 1e-2 * np.max(np.abs(want[:at]))
+    dec.backend.device_status()
+    dec.release()
+
+
+def test_operand_tiles_of_some_heads_at_a_time():
+    """A longer context behind a short one (the room for the operand tiles grows), and the same with memory for one of the two kv heads
+    at a time: the same bits."""
+    rows, pos, got = 64, 16000, []
+    ids = np.random.default_rng(7).integers(0, VOCAB, rows)
+    for short in (False, True):
+        dec, _ = _model(4, pos + rows)
+        keys, values = dec.buffers()[:2]
+        dec.prefill(ids, 0)
+        g = torch.Generator(device="cuda").manual_seed(3)
+        for c in (keys, values):
+            c[:, :, :pos] = torch.randn((*c.shape[:2], pos, 128), device="cuda", generator=g)
+        torch.cuda.synchronize()
+        hog = None
+        if short:   # (64 KB of tiles per head and 64 positions: 16.1 MB for one, 32.1 for both)
+            torch.cuda.empty_cache()
+            hog = torch.empty(torch.cuda.mem_get_info()[0] - (26 << 20), dtype=torch.uint8, device="cuda")
+        dec.prefill(ids, pos)
+        torch.cuda.synchronize()
+        dec.backend.device_status()
+        del hog
+        torch.cuda.empty_cache()
+        got.append([c[1, :, pos:pos + rows].clone() for c in (keys, values)])
+        dec.release()
+    for one, other in zip(*got):
+        assert torch.isfinite(one).all() and torch.equal(one, other)
+
+
 def test_values_that_cancel_keep_their_f32_digits():
     """Keys of zero give every visible value the same weight; two tokens whose values are opposite but for 2^-15 of them alternate,
     so that every second row's mean consists of the values' last bits. Two f16 terms hold a value to 2^-23, and each of the up to
