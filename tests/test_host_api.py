@@ -78,3 +78,19 @@ def test_algorithmic_bytes_table():
     assert F.algorithmic_bytes(Q.Q4_K, 1, 4096, 4096, 2, 2) == 9453568
     assert F.algorithmic_bytes(Q.Q8_0, 1, 4096, 4096, 4, 4) == 17858560
     assert F.algorithmic_bytes(Q.Q4_K, 1, 12288, 4096, 2, 2) == 28344320
+
+
+@pytest.mark.parametrize("gone", ["_cuda_getCurrentRawStream", "_cuda_getDevice"])
+def test_stream_handle_without_the_private_functions(monkeypatch, gone):
+    torch = pytest.importorskip("torch")
+
+    class Stream:
+        cuda_stream = 77
+
+    for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"):
+        monkeypatch.setattr(torch._C, name, lambda *a: 5, raising=False)
+    monkeypatch.setattr(torch.cuda, "is_initialized", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream())
+    assert api._stream_ptr(None) == 5 and api._stream_ptr(None, 1) == 5 and api._stream_ptr(Stream()) == 77
+    monkeypatch.delattr(torch._C, gone)
+    assert api._stream_ptr(None) == 77
