@@ -418,7 +418,9 @@ def _dtype_code(t) -> int:
 
 
 def _result(x, shape, dtype):
-    """Memory for a product of x on its device."""
+    """Memory for a product of x on its device: a plain tensor, whatever class x has."""
+    if type(x) is not _torch().Tensor:
+        return _torch().empty(shape, dtype=dtype or x.dtype, device=x.device)
     return x.new_empty(shape) if dtype is None or dtype == x.dtype else x.new_empty(shape, dtype=dtype)
 
 

@@ -72,7 +72,7 @@ class GroupWeight:
             x = x.float()
         x = x.to(dev).contiguous()
         m = math.prod(x.shape[:-1]) if x.dim() > 1 else 1
-        y = x.new_empty((*x.shape[:-1], self.out_features), dtype=out_dtype or torch.float32)
+        y = api._result(x, (*x.shape[:-1], self.out_features), out_dtype or torch.float32)
         b = self.backend
         b.check(b._lib.nnq_gq_linear(self._handle, x.data_ptr(), api._dtype_code(x), m,
                                      bias.data_ptr() if bias is not None else None, y.data_ptr(), api._dtype_code(y),

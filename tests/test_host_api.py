@@ -94,3 +94,15 @@ def test_stream_handle_without_the_private_functions(monkeypatch, gone):
     assert api._stream_ptr(None) == 5 and api._stream_ptr(None, 1) == 5 and api._stream_ptr(Stream()) == 77
     monkeypatch.delattr(torch._C, gone)
     assert api._stream_ptr(None) == 77
+
+
+def test_results_are_plain_tensors():
+    torch = pytest.importorskip("torch")
+
+    class Mine(torch.Tensor):
+        pass
+
+    for x in (torch.zeros(2, 3), torch.zeros(2, 3).as_subclass(Mine), torch.nn.Parameter(torch.zeros(2, 3))):
+        for dtype in (None, torch.float32, torch.bfloat16):
+            y = api._result(x, (2, 5), dtype)
+            assert type(y) is torch.Tensor and y.shape == (2, 5) and y.dtype == (dtype or torch.float32) and not y.requires_grad
