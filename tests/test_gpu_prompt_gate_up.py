@@ -23,10 +23,8 @@ def _model(fmt, hidden, ffn, max_seq=720, backend=None):
         return api.DeviceWeight.from_device(b, f, torch.from_numpy(F.gen_weight(f, int(rng.integers(1 << 30)), n, k)[0]).cuda(), n, k)
 
     norm = lambda n: (1.0 + 0.1 * rng.standard_normal(n)).astype(np.float32)  # noqa: E731
-    used = 0
-    for i in range(2):
-        ws = [weight(*s) for s in ((256, hidden), (128, hidden), (128, hidden))]
-        ws += [weight(hidden, 256), weight(ffn, hidden), weight(ffn, hidden), weight(hidden, ffn, Q.Q8_0)]
+    used, ws = 0, [weight(*s) for s in ((256, hidden), (128, hidden), (128, hidden), (hidden, 256), (ffn, hidden), (ffn, hidden), (hidden, ffn, Q.Q8_0))]
+    for i in range(2):   # (both layers with the same weights)
         torch.cuda.synchronize()
         free = torch.cuda.mem_get_info()[0]
         dec.set_layer(i, *ws, norm(hidden), norm(hidden), norm(128), norm(128))
@@ -35,7 +33,8 @@ def _model(fmt, hidden, ffn, max_seq=720, backend=None):
     return dec, used
 
 
-@pytest.mark.parametrize("fmt,hidden,ffn", [(Q.Q4_K_GGML, 1280, 768), (Q.Q8_0, 576, 704)])
+# (the last four large enough to be decoded through shared memory: rows of 18, 24 and 32 chunks)
+@pytest.mark.parametrize("fmt,hidden,ffn", [(Q.Q4_K_GGML, 1280, 768), (Q.Q8_0, 576, 704), (Q.Q8_0, 576, 17024), (Q.Q6_K, 768, 12736), (Q.Q4_0, 1024, 9504), (Q.Q8_0, 1024, 9504)])
 def test_same_bits_as_separate_products(fmt, hidden, ffn):
     """Both routes form every sum in the same order, round the same values and take the same activation: keys and values of the
     second layer, behind the first one's activation, have the same bits."""
