@@ -118,6 +118,9 @@ constexpr int kStateWords = 8;    // token, position, steps, context full, previ
 constexpr int kWantRows = 64;     // rows of logits formed together
 
 // h = embedding row of the current token (first layer), or h += delta (NULL: none); xn = RMSNorm(h) * w.
+// The first layer's must wait for the launch in front and must not release its successors early: the attention of a fused step reads
+// the position and the cache ahead of its own wait, and all launches between the two release early. What makes that read safe is that
+// none of them starts before this kernel has ended, and this kernel has waited for the step before, which moved the position on.
 // One CTA; every thread keeps its (up to 8) elements in registers between the two phases.
 __global__ void __launch_bounds__(1024)
 dec_norm_kernel(float *__restrict__ h, const float *__restrict__ delta, const __nv_bfloat16 *__restrict__ embed,
@@ -224,7 +227,7 @@ __device__ __forceinline__ float4 dec_rope_head(const float *src, const float *w
 // ROPE: the kernel takes the products' rows instead of prepared queries. Every CTA norms and rotates the query heads of its kv head;
 // the CTA that has the batch of the current position also does so with the key head and appends key and value. The rest of
 // the cache is older than the kernel in front (a step writes each layer's cache once), so its batches are asked for before
-// that one has ended.
+// that one has ended, and so is the position (see dec_norm_kernel).
 // A step of eight Qwen3-8B-shaped layers behind 16 / 2048 / 8000 positions, with a lane per key, batches of 32, values loaded behind
 // the softmax, and rotation, norms, activation and sums in kernels of their own 653 / 701 / 809 us, now 550 / 565 / 651.
 template <int G, bool ROPE>

@@ -3,7 +3,8 @@
 //
 // As gemm_dense.cu (persistent pairs of CTAs, cta_group::2, rings of TMA boxes, two accumulators in tensor memory), with the weights
 // as the rows of the MMA and the routed rows as its columns: an expert's rows come in any number, and the columns of an MMA come in
-// steps of 32, its rows in steps of 256. An expert's rows are dealt to tiles of at most 256 of equal size; a tile costs what it holds.
+// steps of 32, its rows in steps of 256. An expert's rows are dealt to tiles of at most 256 of equal size; a tile costs the tensor cores
+// what it holds (its copies are boxes of 128 routed rows for each CTA, whatever it holds).
 // Bound by the tensor cores: 16384 routed rows of 32 experts, 2880 x 5760 and 2880 x 2880, 660 us (1.24 PFLOP/s); with the routed rows
 // as the rows of single CTAs' MMAs, 128 at a time, it was 912.
 // The epilogue finds a weight row in a lane and a routed row in a column: a warp stores 32 neighbouring values of one routed row.
