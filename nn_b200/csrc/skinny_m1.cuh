@@ -318,19 +318,20 @@ __device__ __forceinline__ void stage_x_block(const float (&xv)[8], int kb, uint
     if (lane == 0) xinv[kb] = __uint_as_float(ex << 23);
 }
 
-// This lane's 8 activations of super-block kb. FRESH = true reads with loads that bypass L1
-// (ld.global.cg): for a kernel that stages activations another CTA of the same launch has just written.
-template <bool F32X, bool FRESH>
+// This lane's 8 activations of super-block kb. FRESH = 1 reads with loads that bypass L1
+// (ld.global.cg): for a kernel that stages activations another CTA of the same launch has just written; 2 with ordinary ones: for
+// activations that the launch in front writes while this one is resident (a decode step's residual row; past L1 a token is 16 us slower).
+template <bool F32X, int FRESH>
 __device__ __forceinline__ void load_x_block(const void *x, int kb, int lane, float (&xv)[8]) {
     const int i = kb * 256 + lane * 8;
     if (F32X) {
         const float4 *px = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(x) + i);
-        float4 a = FRESH ? __ldcg(px) : __ldg(px), b = FRESH ? __ldcg(px + 1) : __ldg(px + 1);
+        float4 a = FRESH == 2 ? *px : FRESH ? __ldcg(px) : __ldg(px), b = FRESH == 2 ? px[1] : FRESH ? __ldcg(px + 1) : __ldg(px + 1);
         xv[0] = a.x; xv[1] = a.y; xv[2] = a.z; xv[3] = a.w;
         xv[4] = b.x; xv[5] = b.y; xv[6] = b.z; xv[7] = b.w;
     } else {
         const uint4 *pv = reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(x) + i);
-        uint4 v = FRESH ? __ldcg(pv) : __ldg(pv);
+        uint4 v = FRESH == 2 ? *pv : FRESH ? __ldcg(pv) : __ldg(pv);
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -376,11 +377,7 @@ __device__ __forceinline__ float stage_normed_warp(const float *x, const float *
 #pragma unroll 2
     for (int kb = kb_begin; kb < kb_end; kb++) {
         float xv[8], wv[8];
-        // (ordinary loads: the product in front writes the row while this grid is resident; past L1 a token is 16 us slower)
-        const float4 *px = reinterpret_cast<const float4 *>(x + kb * 256 + lane * 8);
-        const float4 xa = px[0], xb = px[1];
-        xv[0] = xa.x; xv[1] = xa.y; xv[2] = xa.z; xv[3] = xa.w;
-        xv[4] = xb.x; xv[5] = xb.y; xv[6] = xb.z; xv[7] = xb.w;
+        load_x_block<true, 2>(x, kb, lane, xv);   // (the product in front writes the row while this grid is resident)
         load_x_block<true, false>(w, kb, lane, wv);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
