@@ -34,7 +34,7 @@ def _model(fmt, hidden, ffn, max_seq=720, backend=None):
 
 
 # (the last four large enough to be decoded through shared memory: rows of 18, 24 and 32 chunks)
-@pytest.mark.parametrize("fmt,hidden,ffn", [(Q.Q4_K_GGML, 1280, 768), (Q.Q8_0, 576, 704), (Q.Q8_0, 576, 17024), (Q.Q6_K, 768, 12736), (Q.Q4_0, 1024, 9504), (Q.Q8_0, 1024, 9504)])
+@pytest.mark.parametrize("fmt,hidden,ffn", [(Q.Q4_K_GGML, 1280, 768), (Q.Q8_0, 576, 704), (Q.Q8_0, 576, 17024), (Q.Q6_K, 768, 12736), (Q.Q4_0, 1024, 9536), (Q.Q8_0, 1024, 9536)])
 def test_same_bits_as_separate_products(fmt, hidden, ffn):
     """Both routes form every sum in the same order, round the same values and take the same activation: keys and values of the
     second layer, behind the first one's activation, have the same bits."""
