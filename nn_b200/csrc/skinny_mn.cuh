@@ -624,8 +624,8 @@ skinny_mn_kernel(const __grid_constant__ SkinnyParams P) {
     constexpr int TB = TF::kBytes;
     constexpr int TE = TF::kElems;   // weights per tile row
     // timed / untimed waits in us: Q8_0 4096 x 4096 at 16 rows 9.9 / 9.1, Q6_K at 8 f32 rows 10.5 / 10.8, Q4_0 4096 x 12288 at 9 rows
-    // 14.9 / 15.6, Q4_K 4096 x 12288 at 16 rows 16.8 / 17.0
-    constexpr bool kTimed = FMT != NNQ_Q8_0 && !STEP;
+    // 14.9 / 15.6, Q4_K 4096 x 12288 at 16 rows 16.8 / 17.0, but four layers of the Qwen3-8B shape 292.0 / 289.6
+    constexpr bool kTimed = FMT != NNQ_Q8_0 && FMT != NNQ_Q4_K && !STEP;
     extern __shared__ __align__(128) uint8_t smem[];
     const MnPlan L = mn_plan(TB, P.stages, NT);
     const int tid = threadIdx.x, lane = tid & 31;
