@@ -82,7 +82,8 @@ moe_router_kernel(const XT *__restrict__ x, const float *__restrict__ rw, const 
 #pragma unroll
             for (int j = 0; j < EB; j++) acc[t][j] = 0.0f;
         // (the weights of several turns are under way at a time: with those of one in flight the kernel waited for them, 65 us at 4096
-        // tokens of 2880 and 32 experts; this and the 16-byte loads of x: 50)
+        // tokens of 2880 and 32 experts; this and the 16-byte loads of x: 50. Five: 2880 is 18 whole groups of turns, other widths end in a
+        // broken one.)
         constexpr int U = 5;
         for (int h0 = lane; h0 < H; h0 += 32 * U) {
             float wv[U][EB];

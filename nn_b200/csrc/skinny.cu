@@ -359,7 +359,10 @@ static nnq_status launch_group(nnq_ctx *ctx, const SkinnyJob *jobs, int count, i
 }
 
 // Launch geometry of the grouped kernel: ways to split K (CTAs of a cluster), ring depth, tiles of K staged together,
-// clusters. `units` units of eight row tiles. The shortest estimate in tiles of a warp that has its SM's share of a CTA for itself.
+// clusters. `units` units of eight row tiles. The shortest estimate in tiles of a warp that has its SM's share of a CTA for itself
+// (two CTAs on an SM: 1.6 each; 0.8 / 0.3 for the end of a unit with / without a cluster; 0.3 per tile of K for staging, 0.5 where K comes in
+// chunks). Of 84 calls (six blocks of 8 to 64 experts, 1 to 64 tokens, bf16 and f32) it takes 1.01 of the shortest time that one split
+// forced on both products gives, at worst 1.24; one, two or four CTAs for all take 1.07, 1.07 and 1.08 of its own.
 struct GroupedShape {
     int slices, stages, chunk, clusters, smem;
 };
