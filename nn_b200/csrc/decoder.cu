@@ -731,6 +731,8 @@ dec_attn_rows_kernel(const float *__restrict__ qrot, const float *__restrict__ k
     }
 }
 
+// A block of rows of the kernel above, for the one below. (The kernel above does not call it: made of this, of a loop around it or without
+// the test of `top` it is scheduled otherwise and takes 3 to 23 % longer for one or another size of group.)
 template <int G, int R>
 __device__ __forceinline__ void attend_rows(float (*qs)[128], const float *__restrict__ qrot, const float *__restrict__ kcache, const float *__restrict__ vcache, int pos0, int n,
                                             float scale, void *__restrict__ out, int act_dt, int n_heads, int hd, int max_seq, int kvh, int r0, int lane) {
@@ -812,8 +814,9 @@ __device__ __forceinline__ void attend_rows(float (*qs)[128], const float *__res
     }
 }
 
-// The same behind the tensor-core kernel for many blocks of rows. As a rule all CTAs return at once, and 4096 of one warp took 14 us
-// to do so: four warps in each, a block of rows per warp, and no more CTAs for a kv head than the GPU holds at a time.
+// The same behind the tensor-core kernel for many blocks of rows (more than 64 of a kv head; fewer are spread over more SMs by CTAs of one
+// warp). As a rule all CTAs return at once, and 4096 of one warp took 14 us to do so: four warps in each, a block of rows per warp,
+// and no more CTAs for a kv head than the GPU holds at a time.
 constexpr int kLeftWarps = 4, kLeftBlocks = 64;
 template <int G, int R>
 __global__ void __launch_bounds__(kLeftWarps * 32)

@@ -180,8 +180,8 @@ gemm_experts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
                 const int left = cnt - c0;   // routed rows of these 32 columns
                 if (h_out) {
                     // Interleaved gate / up rows (2j, 2j + 1) lie in neighbouring lanes: an even lane forms h = clamp(silu(g), +-limit) * u of
-                    // every even column, an odd one of every odd column. (Fast exponential and division, 2^-22 relative: far below the bf16
-                    // rounding of h.)
+                    // every even column, an odd one of every odd column. (Fast exponential and division, 2^-22 relative near zero, 2^-20
+                    // at -16: far below the bf16 rounding of h.)
                     __nv_bfloat16 *h = h_out + (size_t)(m0 + c0 + (lane & 1)) * I + (row >> 1);
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
