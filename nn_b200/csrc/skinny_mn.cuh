@@ -57,15 +57,14 @@ __device__ __forceinline__ void split_bf16(float a, float b, uint32_t &hi, uint3
     lo = *reinterpret_cast<uint32_t *>(&l);
 }
 
-// elements [e0, e0+4) and [e1, e1+4) of the token row x (element offsets); FRESH: not through the read-only path
-template <bool F32X, bool FRESH = false>
+// elements [e0, e0+4) and [e1, e1+4) of the token row x (element offsets)
+template <bool F32X>
 __device__ __forceinline__ XB<F32X> load_xb(const void *x, int e0, int e1) {
-    auto ld = [](auto *p) { return FRESH ? __ldcg(p) : __ldg(p); };
     XB<F32X> r;
     if (F32X) {
         const float *p = reinterpret_cast<const float *>(x);
-        const float4 u = ld(reinterpret_cast<const float4 *>(p + e0));
-        const float4 v = ld(reinterpret_cast<const float4 *>(p + e1));
+        const float4 u = __ldg(reinterpret_cast<const float4 *>(p + e0));
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(p + e1));
         split_bf16(u.x, u.y, r.hi.x, r.lo.x);
         split_bf16(u.z, u.w, r.hi.y, r.lo.y);
         split_bf16(v.x, v.y, r.hi.z, r.lo.z);
@@ -73,10 +72,10 @@ __device__ __forceinline__ XB<F32X> load_xb(const void *x, int e0, int e1) {
     } else {
         const __nv_bfloat16 *p = reinterpret_cast<const __nv_bfloat16 *>(x);
         if (e1 == e0 + 4) {
-            r.hi = ld(reinterpret_cast<const uint4 *>(p + e0));
+            r.hi = __ldg(reinterpret_cast<const uint4 *>(p + e0));
         } else {
-            const uint2 u = ld(reinterpret_cast<const uint2 *>(p + e0));
-            const uint2 v = ld(reinterpret_cast<const uint2 *>(p + e1));
+            const uint2 u = __ldg(reinterpret_cast<const uint2 *>(p + e0));
+            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p + e1));
             r.hi = make_uint4(u.x, u.y, v.x, v.y);
         }
         r.lo = make_uint4(0, 0, 0, 0);
@@ -584,7 +583,7 @@ __device__ __forceinline__ void mn_stage(uint8_t *xs, float *sums, int t0, int t
         XB<F32X> xb;
         xb.hi = xb.lo = make_uint4(0, 0, 0, 0);
         const int e = t0 * TF::kElems + block * 32;
-        if (r) xb = SUMS == 2 ? load_xb<F32X, true>(r, e + 4 * t, e + 4 * t + 16) : load_xb<F32X, true>(r, e + 8 * t, e + 8 * t + 4);
+        if (r) xb = SUMS == 2 ? load_xb<F32X>(r, e + 4 * t, e + 4 * t + 16) : load_xb<F32X>(r, e + 8 * t, e + 8 * t + 4);
         uint4 *dst = reinterpret_cast<uint4 *>(xs) + i * (F32X ? 64 : 32) + lane;
         dst[0] = xb.hi;
         if (F32X) dst[32] = xb.lo;
@@ -849,7 +848,9 @@ skinny_grouped_kernel(const __grid_constant__ GroupedParams P) {
     const int kb_lo = rank * P.kblocks / slices, nkb = (rank + 1) * P.kblocks / slices - kb_lo;
     MnRing<TB> R;
     R.init(smem, reinterpret_cast<uint64_t *>(smem + L.bar_off), warp, lane, P.stages, nkb);
-    // the routing tables come from the kernels before this one
+    // The routing tables and rows come from the kernels before this one. Those must not release early: tables and rows are read through the
+    // read-only path, which wants them written before this grid is resident (with ordinary loads the staging waits for each in turn, calls of
+    // few f32 rows 3 to 11 % longer).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (warp == 0) {   // (at most 64 experts: two per lane)
@@ -936,7 +937,7 @@ skinny_grouped_kernel(const __grid_constant__ GroupedParams P) {
         const int r0 = P.offset[e] + (q - goff[e]) * kGroupRows, cnt = min(kGroupRows, P.offset[e + 1] - r0);
         auto row = [&](int col) -> const uint8_t * {
             if (col >= cnt) return nullptr;
-            const int src = P.rowtok ? __ldcg(P.rowtok + r0 + col) / P.top_k : r0 + col;   // (the kernels in front write tables and rows while this grid is resident)
+            const int src = P.rowtok ? __ldg(P.rowtok + r0 + col) / P.top_k : r0 + col;
             return reinterpret_cast<const uint8_t *>(P.x) + (size_t)src * ldx;
         };
         float y[NT][4];
