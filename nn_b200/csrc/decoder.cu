@@ -641,98 +641,6 @@ dec_qk_rope_rows_kernel(const float *__restrict__ q, const float *__restrict__ k
 // memory), so that a key / value row is read once per R rows; row r sees keys 0 .. pos0 + r (the mask
 // of the reference's prompt pass: crates/nn-core/src/layers/attention/sdpa.rs:118-141). Same
 // batch-of-32-keys scheme as the decode kernel, normalised output written directly.
-// top: not NULL behind the tensor-core kernel, which leaves the kv heads that hold an infinity or a NaN to this one.
-template <int G, int R>
-__global__ void __launch_bounds__(32)
-dec_attn_rows_kernel(const float *__restrict__ qrot, const float *__restrict__ kcache, const float *__restrict__ vcache, int pos0,
-                     int n, float scale, void *__restrict__ out, int act_dt, int n_heads, int hd, int max_seq, const uint2 *top, int tiles) {
-    constexpr int P = G * R;   // pair p = r * G + g
-    __shared__ __align__(16) float qs[P][128];
-    pdl_prologue();
-    if (top) {
-        const uint2 t = attn_largest(top + (size_t)blockIdx.x * tiles, tiles);
-        if (max(t.x, t.y) < kNotFinite) return;
-    }
-    const int kvh = blockIdx.x, r0 = blockIdx.y * R, lane = threadIdx.x;
-    const int rows = min(R, n - r0);
-    const int jmax = pos0 + r0 + rows;   // keys the last row of this block sees
-#pragma unroll
-    for (int p = 0; p < P; p++) {
-        const int row = r0 + min(p / G, rows - 1);   // rows past the end repeat the last one; not stored
-        *reinterpret_cast<float4 *>(&qs[p][4 * lane]) =
-            *reinterpret_cast<const float4 *>(qrot + (size_t)row * n_heads * hd + (kvh * G + p % G) * hd + 4 * lane);
-    }
-    __syncwarp();
-    float m[P], l[P];
-    float4 acc[P];
-#pragma unroll
-    for (int p = 0; p < P; p++) {
-        m[p] = -INFINITY;
-        l[p] = 0.0f;
-        acc[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-    const float *kb = kcache + (size_t)kvh * max_seq * hd, *vb = vcache + (size_t)kvh * max_seq * hd;
-    for (int b0 = 0; b0 < jmax; b0 += 32) {
-        const int j = b0 + lane;
-        const float4 *krow = reinterpret_cast<const float4 *>(kb + (size_t)(j < jmax ? j : b0) * hd);
-        float dot[P];
-#pragma unroll
-        for (int p = 0; p < P; p++) dot[p] = 0.0f;
-#pragma unroll 8
-        for (int d4 = 0; d4 < 32; d4++) {
-            const float4 kv = krow[d4];
-#pragma unroll
-            for (int p = 0; p < P; p++) {
-                const float4 qv = *reinterpret_cast<const float4 *>(&qs[p][4 * d4]);
-                dot[p] = fmaf(qv.x, kv.x, fmaf(qv.y, kv.y, fmaf(qv.z, kv.z, fmaf(qv.w, kv.w, dot[p]))));
-            }
-        }
-#pragma unroll
-        for (int p = 0; p < P; p++) {
-            // key j is visible to row r0 + p / G up to position pos0 + row; the first batch holds key 0
-            // for every row, so the running maximum is finite from then on
-            const bool valid = j <= pos0 + r0 + min(p / G, rows - 1);
-            const float sc = valid ? dot[p] * scale : -INFINITY;
-            float bm = sc;
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, off));
-            const float mn = fmaxf(m[p], bm);
-            const float corr = expf(m[p] - mn);
-            dot[p] = expf(sc - mn);   // the probability, kept in place of the score
-            float ps = dot[p];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) ps += __shfl_xor_sync(0xFFFFFFFFu, ps, off);
-            l[p] = l[p] * corr + ps;
-            acc[p].x *= corr; acc[p].y *= corr; acc[p].z *= corr; acc[p].w *= corr;
-            m[p] = mn;
-        }
-        const int nb = min(32, jmax - b0);
-        for (int jj = 0; jj < nb; jj++) {
-            const float4 vv = *reinterpret_cast<const float4 *>(vb + (size_t)(b0 + jj) * hd + 4 * lane);
-#pragma unroll
-            for (int p = 0; p < P; p++) {
-                const float pj = __shfl_sync(0xFFFFFFFFu, dot[p], jj);
-                acc[p].x = fmaf(pj, vv.x, acc[p].x);
-                acc[p].y = fmaf(pj, vv.y, acc[p].y);
-                acc[p].z = fmaf(pj, vv.z, acc[p].z);
-                acc[p].w = fmaf(pj, vv.w, acc[p].w);
-            }
-        }
-    }
-#pragma unroll
-    for (int p = 0; p < P; p++) {
-        if (p / G >= rows) continue;
-        char *orow = reinterpret_cast<char *>(out) + (size_t)(r0 + p / G) * n_heads * hd * (act_dt == NNQ_F32 ? 4 : 2);
-        const int base = (kvh * G + p % G) * hd + 4 * lane;
-        store_act(orow, act_dt, base, acc[p].x / l[p]);
-        store_act(orow, act_dt, base + 1, acc[p].y / l[p]);
-        store_act(orow, act_dt, base + 2, acc[p].z / l[p]);
-        store_act(orow, act_dt, base + 3, acc[p].w / l[p]);
-    }
-}
-
-// A block of rows of the kernel above, for the one below. (The kernel above does not call it: made of this, of a loop around it or without
-// the test of `top` it is scheduled otherwise and takes 3 to 23 % longer for one or another size of group.)
 template <int G, int R>
 __device__ __forceinline__ void attend_rows(float (*qs)[128], const float *__restrict__ qrot, const float *__restrict__ kcache, const float *__restrict__ vcache, int pos0, int n,
                                             float scale, void *__restrict__ out, int act_dt, int n_heads, int hd, int max_seq, int kvh, int r0, int lane) {
@@ -812,6 +720,21 @@ __device__ __forceinline__ void attend_rows(float (*qs)[128], const float *__res
         store_act(orow, act_dt, base + 2, acc[p].z / l[p]);
         store_act(orow, act_dt, base + 3, acc[p].w / l[p]);
     }
+}
+
+// top: not NULL behind the tensor-core kernel, which leaves the kv heads that hold an infinity or a NaN to this one. (How the body is
+// scheduled depends on what stands around it: in a loop over blocks of rows 16 / 8 heads took 5 to 10 % longer, without the test of `top` 2.)
+template <int G, int R>
+__global__ void __launch_bounds__(32)
+dec_attn_rows_kernel(const float *__restrict__ qrot, const float *__restrict__ kcache, const float *__restrict__ vcache, int pos0,
+                     int n, float scale, void *__restrict__ out, int act_dt, int n_heads, int hd, int max_seq, const uint2 *top, int tiles) {
+    __shared__ __align__(16) float qs[G * R][128];
+    pdl_prologue();
+    if (top) {
+        const uint2 t = attn_largest(top + (size_t)blockIdx.x * tiles, tiles);
+        if (max(t.x, t.y) < kNotFinite) return;
+    }
+    attend_rows<G, R>(qs, qrot, kcache, vcache, pos0, n, scale, out, act_dt, n_heads, hd, max_seq, blockIdx.x, blockIdx.y * R, threadIdx.x);
 }
 
 // The same behind the tensor-core kernel for many blocks of rows (more than 64 of a kv head; fewer are spread over more SMs by CTAs of one
