@@ -723,7 +723,7 @@ __device__ __forceinline__ void attend_rows(float (*qs)[128], const float *__res
 }
 
 // top: not NULL behind the tensor-core kernel, which leaves the kv heads that hold an infinity or a NaN to this one. (How the body is
-// scheduled depends on what stands around it: in a loop over blocks of rows 16 / 8 heads took 5 to 10 % longer, without the test of `top` 2.)
+// scheduled depends on what stands around it: written out in a loop over blocks of rows, 16 / 8 heads took 5 to 10 % longer.)
 template <int G, int R>
 __global__ void __launch_bounds__(32)
 dec_attn_rows_kernel(const float *__restrict__ qrot, const float *__restrict__ kcache, const float *__restrict__ vcache, int pos0,
