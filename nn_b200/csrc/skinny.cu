@@ -368,7 +368,7 @@ struct GroupedShape {
 };
 
 static GroupedShape grouped_shape(int kblocks, int sb, int tile_bytes, int nt, bool f32x, int sums, int64_t units, int sms) {
-    static const int fit148[9] = {0, 296, 148, 93, 71, 56, 45, 37, 33};   // clusters resident at two CTAs per SM
+    static const int fit148[9] = {0, 296, 148, 93, 71, 56, 45, 37, 33};   // clusters of this shared memory resident on 148 SMs (cudaOccupancyMaxActiveClusters)
     static const char *env = diag_env("NNQ_GROUPED_SLICES"), *env_st = diag_env("NNQ_GROUPED_STAGES");   // tuning aids
     const int forced = env ? atoi(env) : 0, forced_st = env_st ? atoi(env_st) : 0;
     GroupedShape best = {};
